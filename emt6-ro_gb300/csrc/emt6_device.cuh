@@ -209,29 +209,39 @@ __device__ __forceinline__ void store_cell(float4 *c, const DCell &d) {
   c[2] = make_float4(d.t4, __uint_as_float(d.mode | (d.phase << 8)), 0.f, 0.f);
 }
 
-// cell.cu:72-82 (+ :33-70)
+// cell.cu:33-70: the metabolic mode that a cell's levels allow; false if none
+// does (the cell dies).  g1s: held at the G1/S check; rest: in a phase that can
+// be quiescent.  Every condition is evaluated and combined without branches:
+// the lanes of a warp hold cells of all modes and phases.
+__device__ __forceinline__ bool metabolic_mode(const KParams &p, float l0, float l1, float l2,
+                                               bool g1s, bool rest, uint32_t &mode) {
+  const bool q = l2 < p.quiescence_gi, d = l2 < p.death_gi;
+  const bool a0 = (l0 >= p.met[0][0]) & (l1 >= p.met[0][1]) & q & !g1s;
+  const bool a1 = (l0 >= p.met[1][0]) & (l1 >= p.met[1][1]) & q & !g1s;
+  const bool a2 = (l0 >= p.met[2][0]) & (l1 >= p.met[2][1]) & d & rest;
+  const bool a3 = (l0 >= p.met[3][0]) & (l1 >= p.met[3][1]) & d & rest;
+  mode = a0 ? 0u : a1 ? 1u : a2 ? 2u : 3u;
+  return a0 | a1 | a2 | a3;
+}
+
+// cell.cu:72-82
 __device__ __forceinline__ bool update_state(DCell &c, float l0, float l1, float l2,
                                              const KParams &p, uint32_t vac) {
-  if (c.prolif >= c.t4 - p.dt_h) return false;
-  bool g1s = c.prolif > (c.t0 - p.dt2_h) && c.phase == 0 && vac <= 1;
-  if (!g1s) {
-    if (l0 >= p.met[0][0] && l1 >= p.met[0][1] && l2 < p.quiescence_gi) {
-      c.mode = 0;
-      return true;
-    } else if (l0 >= p.met[1][0] && l1 >= p.met[1][1] && l2 < p.quiescence_gi) {
-      c.mode = 1;
-      return true;
-    }
-  }
-  if (c.phase != 0 && c.phase != 2) return false;
-  if (l0 >= p.met[2][0] && l1 >= p.met[2][1] && l2 < p.death_gi) {
-    c.mode = 2;
-    return true;
-  } else if (l0 >= p.met[3][0] && l1 >= p.met[3][1] && l2 < p.death_gi) {
-    c.mode = 3;
-    return true;
-  }
-  return false;
+  const bool old = c.prolif >= c.t4 - p.dt_h;
+  const bool g1s = (c.prolif > (c.t0 - p.dt2_h)) & (c.phase == 0) & (vac <= 1);
+  uint32_t mode;
+  const bool alive =
+      !old & metabolic_mode(p, l0, l1, l2, g1s, (c.phase == 0) | (c.phase == 2), mode);
+  c.mode = alive ? mode : c.mode;
+  return alive;
+}
+
+// consumption of the cell's mode (a select chain: an indexed constant load
+// would replay for every mode of the warp)
+__device__ __forceinline__ float met_of(const KParams &p, uint32_t mode, int k) {
+  const float lo = mode == 0 ? p.met[0][k] : p.met[1][k];
+  const float hi = mode == 2 ? p.met[2][k] : p.met[3][k];
+  return mode < 2 ? lo : hi;
 }
 
 // cell.cu:84-91, :93-100
@@ -243,23 +253,21 @@ __device__ __forceinline__ void irradiate(DCell &c, float dose, const KParams &p
 
 // cell.cu:21-32
 __device__ __forceinline__ bool progress_clock(DCell &c, const KParams &p) {
-  if ((c.mode == 0 || c.mode == 1) && c.tir == 0) {
-    c.prolif += p.dt_h;
-    uint32_t cur = c.phase;
-    float tc = cur == 0 ? c.t0 : cur == 1 ? c.t1 : cur == 2 ? c.t2 : cur == 3 ? c.t3 : c.t4;
-    c.phase = cur + (c.prolif > tc ? 1u : 0u);
-    return c.phase != cur && c.phase != 4;
-  }
-  return false;
+  const bool adv = (c.mode < 2) & (c.tir == 0);
+  const float np = c.prolif + p.dt_h;
+  const uint32_t cur = c.phase;
+  const float tc = cur == 0 ? c.t0 : cur == 1 ? c.t1 : cur == 2 ? c.t2 : cur == 3 ? c.t3 : c.t4;
+  const bool next = adv & (np > tc);
+  c.prolif = adv ? np : c.prolif;
+  c.phase = cur + (next ? 1u : 0u);
+  return next & (c.phase != 4);
 }
 
 // cell.h:104-107: advance the repair clock; true if the survival decision fires
 __device__ __forceinline__ bool repair_pre(DCell &c, const KParams &p, bool cycle_changed) {
-  if (c.tir > 0 || (c.irr > 0 && cycle_changed)) {
-    c.tir += p.dt_h;
-    if (c.tir >= c.delay) return true;
-  }
-  return false;
+  const bool on = (c.tir > 0) | ((c.irr > 0) & cycle_changed);
+  c.tir = on ? c.tir + p.dt_h : c.tir;
+  return on & (c.tir >= c.delay);
 }
 
 __device__ __forceinline__ float death_prob(const DCell &c, const KParams &p) {

@@ -401,15 +401,22 @@ struct emt6_batch {
       occ_known = true;
     }
     const int *per_sm = per_sm_cache;
+    // A batch that is resident at once needs neither an order nor a queue: its
+    // CTAs all start together (four small launches less per chunk, which a
+    // recording pays for every step).
+    const bool resident = n <= (int64_t)std::min(per_sm[0], per_sm[1]) * sms;
+    if (resident) a.order = nullptr;
     uint32_t t = t_host;
     while (t < target) {
       const uint32_t end = (uint32_t)std::min<uint64_t>(target, (uint64_t)t + chunk);
       if (has_horizon && t >= max_horizon) break;
-      EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, stream));
-      *count += 3;
+      if (!resident) {
+        EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, stream));
+        *count += 3;
+      }
       for (int wide = 0; wide < 2; ++wide) {
         int grid = (int)std::min<int64_t>(n, 0x7fffffff);
-        if (sched == 1) {
+        if (sched == 1 && !resident) {
           grid = (int)std::min<int64_t>(n, (int64_t)per_sm[wide] * sms);
           EMT6_CUDA(cudaMemsetAsync(ticket.p, 0, sizeof(uint32_t), stream));
           a.queue = 1;

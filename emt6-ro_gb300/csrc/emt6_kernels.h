@@ -51,11 +51,11 @@ struct ResetArgs {
   int64_t nsims;
 };
 
-size_t run_kernel_smem(int HW, int lcap, bool wide);
+size_t run_kernel_smem(int H, int W, int lcap, bool wide);
 int max_ctas_per_sm(const KParams &p, bool wide);
 // Advance every simulation to step min(t_end, horizon).  wide = false runs the
-// narrow-region kernel (4 CTAs/SM), which stops a simulation at the first step
-// whose ROI is wider than 31 columns; wide = true finishes such simulations.
+// narrow-region kernel (6 CTAs/SM), which stops a simulation at the first step
+// whose region it cannot hold; wide = true finishes such simulations.
 cudaError_t launch_run(const RunArgs &a, uint32_t t_end, bool wide, int grid,
                        cudaStream_t stream);
 cudaError_t launch_reset(const ResetArgs &a, cudaStream_t stream);

@@ -1,0 +1,200 @@
+// emt6_tiles.cuh -- register tiles of the diffusion step, one warp per field.
+//
+// A warp holds one field's active block in registers for the whole step (23 +
+// 1 substeps): lane = 8 * bw + bl owns the C columns C*bl .. and the R rows
+// R*bw .. of an 8C x 4R tile.  Horizontal neighbours across lanes cost two
+// shuffles per row and lane, vertical ones two per column, so a lane's C x R
+// slots need 2 (C + R) shuffles per substep, and no warp waits for another
+// one inside a step.
+//
+// With H = x_left + x_right and G = b*x + d*H per site (fmaf(d, H, b*x)):
+//   x' = a*x + b*(H + x_up + x_down) + d*(H_up + H_down)
+//      = fmaf(a, x, fmaf(b, H, G_up + G_down))
+// so a site needs its own x and H and the G of the rows above and below: six
+// FP32 operations, one bit test (the last FFMA is predicated on the site's
+// free bit) and 2 (C + R) / (C R) shuffles.
+#pragma once
+#include <cstdint>
+
+#include "emt6_device.cuh"
+
+namespace emt6 {
+
+// How a region is laid on a tile (tile_mapping).  Tile row 0 / column 0 is
+// region row / column `off`; slots that hold no free site start at `fill`
+// (block mode: the external level) or at the region's own value.
+struct TileMap {
+  int tile;  // index of tile_shape, or -1
+  int off;   // 1: block mode (rows and columns 1..2d of an unclipped disc), 0: whole region
+  int xrow, xcol;  // block mode: the ROI's last row / column lies outside the tile
+};
+
+// C, R: columns and rows per lane.  RE / CE: the rows / columns may fill the
+// tile exactly, at the price of selects that replace what the rotating
+// shuffles bring round from the opposite edge; without them one spare row /
+// column of constant slots is what comes round.
+struct TileShape {
+  int C, R;
+  bool RE, CE;
+};
+// Ordered by slots per lane; a region takes the first one it fits.  Discs of
+// distance d (2d x 2d blocks) are what fills them: (2,3) d <= 6, (2,4) 7-8,
+// (3,5) 9-10, (3,6) 11-12, (4,7) 13-14, (4,8) 15-16, (5,9) 17-18, (5,10)
+// 19-20, (6,11) 21-22, (6,12) 23-24; the last two hold any other region of a
+// 54 x 60 interior.
+constexpr int kNumTiles = 20, kNarrowTiles = 12;
+__host__ __device__ constexpr TileShape tile_shape(int k) {
+  constexpr TileShape shapes[kNumTiles] = {
+      {1, 2, false, false}, {2, 3, true, false},   {2, 4, false, false}, {2, 4, true, true},
+      {3, 5, false, false}, {3, 5, true, false},   {3, 6, false, false}, {3, 6, true, true},
+      {4, 7, false, false}, {4, 7, true, false},   {4, 8, false, false}, {4, 8, true, true},
+      {5, 9, true, false},  {5, 10, false, false}, {5, 10, true, true},  {6, 11, true, false},
+      {6, 12, false, false}, {6, 12, true, true},  {7, 14, true, false}, {8, 14, true, false}};
+  return shapes[k];
+}
+// words of a field's slots for a tile's last row and column (8C + 4R)
+constexpr int kEdgeNarrow = 64, kEdgeWide = 120;
+
+template <int C, int R, bool RE, bool CE>
+__device__ __forceinline__ void diffuse_tile(float *__restrict__ f, const uint64_t *__restrict__ colmask,
+                                             float *__restrict__ edge, const TileMap &tm, int r0, int c0,
+                                             int h, int w, int W, float ext, float ca, float cb,
+                                             float cd, int nfree) {
+  const int lane = threadIdx.x & 31, bw = lane >> 3, bl = lane & 7;
+  const int left = (lane & 24) | ((bl + 7) & 7), right = (lane & 24) | ((bl + 1) & 7);
+  const int up = (lane + 24) & 31, dn = (lane + 8) & 31;
+  const int nrow = h + 2, ncol = w + 2, off = tm.off;
+  const float out = off ? ext : 0.f;  // sites beyond the tile
+  const int base = bw * R + off, j0 = bl * C + off;
+  const uint32_t rowsel = (1u << R) - 1u;
+  const uint32_t roirows = (uint32_t)(((((1ull << h) - 1ull) << 1)) >> base) & rowsel;
+  float *g = f + (r0 - 1 + base) * W + (c0 - 1 + j0);
+  uint32_t fm[C];  // free sites of the lane's columns
+  float X[R][C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    fm[c] = (j0 + c < ncol) ? (uint32_t)(colmask[j0 + c] >> base) & rowsel : 0u;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      float v = (base + i < nrow && j0 + c < ncol) ? ext : out;
+      if (fm[c] & (1u << i)) v = g[i * W + c];
+      X[i][c] = v;
+    }
+  }
+  const float gout = fmaf(cd, out + out, cb * out);
+  for (int s = 0; s <= nfree; ++s) {
+    if (s == nfree) {
+      // final substep: every site of the ROI
+#pragma unroll
+      for (int c = 0; c < C; ++c) fm[c] = (j0 + c >= 1 && j0 + c <= w) ? roirows : 0u;
+      if (RE && bw == 3) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) edge[C * bl + c] = X[R - 1][c];
+      }
+      if (CE && bl == 7) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) edge[8 * C + bw * R + i] = X[i][C - 1];
+      }
+    }
+    float lv[R], rv[R];
+    auto hshuffle = [&](int i) {
+      lv[i] = __shfl_sync(kFull, X[i][C - 1], left);
+      rv[i] = __shfl_sync(kFull, X[i][0], right);
+      if (CE) {
+        lv[i] = bl == 0 ? out : lv[i];
+        rv[i] = bl == 7 ? out : rv[i];
+      }
+    };
+    auto hsum = [&](int i, int c) -> float {
+      return (c == 0 ? lv[i] : X[i][c > 0 ? c - 1 : 0]) +
+             (c == C - 1 ? rv[i] : X[i][c < C - 1 ? c + 1 : 0]);
+    };
+    // the band's first and last rows first: their G crosses to other lanes.
+    // Tiles of up to 32 slots fetch every row's neighbours at once, larger
+    // ones a row ahead (their registers are taken by the tile).
+    constexpr bool AHEAD = C * R > 50;
+    hshuffle(0);
+    if (R > 1) hshuffle(R - 1);
+    if (!AHEAD) {
+#pragma unroll
+      for (int i = 1; i < R - 1; ++i) hshuffle(i);
+    } else if (R > 2) {
+      hshuffle(1);
+    }
+    float hb[C], gb[C], hc[C], gc[C], gm[C], gx[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      hc[c] = hsum(0, c);
+      gc[c] = fmaf(cd, hc[c], cb * X[0][c]);
+      hb[c] = hsum(R - 1, c);
+      gb[c] = fmaf(cd, hb[c], cb * X[R - 1][c]);
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      gm[c] = __shfl_sync(kFull, gb[c], up);  // the row above the band
+      gx[c] = __shfl_sync(kFull, gc[c], dn);  // the row below it
+      if (RE) {
+        gm[c] = bw == 0 ? gout : gm[c];
+        gx[c] = bw == 3 ? gout : gx[c];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (AHEAD && i + 2 < R - 1) hshuffle(i + 2 < R ? i + 2 : 0);
+      float hn[C], gn[C];
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        if (i + 1 == R) {
+          hn[c] = 0.f;
+          gn[c] = gx[c];
+        } else if (i + 1 == R - 1) {
+          hn[c] = hb[c];
+          gn[c] = gb[c];
+        } else {
+          hn[c] = hsum(i + 1 < R ? i + 1 : 0, c);
+          gn[c] = fmaf(cd, hn[c], cb * X[i + 1 < R ? i + 1 : 0][c]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const float t = fmaf(cb, hc[c], gm[c] + gn[c]);
+        if (fm[c] & (1u << i)) X[i][c] = fmaf(ca, X[i][c], t);
+        gm[c] = gc[c];
+        gc[c] = gn[c];
+        hc[c] = hn[c];
+      }
+    }
+  }
+  // the last substep's bits are the sites to store
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (fm[c] & (1u << i)) g[i * W + c] = X[i][c];
+  if (RE && (tm.xrow | tm.xcol)) {
+    // block mode with 2d = 4R rows (8C columns): the final substep of the
+    // ROI's last row (column) n = 2d + 1, outside the tile.  Every site there
+    // is fixed (x = ext) and so are its neighbours outside the tile; the
+    // tile's last row and column are those before the substep.
+    __syncwarp();
+    const int n = w;
+    const float gfix = fmaf(cd, ext + ext, cb * ext);  // G of an all-fixed row
+    float *q = f + (r0 - 1) * W + (c0 - 1);
+    if (tm.xrow)
+      for (int j = lane + 1; j <= n; j += 32) {  // (n, j)
+        const float xl = j >= 2 ? edge[j - 2] : ext, xc = j <= n - 1 ? edge[j - 1] : ext,
+                    xr = j <= n - 2 ? edge[j] : ext;
+        const float gu = fmaf(cd, xl + xr, cb * xc);
+        q[n * W + j] = fmaf(ca, ext, fmaf(cb, ext + ext, gu + gfix));
+      }
+    if (CE && tm.xcol)
+      for (int i = lane + 1; i <= n - 1; i += 32) {  // (i, n); (n, n) is with the row
+        const float xu = i >= 2 ? edge[8 * C + i - 2] : ext, xc = edge[8 * C + i - 1],
+                    xd = i <= n - 2 ? edge[8 * C + i] : ext;
+        const float gu = fmaf(cd, xu + ext, cb * ext), gd = fmaf(cd, xd + ext, cb * ext);
+        q[i * W + n] = fmaf(ca, ext, fmaf(cb, xc + ext, gu + gd));
+      }
+  }
+}
+
+}  // namespace emt6
