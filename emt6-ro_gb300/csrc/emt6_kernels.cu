@@ -62,7 +62,7 @@ constexpr int kWindowRows = 40;
 constexpr uint32_t kNarrowSmem = 44u * 1024u, kMinEntries = 1024;
 
 struct SmemLayout {
-  uint32_t fld, st, colmask, edge, misc, h0, h1, list, fl, total;
+  uint32_t fld, st, colmask, masks, edge, misc, h0, h1, list, fl, total;
   int rows, plane, entries;  // window rows, floats of a field's window, list capacity
 };
 
@@ -78,6 +78,7 @@ __host__ __device__ inline SmemLayout smem_layout(int H, int W, int lcap, bool w
   L.fld = o; o += align_up(3u * (uint32_t)L.plane, 32) * 4u;
   L.st = o; o += align_up((uint32_t)HW, 128);
   L.colmask = o; o += 64 * 8;
+  L.masks = o; o += 3u * (wide ? kWordsWide : kWordsNarrow) * 32u * 4u;
   L.edge = o; o += 3u * (wide ? kEdgeWide : kEdgeNarrow) * 4u;
   L.misc = o; o += align_up(sizeof(Misc), 16);
   L.entries = lcap;
@@ -299,9 +300,9 @@ __device__ void tile_mapping(const uint64_t *colmask, Misc *m, uint32_t layouts,
   m->nfs = nfs;
   int need = max(m->w0, 0);  // an empty region needs no other window
   const uint64_t ra = ((uint64_t)rhi << 32) | rlo, ca = ((uint64_t)chi << 32) | clo;
-  TileMap tm = {-1, 0, 0, 0};
+  TileMap tm = {-1, 1, 1, 0, 0, 0};
   if (h == 0 || w == 0) {
-    tm.tile = 0;
+    tm.tile = 0;  // never diffused
   } else {
     const uint32_t bit = d <= 16 ? kLayoutBands : kLayoutWideBands;
     const bool block = h == 2 * d + 1 && w == h && (layouts & bit) && !((ra | ca) & 1ull) &&
@@ -314,6 +315,8 @@ __device__ void tile_mapping(const uint64_t *colmask, Misc *m, uint32_t layouts,
       if (tm.tile < 0 && nr + (t.RE && exact ? 0 : 1) <= 4 * t.R &&
           nc + (t.CE && exact ? 0 : 1) <= 8 * t.C) {
         tm.tile = k;
+        tm.C = t.C;
+        tm.R = t.R;
         tm.off = block;
         tm.xrow = block && nr == 4 * t.R;
         tm.xcol = block && nc == 8 * t.C;
@@ -331,10 +334,35 @@ __device__ void tile_mapping(const uint64_t *colmask, Misc *m, uint32_t layouts,
   if (tm.tile < 0 || tm.tile >= tiles) m->park = 1;
 }
 
+// The slot bits of the region's tile (emt6_tiles.cuh), warp k builds kind k.
+template <bool WIDE>
+__device__ void build_masks(uint32_t *masks, const uint64_t *colmask, const Misc *m) {
+  constexpr int WORDS = WIDE ? kWordsWide : kWordsNarrow;
+  const int kind = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (kind > 2) return;
+  const int C = m->tm.C, R = m->tm.R, off = m->tm.off, h = m->roi[2], w = m->roi[3];
+  const int r0 = (lane >> 3) * R + off, c0 = (lane & 7) * C + off;
+  uint32_t bits = 0;
+  int q = 0;
+  for (int i = 0; i < R; ++i)
+    for (int c = 0; c < C; ++c) {
+      const int row = r0 + i, col = c0 + c;
+      bool on;
+      if (kind == kFreeBits) on = col < w + 2 && ((colmask[col] >> row) & 1ull);
+      else if (kind == kRoiBits) on = row >= 1 && row <= h && col >= 1 && col <= w;
+      else on = row < h + 2 && col < w + 2;
+      bits |= (on ? 1u : 0u) << slot_bit(q % 28);
+      if (++q % 28 == 0 || q == C * R) {
+        masks[(kind * WORDS + (q - 1) / 28) * 32 + lane] = bits;
+        bits = 0;
+      }
+    }
+}
+
 // One diffusion step of the region: warp w diffuses field w.  `fld` is the
 // window of rows from m->w0.
 template <bool WIDE>
-__device__ __forceinline__ void diffuse_step(float *fld, int plane, const uint64_t *colmask,
+__device__ __forceinline__ void diffuse_step(float *fld, int plane, const uint32_t *masks,
                                              float *edge, const Misc *m, const KParams &p) {
   const int h = m->roi[2], w = m->roi[3];
   if (h == 0 || w == 0) return;
@@ -349,7 +377,7 @@ __device__ __forceinline__ void diffuse_step(float *fld, int plane, const uint64
 #define EMT6_TILE(K)                                                                              \
   case K:                                                                                         \
     diffuse_tile<tile_shape(K).C, tile_shape(K).R, tile_shape(K).RE, tile_shape(K).CE>(           \
-        f, colmask, e, tm, r0, c0, h, w, p.W, ext, ca, cb, cd, p.nfree);                          \
+        f, masks, WIDE ? kWordsWide : kWordsNarrow, e, tm, r0, c0, w, p.W, ext, ca, cb, cd, p.nfree); \
     break;
   switch (tm.tile) {
     EMT6_TILE(0) EMT6_TILE(1) EMT6_TILE(2) EMT6_TILE(3) EMT6_TILE(4) EMT6_TILE(5)
@@ -657,6 +685,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
   const Hot hot = {reinterpret_cast<float *>(sm + L.h0), reinterpret_cast<float *>(sm + L.h1),
                    reinterpret_cast<uint16_t *>(sm + L.fl)};
   uint64_t *colmask = reinterpret_cast<uint64_t *>(sm + L.colmask);
+  uint32_t *masks = reinterpret_cast<uint32_t *>(sm + L.masks);
   float *edge = reinterpret_cast<float *>(sm + L.edge);
   Misc *m = reinterpret_cast<Misc *>(sm + L.misc);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -729,6 +758,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
         }
         if (wid == 0) tile_mapping(colmask, m, p.layouts, tiles, H, rows);
         __syncthreads();
+        if (WIDE || !m->park) build_masks<WIDE>(masks, colmask, m);
         const int w0 = m->w0, need = m->wneed;
         if (w0 != need) {
           // (another) window of the fields; a parked simulation needs none
@@ -740,8 +770,8 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
           } else if (tid == 0) {
             m->w0 = -1;
           }
-          __syncthreads();
         }
+        __syncthreads();
       }
       if (!WIDE && t == step0 && t % 32 != 0) {
         // between ROI updates cells may lie beyond the ROI, and beyond the
@@ -774,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
           list[e] = (uint16_t)(s | (vac << kSiteBits));
         }
       dirty = false;
-      diffuse_step<WIDE>(fld, plane, colmask, edge, m, p);
+      diffuse_step<WIDE>(fld, plane, masks, edge, m, p);
       // diffused site-substeps: free sites x free substeps + the final ROI pass
       if (tid == 0 && m->roi[2] > 0)
         m->diffused += m->nfs * (unsigned long long)p.nfree +
@@ -1168,6 +1198,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5)
   uint8_t *st = sm + L.st;
   uint16_t *list = reinterpret_cast<uint16_t *>(sm + L.list);
   uint64_t *colmask = reinterpret_cast<uint64_t *>(sm + L.colmask);
+  uint32_t *masks = reinterpret_cast<uint32_t *>(sm + L.masks);
   float *edge = reinterpret_cast<float *>(sm + L.edge);
   Misc *m = reinterpret_cast<Misc *>(sm + L.misc);
   for (int q = threadIdx.x; q < HW; q += NT) st[q] = gst ? gst[q] : 0;
@@ -1205,10 +1236,11 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5)
     }
     __syncthreads();
     if (!WIDE && m->park) return;
+    build_masks<WIDE>(masks, colmask, m);
     for (int q = threadIdx.x; q < 3 * L.plane; q += NT)
       fld[q] = gfld[q / L.plane * HW + m->w0 * p.W + q % L.plane];
     __syncthreads();
-    diffuse_step<WIDE>(fld, L.plane, colmask, edge, m, p);
+    diffuse_step<WIDE>(fld, L.plane, masks, edge, m, p);
     __syncthreads();
     for (int q = threadIdx.x; q < 3 * L.plane; q += NT)
       gfld[q / L.plane * HW + m->w0 * p.W + q % L.plane] = fld[q];
