@@ -292,7 +292,7 @@ struct emt6_batch {
   unsigned long long launches = 0;  // kernels issued by this handle
   bool use_graph = false;
   bool occ_known = false;
-  int per_sm_cache[2] = {1, 1};
+  int per_sm_cache[emt6::kTiers] = {1, 1, 1};
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_key[5] = {0, 0, 0, 0, 0};
   unsigned long long graph_kernels = 0;
@@ -396,15 +396,15 @@ struct emt6_batch {
     int sms = 0;
     EMT6_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     if (!occ_known) {
-      for (int wide = 0; wide < 2; ++wide)
-        per_sm_cache[wide] = std::max(emt6::max_ctas_per_sm(kp, wide != 0), 1);
+      for (int tier = 0; tier < emt6::kTiers; ++tier)
+        per_sm_cache[tier] = std::max(emt6::max_ctas_per_sm(kp, tier), 1);
       occ_known = true;
     }
     const int *per_sm = per_sm_cache;
     // A batch that is resident at once needs neither an order nor a queue: its
-    // CTAs all start together (four small launches less per chunk, which a
-    // recording pays for every step).
-    const bool resident = n <= (int64_t)std::min(per_sm[0], per_sm[1]) * sms;
+    // CTAs all start together, at the tier with the fewest per SM too (five
+    // launches less per chunk, which a recording pays for every step).
+    const bool resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierFull]) * sms;
     if (resident) a.order = nullptr;
     uint32_t t = t_host;
     while (t < target) {
@@ -414,14 +414,15 @@ struct emt6_batch {
         EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, stream));
         *count += 3;
       }
-      for (int wide = 0; wide < 2; ++wide) {
+      for (int tier = 0; tier < emt6::kTiers; ++tier) {
+        if (resident && tier == emt6::kTierWide) continue;
         int grid = (int)std::min<int64_t>(n, 0x7fffffff);
         if (sched == 1 && !resident) {
-          grid = (int)std::min<int64_t>(n, (int64_t)per_sm[wide] * sms);
+          grid = (int)std::min<int64_t>(n, (int64_t)per_sm[tier] * sms);
           EMT6_CUDA(cudaMemsetAsync(ticket.p, 0, sizeof(uint32_t), stream));
           a.queue = 1;
         }
-        EMT6_CUDA(emt6::launch_run(a, end, wide != 0, grid, stream));
+        EMT6_CUDA(emt6::launch_run(a, end, tier, grid, stream));
         *count += 1;
       }
       t = end;
@@ -448,8 +449,8 @@ struct emt6_batch {
       }
       // occupancy queries and attributes outside the capture
       if (!occ_known) {
-        for (int wide = 0; wide < 2; ++wide)
-          per_sm_cache[wide] = std::max(emt6::max_ctas_per_sm(kp, wide != 0), 1);
+        for (int tier = 0; tier < emt6::kTiers; ++tier)
+          per_sm_cache[tier] = std::max(emt6::max_ctas_per_sm(kp, tier), 1);
         occ_known = true;
       }
       EMT6_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));

@@ -6,8 +6,8 @@
 // stay in global memory, where the few hundred live cells of each resident
 // simulation stay L2-resident.  Two kernels: run_kernel<false> (5 CTAs/SM, a
 // window of at most 40 lattice rows on chip) for regions that fit a tile of 32
-// slots per lane, and run_kernel<true> (4 CTAs/SM, the whole lattice) for
-// larger ones.  Per step (reference cadence,
+// slots per lane, and run_kernel<true> (4 CTAs/SM, the whole lattice; 3 CTAs/SM
+// for lists longer than 1,500 entries) for larger ones.  Per step (reference cadence,
 // src/emt6ro/simulation/simulation.cu:153-166):
 //   t % 128 == 0  rebuild the occupied list        (simulation.cu:41-64)
 //   t % 32  == 0  ROI + circular fixed-value mask   (diffusion.cu:65-100)
@@ -54,20 +54,24 @@ struct Misc {
 
 __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
-// Rows of the field window and entries of the occupied list on chip.  The wide
-// kernel holds the whole lattice.  The narrow one holds the region's rows (35
-// at most) with room to move, and as many list entries as leave 5 CTAs on an
-// SM (44 KB each): fewer rows or entries would only park simulations.
+// Rows of the field window and entries of the occupied list on chip, by tier of
+// launch.  kTierNarrow holds the region's rows (35 at most) with room to move, and
+// as many list entries as leave 5 CTAs on an SM; fewer rows or entries would
+// only park simulations.  kTierWide holds the whole lattice and the entries that
+// leave 4 CTAs (12 warps, 3 on each quarter of the SM; with 3 CTAs one quarter
+// has 3 warps and the CTAs wait for it: 23% slower diffusion); longer lists are
+// kTierFull's, 3 CTAs.
 constexpr int kWindowRows = 40;
-constexpr uint32_t kNarrowSmem = 44u * 1024u, kMinEntries = 1024;
+constexpr uint32_t kEntryBytes = 4 + 4 + 2 + 1, kMinEntries = 1024;
 
 struct SmemLayout {
   uint32_t fld, st, colmask, masks, edge, misc, h0, h1, list, fl, total;
   int rows, plane, entries;  // window rows, floats of a field's window, list capacity
 };
 
-__host__ __device__ inline SmemLayout smem_layout(int H, int W, int lcap, bool wide) {
+__host__ __device__ inline SmemLayout smem_layout(int H, int W, int lcap, int tier) {
   SmemLayout L;
+  const bool wide = tier != kTierNarrow;
   const int HW = H * W;
   L.rows = wide || H < kWindowRows ? H : kWindowRows;
   L.plane = L.rows * W;
@@ -81,22 +85,26 @@ __host__ __device__ inline SmemLayout smem_layout(int H, int W, int lcap, bool w
   L.masks = o; o += 3u * (wide ? kWordsWide : kWordsNarrow) * 32u * 4u;
   L.edge = o; o += 3u * (wide ? kEdgeWide : kEdgeNarrow) * 4u;
   L.misc = o; o += align_up(sizeof(Misc), 16);
-  L.entries = lcap;
-  if (!wide) {
-    const uint32_t left = o < kNarrowSmem ? (kNarrowSmem - o) / 12u : 0u;
+  // a rebuilt list holds at most the interior, and 128 divisions can follow
+  L.entries = lcap - 128;
+  if (tier != kTierFull) {
+    const uint32_t room = tier == kTierNarrow ? 44u * 1024u : 55u * 1024u + 512u;
+    const uint32_t left = o < room ? (room - o) / kEntryBytes : 0u;
     const uint32_t fit = left > kMinEntries ? left : kMinEntries;
-    if (fit < (uint32_t)lcap) L.entries = (int)fit;
+    if (fit < (uint32_t)L.entries) L.entries = (int)fit;
   }
-  L.h0 = o; o += align_up((uint32_t)L.entries * 4u, 16);
-  L.h1 = o; o += align_up((uint32_t)L.entries * 4u, 16);
-  L.list = o; o += align_up((uint32_t)L.entries * 2u, 16);
-  L.fl = o; o += align_up((uint32_t)L.entries * 2u, 16);
+  L.entries &= ~15;  // keeps the arrays aligned
+  if (tier == kTierFull) L.entries = (lcap - 128 + 15) & ~15;
+  L.h0 = o; o += (uint32_t)L.entries * 4u;
+  L.h1 = o; o += (uint32_t)L.entries * 4u;
+  L.list = o; o += (uint32_t)L.entries * 2u;
+  L.fl = o; o += (uint32_t)L.entries;
   L.total = o;
   return L;
 }
 
-size_t run_kernel_smem(int H, int W, int lcap, bool wide) {
-  return smem_layout(H, W, lcap, wide).total;
+size_t run_kernel_smem(int H, int W, int lcap, int tier) {
+  return smem_layout(H, W, lcap, tier).total;
 }
 
 // list entries on chip: site index in the low bits, vacant neighbours above
@@ -513,14 +521,24 @@ __device__ __noinline__ bool step_site(const KParams &p, float *lv, int plane, u
 //     kG (with kT): the G1/S check's clock condition.
 //   kSlow: any other record (stepped from global memory)
 //   kGone: no cell, or a site listed more than once (stepped in list order)
-// Entries of class kSlow and kGone hold ready | occurrence in the high byte.
+// Entries of class kSlow and kGone have, in h0's place, kReady | occurrence of
+// a cell that is ready to divide, or 0.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kT = 32u, kG = 64u, kOld = 128u, kReady = 0x8000u;
+constexpr uint32_t kT = 32u, kG = 64u, kOld = 128u, kReady = 0x100u;
 constexpr uint32_t kClass = 7u << 2, kSlow = 6u << 2, kGone = 7u << 2;
 
 struct Hot {
   float *h0, *h1;
-  uint16_t *fl;
+  uint8_t *fl;
+  __device__ __forceinline__ void idle(uint32_t e, uint32_t cls, uint32_t ready) const {
+    fl[e] = (uint8_t)cls;
+    h0[e] = __uint_as_float(ready);
+  }
+  // kReady | occurrence of a cell that is ready to divide, else 0
+  __device__ __forceinline__ uint32_t ready(uint32_t e) const {
+    const uint32_t cls = fl[e] & kClass;
+    return cls < kSlow ? (cls == 16u ? kReady : 0u) : __float_as_uint(h0[e]);
+  }
 };
 
 __device__ __forceinline__ void classify(const KParams &p, const DCell &c, const Hot &h, uint32_t e) {
@@ -528,21 +546,23 @@ __device__ __forceinline__ void classify(const KParams &p, const DCell &c, const
   const float lim = c.t4 - p.dt_h;
   const bool old = c.prolif >= lim;
   uint32_t f = kSlow;
+  float h0 = 0.f;
   if (c.mode <= 3 && c.phase <= 4) {
     if (c.tir == 0) {
       // (the G1/S check reads the end of phase 0 itself)
       if (c.phase != 0 || tc <= lim) {
         f = c.mode | (c.phase << 2) | (old ? kOld : 0u);
-        h.h0[e] = c.prolif;
+        h0 = c.prolif;
         h.h1[e] = fminf(tc, lim);
       }
     } else if (!old) {
       f = c.mode | (c.phase << 2) | kT | (c.prolif > c.t0 - p.dt2_h ? kG : 0u);
-      h.h0[e] = c.tir;
+      h0 = c.tir;
       h.h1[e] = c.delay;
     }
   }
-  h.fl[e] = (uint16_t)f;
+  h.h0[e] = h0;
+  h.fl[e] = (uint8_t)f;
 }
 
 // the cell of a hot entry, its clock and flags merged into the global record
@@ -583,7 +603,7 @@ __device__ __noinline__ void gather_cells(const KParams &p, const uint8_t *st, c
       const uint32_t e = e0 + u * NT;
       if (e >= n) break;
       if (on[u]) classify(p, c[u], h, e);
-      else h.fl[e] = (uint16_t)kGone;
+      else h.idle(e, kGone, 0);
     }
   }
 }
@@ -624,10 +644,10 @@ __device__ __noinline__ bool cell_event(const KParams &p, Misc *m, float4 *rec, 
   store_clocks(rec, c);
   if (dead) {
     *st = (*st & ~kStMask) | kVacant;
-    h.fl[e] = (uint16_t)kGone;
+    h.idle(e, kGone, 0);
   } else {
     classify(p, c, h, e);
-    if (c.phase == 4 && h.fl[e] == kSlow) h.fl[e] = (uint16_t)(kSlow | kReady);
+    if (c.phase == 4 && h.fl[e] == kSlow) h.idle(e, kSlow, kReady);
   }
   return dead;
 }
@@ -642,11 +662,11 @@ __device__ __noinline__ uint32_t step_entry(const KParams &p, Misc *m, float *lv
   bool died;
   const bool ready = step_site(p, lv, plane, st, rec, s, vac, dose, t, sim, 0, epoch, m, &died);
   if (died) {
-    h.fl[e] = (uint16_t)kGone;
+    h.idle(e, kGone, 0);
     return 2u;
   }
   classify(p, load_cell(rec), h, e);
-  if (ready && (h.fl[e] & kClass) == kSlow) h.fl[e] = (uint16_t)(kSlow | kReady);
+  if (ready && h.fl[e] == kSlow) h.idle(e, kSlow, kReady);
   return ready ? 1u : 0u;
 }
 
@@ -671,19 +691,20 @@ __device__ __forceinline__ uint32_t occurrence(const uint16_t *list, const uint8
 // WIDE = false: regions that fit a tile of at most 32 slots per lane (discs up
 // to distance 16, clipped regions up to 32 x 32), 5 CTAs/SM.  A simulation it
 // cannot hold (region, window or list) is parked at the start of that step for
-// the WIDE = true kernel: any region, 4 CTAs/SM.
+// the WIDE = true kernel: any region, 4 CTAs/SM (3 as kTierFull).
 template <bool WIDE>
-__global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __grid_constant__ RunArgs a, uint32_t t_end) {
+__global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __grid_constant__ RunArgs a, uint32_t t_end, int tier) {
   constexpr int NT = kThreads;
   extern __shared__ __align__(16) uint8_t sm[];
   const KParams &p = a.p;
   const int H = p.H, W = p.W, HW = p.HW;
-  const SmemLayout L = smem_layout(H, W, p.lcap, WIDE);
+  const SmemLayout L = smem_layout(H, W, p.lcap, WIDE ? tier : kTierNarrow);
+  const bool last = WIDE && tier == kTierFull;  // holds every simulation
   float *fld = reinterpret_cast<float *>(sm + L.fld);
   uint8_t *st = sm + L.st;
   uint16_t *list = reinterpret_cast<uint16_t *>(sm + L.list);
   const Hot hot = {reinterpret_cast<float *>(sm + L.h0), reinterpret_cast<float *>(sm + L.h1),
-                   reinterpret_cast<uint16_t *>(sm + L.fl)};
+                   sm + L.fl};
   uint64_t *colmask = reinterpret_cast<uint64_t *>(sm + L.colmask);
   uint32_t *masks = reinterpret_cast<uint32_t *>(sm + L.masks);
   float *edge = reinterpret_cast<float *>(sm + L.edge);
@@ -711,7 +732,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
     // nothing to do for a simulation already at its target step
     if (step0 >= t_stop) continue;
     const int4 meta = a.meta[sim];
-    if (!WIDE && meta.x >= L.entries) continue;  // the list does not fit: the wide kernel's
+    if (!last && meta.x >= L.entries) continue;  // the list does not fit: a later tier's
 
     // ---- load the simulation into shared memory (its fields when the window
     //      is known) ----
@@ -758,13 +779,13 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
         }
         if (wid == 0) tile_mapping(colmask, m, p.layouts, tiles, H, rows);
         __syncthreads();
-        if (WIDE || !m->park) build_masks<WIDE>(masks, colmask, m);
+        if (last || !m->park) build_masks<WIDE>(masks, colmask, m);
         const int w0 = m->w0, need = m->wneed;
         if (w0 != need) {
           // (another) window of the fields; a parked simulation needs none
           if (w0 >= 0) store_window<NT>(fld, gfld, w0, plane, W, HW, a.fstride);
           __syncthreads();
-          if (WIDE || !m->park) {
+          if (last || !m->park) {
             load_window<NT>(fld, gfld, need, plane, W, HW, a.fstride);
             if (tid == 0) m->w0 = need;
           } else if (tid == 0) {
@@ -783,10 +804,10 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
         }
         __syncthreads();
       }
-      // a simulation this kernel cannot hold is left for the wide one; the
+      // a simulation this launch cannot hold is left for a later tier; the
       // state stored is the state at the start of step t (the list rebuild and
       // ROI above are recomputed identically there)
-      if (!WIDE && (m->park || m->n >= (uint32_t)L.entries)) break;
+      if (!last && (m->park || m->n >= (uint32_t)L.entries)) break;
       const uint32_t n = m->n;
       const int fo = m->w0 * W;
       if (!onchip) gather_cells<NT>(p, st, list, cells, hot, n);
@@ -850,14 +871,13 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
             lv[plane] = l1 - met_of(p, mode, 1);
             lv[2 * plane] = l2 - met_of(p, mode, 2);
             if (moves) hot.h0[e] = next;
-            if (mode != (f & 3u)) hot.fl[e] = (uint16_t)((f & ~3u) | mode);
+            if (mode != (f & 3u)) hot.fl[e] = (uint8_t)((f & ~3u) | mode);
           }
           bool ready = alive & (cls == 16);
           if (!alive | (moves & (next >= thr))) {
             const bool died = cell_event(p, m, cells + 3 * s, st + s, hot, e, alive, s, t,
                                          (uint32_t)sim, a.epoch);
-            const uint32_t g = hot.fl[e];
-            ready = (g & kClass) == 16u || (g & (kClass | kReady)) == (kSlow | kReady);
+            ready = hot.ready(e) != 0;
             may_divide |= died;
           }
           may_divide |= ready & (vac != 0);
@@ -877,7 +897,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
             const uint32_t occ = occurrence(list, st, ee, n0);
             if (lane == 0) {
               const int s = list[ee] & kSiteMask;
-              uint32_t res = kGone;
+              uint32_t res = 0;
               if ((st[s] & kStMask) == kOccupied) {
                 const uint32_t vac = list[ee] >> kSiteBits;
                 bool died;
@@ -885,11 +905,11 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
                                              dose, t, (uint32_t)sim, occ, a.epoch, m, &died);
                 if (ready) {
                   if (occ > 127) atomicOr(a.err, 4u);
-                  res = kGone | kReady | ((occ & 0x7fu) << 8);
+                  res = kReady | (occ & 0x7fu);
                 }
                 may_divide |= (ready & (vac != 0)) | died;
               }
-              hot.fl[ee] = (uint16_t)res;
+              hot.idle(ee, kGone, res);
             }
             __syncwarp();
           }
@@ -902,10 +922,8 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
       // ---- division arbitration: lowest list index with a vacant target ----
       int best = 0x7fffffff, best_target = -1;
       for (uint32_t e = tid; e < n; e += NT) {
-        const uint32_t f = hot.fl[e];
-        if ((f & kClass) < kSlow ? (f & kClass) == 16u : (f & kReady) != 0) {
-          // occurrence of a site listed more than once
-          const uint32_t occ = (f & kClass) == kGone ? (f >> 8) & 0x7fu : 0u;
+        const uint32_t ready = hot.ready(e);
+        if (ready) {
           const int s = list[e] & kSiteMask;
           // a cell none of whose neighbours is vacant now cannot divide,
           // whatever the draw: skip the draw (interior cells stay ready)
@@ -918,7 +936,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
                             ((st[s + W] & kStMask) == kVacant) |
                             ((st[s + W + 1] & kStMask) == kVacant);
           if (!open) continue;
-          const float u = u01(draw(p, t, (uint32_t)sim, (uint32_t)s, occ, 0, a.epoch).x);
+          const float u = u01(draw(p, t, (uint32_t)sim, (uint32_t)s, ready & 0x7fu, 0, a.epoch).x);
           const int tg = choose_neighbour(s, W, u);
           if ((st[tg] & kStMask) == kVacant) {
             best = (int)e;
@@ -970,7 +988,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
           if (m->n < (uint32_t)L.entries) {
             const uint32_t ce = m->n++;
             list[ce] = (uint16_t)child;
-            if (listed) hot.fl[ce] = (uint16_t)kGone;
+            if (listed) hot.idle(ce, kGone, 0);
             else classify(p, cc, hot, ce);
           } else {
             atomicOr(a.err, 1u);
@@ -982,7 +1000,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
     }
 
     // ---- write the simulation back (nothing changed when the first step parks) ----
-    if (!WIDE && t == step0) {
+    if (!last && t == step0) {
       __syncthreads();
       continue;
     }
@@ -1193,7 +1211,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5)
   constexpr int NT = kThreads;
   extern __shared__ __align__(16) uint8_t sm[];
   const int HW = p.HW;
-  const SmemLayout L = smem_layout(p.H, p.W, p.lcap, WIDE);
+  const SmemLayout L = smem_layout(p.H, p.W, p.lcap, WIDE ? kTierFull : kTierNarrow);
   float *fld = reinterpret_cast<float *>(sm + L.fld);
   uint8_t *st = sm + L.st;
   uint16_t *list = reinterpret_cast<uint16_t *>(sm + L.list);
@@ -1268,15 +1286,14 @@ static cudaError_t ensure_smem(bool wide, size_t smem) {
   return e;
 }
 
-cudaError_t launch_run(const RunArgs &a, uint32_t t_end, bool wide, int grid,
-                       cudaStream_t stream) {
-  const size_t smem = run_kernel_smem(a.p.H, a.p.W, a.p.lcap, wide);
-  cudaError_t e = ensure_smem(wide, smem);
+cudaError_t launch_run(const RunArgs &a, uint32_t t_end, int tier, int grid, cudaStream_t stream) {
+  const size_t smem = run_kernel_smem(a.p.H, a.p.W, a.p.lcap, tier);
+  cudaError_t e = ensure_smem(tier != kTierNarrow, smem);
   if (e != cudaSuccess) return e;
-  if (wide)
-    run_kernel<true><<<grid, kThreads, smem, stream>>>(a, t_end);
+  if (tier != kTierNarrow)
+    run_kernel<true><<<grid, kThreads, smem, stream>>>(a, t_end, tier);
   else
-    run_kernel<false><<<grid, kThreads, smem, stream>>>(a, t_end);
+    run_kernel<false><<<grid, kThreads, smem, stream>>>(a, t_end, tier);
   return cudaGetLastError();
 }
 
@@ -1300,8 +1317,9 @@ cudaError_t launch_reset(const ResetArgs &a, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-int max_ctas_per_sm(const KParams &p, bool wide) {
-  const size_t smem = run_kernel_smem(p.H, p.W, p.lcap, wide);
+int max_ctas_per_sm(const KParams &p, int tier) {
+  const bool wide = tier != kTierNarrow;
+  const size_t smem = run_kernel_smem(p.H, p.W, p.lcap, tier);
   int n = 0;
   if (ensure_smem(wide, smem) != cudaSuccess) return 0;
   if (wide) {
@@ -1414,7 +1432,7 @@ cudaError_t launch_test_block(const KParams &p, int mode, bool wide, float *fld,
                               const uint8_t *st, int32_t *roi, uint8_t *mask, uint16_t *list,
                               uint32_t *n) {
   wide = wide || mode < 2;  // lists and ROIs of any size
-  const size_t smem = run_kernel_smem(p.H, p.W, p.lcap, wide);
+  const size_t smem = run_kernel_smem(p.H, p.W, p.lcap, wide ? kTierFull : kTierNarrow);
   cudaError_t e;
   if (wide) {
     e = cudaFuncSetAttribute(test_block_kernel<true>,

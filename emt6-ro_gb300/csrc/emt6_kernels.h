@@ -51,13 +51,15 @@ struct ResetArgs {
   int64_t nsims;
 };
 
-size_t run_kernel_smem(int H, int W, int lcap, bool wide);
-int max_ctas_per_sm(const KParams &p, bool wide);
-// Advance every simulation to step min(t_end, horizon).  wide = false runs the
-// narrow-region kernel (6 CTAs/SM), which stops a simulation at the first step
-// whose region it cannot hold; wide = true finishes such simulations.
-cudaError_t launch_run(const RunArgs &a, uint32_t t_end, bool wide, int grid,
-                       cudaStream_t stream);
+// Tiers of a step launch, in this order: each takes the simulations that the
+// ones before left short of the target step (regions too wide, lists too long
+// for the shared memory that lets 5 or 4 CTAs share an SM).  kTierFull holds any;
+// kTierWide may be skipped.
+enum { kTierNarrow = 0, kTierWide = 1, kTierFull = 2, kTiers = 3 };
+size_t run_kernel_smem(int H, int W, int lcap, int tier);
+int max_ctas_per_sm(const KParams &p, int tier);
+// Advance the simulations that `tier` holds to step min(t_end, horizon).
+cudaError_t launch_run(const RunArgs &a, uint32_t t_end, int tier, int grid, cudaStream_t stream);
 cudaError_t launch_reset(const ResetArgs &a, cudaStream_t stream);
 // simulations sorted largest region first into out[0 .. a.nsims) for the
 // launches of a chunk ending at t_end; hist holds kOrderKeys counters
