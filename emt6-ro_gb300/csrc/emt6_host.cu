@@ -292,7 +292,8 @@ struct emt6_batch {
   unsigned long long launches = 0;  // kernels issued by this handle
   bool use_graph = false;
   bool occ_known = false;
-  int per_sm_cache[emt6::kTiers] = {1, 1, 1};
+  bool resident = false;
+  int sms = 0, per_sm[emt6::kTiers] = {1, 1, 1};
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_key[5] = {0, 0, 0, 0, 0};
   unsigned long long graph_kernels = 0;
@@ -303,7 +304,10 @@ struct emt6_batch {
   DevBuf<float4> cell, tpl_cell;
   DevBuf<uint16_t> list;
   DevBuf<int4> meta;
-  DevBuf<int32_t> roi, sim_tumor, sim_protocol;
+  DevBuf<int32_t> roi, sim_tumor, sim_protocol, tpl_roi;
+  DevBuf<uint8_t> tier;  // per chunk: the launch tier of each simulation
+  cudaStream_t side[2] = {nullptr, nullptr};  // the wide tiers', beside `stream`
+  cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
   DevBuf<uint32_t> step, horizon, counts, err, ticket, order_hist;
   DevBuf<int64_t> order;  // per chunk: simulations by region, largest first
   DevBuf<unsigned long long> diffused;
@@ -314,6 +318,12 @@ struct emt6_batch {
       DeviceGuard g(device);
       cudaStreamSynchronize(stream);
       if (graph_exec) cudaGraphExecDestroy(graph_exec);
+      for (int k = 0; k < 2; ++k) {
+        if (side[k]) cudaStreamSynchronize(side[k]);
+        if (join[k]) cudaEventDestroy(join[k]);
+        if (side[k]) cudaStreamDestroy(side[k]);
+      }
+      if (fork) cudaEventDestroy(fork);
       cudaStreamDestroy(stream);
     }
   }
@@ -342,6 +352,7 @@ struct emt6_batch {
     a.queue = 0;
     a.ticket = ticket.p;
     a.order = order.p;
+    a.tier_of = nullptr;
     return a;
   }
 
@@ -375,6 +386,7 @@ struct emt6_batch {
     r.tpl_fld = tpl_fld.p;
     r.tpl_st = tpl_st.p;
     r.tpl_cell = tpl_cell.p;
+    r.tpl_roi = tpl_roi.p;
     r.sim_tumor = sim_tumor.p;
     r.fstride = fstride;
     r.sstride = sstride;
@@ -390,40 +402,76 @@ struct emt6_batch {
     return EMT6_OK;
   }
 
+  // Occupancy, kernel attributes, side streams and events of issue(): once, and
+  // outside any capture.
+  int prepare_launch() {
+    if (occ_known) return EMT6_OK;
+    EMT6_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    for (int tier = 0; tier < emt6::kTiers; ++tier)
+      per_sm[tier] = std::max(emt6::max_ctas_per_sm(kp, tier), 1);
+    // A batch that is resident at once needs neither an order nor a queue: its
+    // CTAs all start together, at the tier with the fewest per SM too.
+    resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierFull]) * sms;
+    if (!resident) {
+      for (int k = 0; k < 2; ++k) {
+        EMT6_CUDA(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
+        EMT6_CUDA(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming));
+      }
+      EMT6_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    }
+    occ_known = true;
+    return EMT6_OK;
+  }
+
+  int launch(emt6::RunArgs a, uint32_t end, int tier, cudaStream_t st, unsigned long long *count) {
+    int grid = (int)std::min<int64_t>(n, 0x7fffffff);
+    if (sched == 1 && !resident) {
+      grid = (int)std::min<int64_t>(n, (int64_t)per_sm[tier] * sms);
+      a.queue = 1;
+      a.ticket = ticket.p + (a.tier_of ? tier : emt6::kTiers);
+    }
+    EMT6_CUDA(emt6::launch_run(a, end, tier, grid, st));
+    *count += 1;
+    return EMT6_OK;
+  }
+
   // launches of one run() call from t_host to target, on the handle's stream
   int issue(uint32_t target, unsigned long long *count) {
     emt6::RunArgs a = run_args();
-    int sms = 0;
-    EMT6_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    if (!occ_known) {
-      for (int tier = 0; tier < emt6::kTiers; ++tier)
-        per_sm_cache[tier] = std::max(emt6::max_ctas_per_sm(kp, tier), 1);
-      occ_known = true;
-    }
-    const int *per_sm = per_sm_cache;
-    // A batch that is resident at once needs neither an order nor a queue: its
-    // CTAs all start together, at the tier with the fewest per SM too (five
-    // launches less per chunk, which a recording pays for every step).
-    const bool resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierFull]) * sms;
-    if (resident) a.order = nullptr;
     uint32_t t = t_host;
     while (t < target) {
       const uint32_t end = (uint32_t)std::min<uint64_t>(target, (uint64_t)t + chunk);
       if (has_horizon && t >= max_horizon) break;
-      if (!resident) {
-        EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, stream));
-        *count += 3;
-      }
-      for (int tier = 0; tier < emt6::kTiers; ++tier) {
-        if (resident && tier == emt6::kTierWide) continue;
-        int grid = (int)std::min<int64_t>(n, 0x7fffffff);
-        if (sched == 1 && !resident) {
-          grid = (int)std::min<int64_t>(n, (int64_t)per_sm[tier] * sms);
-          EMT6_CUDA(cudaMemsetAsync(ticket.p, 0, sizeof(uint32_t), stream));
-          a.queue = 1;
+      if (resident) {
+        a.order = nullptr;
+        for (int tier : {emt6::kTierNarrow, emt6::kTierFull}) {
+          const int rc = launch(a, end, tier, stream, count);
+          if (rc) return rc;
         }
-        EMT6_CUDA(emt6::launch_run(a, end, tier, grid, stream));
-        *count += 1;
+      } else {
+        // The tiers side by side, the largest simulations' first, each on the
+        // simulations expected to fit it: three launches in a row would leave
+        // most SMs idle at the end of each.  What outgrows its tier meanwhile is
+        // finished by the last launch.
+        EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, tier.p, stream));
+        *count += 3;
+        if (sched == 1)
+          EMT6_CUDA(cudaMemsetAsync(ticket.p, 0, (emt6::kTiers + 1) * sizeof(uint32_t), stream));
+        EMT6_CUDA(cudaEventRecord(fork, stream));
+        emt6::RunArgs b = a;
+        b.tier_of = tier.p;
+        const int order_of[2] = {emt6::kTierFull, emt6::kTierWide};
+        for (int k = 0; k < 2; ++k) {
+          EMT6_CUDA(cudaStreamWaitEvent(side[k], fork, 0));
+          const int rc = launch(b, end, order_of[k], side[k], count);
+          if (rc) return rc;
+          EMT6_CUDA(cudaEventRecord(join[k], side[k]));
+        }
+        int rc = launch(b, end, emt6::kTierNarrow, stream, count);
+        if (rc) return rc;
+        for (int k = 0; k < 2; ++k) EMT6_CUDA(cudaStreamWaitEvent(stream, join[k], 0));
+        rc = launch(a, end, emt6::kTierFull, stream, count);
+        if (rc) return rc;
       }
       t = end;
     }
@@ -433,6 +481,10 @@ struct emt6_batch {
   int run(uint32_t nsteps) {
     const uint64_t target64 = (uint64_t)t_host + nsteps;
     const uint32_t target = target64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)target64;
+    {
+      const int rc = prepare_launch();
+      if (rc) return rc;
+    }
     if (!use_graph) {
       int rc = issue(target, &launches);
       if (rc) return rc;
@@ -446,12 +498,6 @@ struct emt6_batch {
       if (graph_exec) {
         cudaGraphExecDestroy(graph_exec);
         graph_exec = nullptr;
-      }
-      // occupancy queries and attributes outside the capture
-      if (!occ_known) {
-        for (int tier = 0; tier < emt6::kTiers; ++tier)
-          per_sm_cache[tier] = std::max(emt6::max_ctas_per_sm(kp, tier), 1);
-        occ_known = true;
       }
       EMT6_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
       unsigned long long nodes = 0;
@@ -539,6 +585,34 @@ __global__ void summary_kernel(const float *fld, uint32_t fstride, const uint8_t
     }
     __syncthreads();
   }
+}
+
+// ROI (diffusion.cu:16-63) and cell count of a tumour: the launch order and
+// tiers of simulations that have not taken a step yet
+void template_roi(const uint8_t *st, int H, int W, int32_t roi[8]) {
+  int lo_r = H, lo_c = W, hi_r = 0, hi_c = 0, cells = 0;
+  for (int r = 0; r < H; ++r)
+    for (int c = 0; c < W; ++c)
+      if (st[r * W + c] == 1) {
+        lo_r = std::min(lo_r, r);
+        lo_c = std::min(lo_c, c);
+        hi_r = std::max(hi_r, r);
+        hi_c = std::max(hi_c, c);
+        ++cells;
+      }
+  if (!cells) return;
+  const int mr = lo_r + (hi_r - lo_r + 1) / 2, mc = lo_c + (hi_c - lo_c + 1) / 2;
+  int far = 0;
+  for (int r = lo_r; r <= hi_r; ++r)
+    for (int c = lo_c; c <= hi_c; ++c)
+      if (st[r * W + c] == 1) far = std::max(far, (mr - r) * (mr - r) + (mc - c) * (mc - c));
+  const int d = (int)std::ceil(std::sqrt((double)far));
+  roi[0] = mr <= d ? 1 : mr - d;
+  roi[1] = mc <= d ? 1 : mc - d;
+  roi[2] = mr + d >= H - 1 ? H - 1 - roi[0] : mr + d - roi[0] + 1;
+  roi[3] = mc + d >= W - 1 ? W - 1 - roi[1] : mc + d - roi[1] + 1;
+  roi[4] = d;
+  roi[5] = cells;
 }
 
 void site_to_records(const emt6_site &s, float *fld3, uint8_t *stv, float4 *cell3) {
@@ -772,7 +846,7 @@ int emt6_batch_create(const emt6_params *p, const emt6_site *tumors, int32_t n_t
   EMT6_CUDA(b->sim_tumor.alloc((size_t)n_sims));
   EMT6_CUDA(b->sim_protocol.alloc((size_t)n_sims));
   EMT6_CUDA(b->err.alloc(1));
-  EMT6_CUDA(b->ticket.alloc(1));
+  EMT6_CUDA(b->ticket.alloc(emt6::kTiers + 1));
   EMT6_CUDA(b->diffused.alloc(1));
   EMT6_CUDA(b->doses.alloc((size_t)n_protocols * std::max<uint32_t>(protocol_bins, 1)));
   EMT6_CUDA(b->tpl_fld.alloc((size_t)n_tumors * b->fstride));
@@ -792,6 +866,11 @@ int emt6_batch_create(const emt6_params *p, const emt6_site *tumors, int32_t n_t
         site_to_records(tumors[t * HW + q], f3, &hs[t * b->sstride + q], &hc[(t * HW + q) * 3]);
         for (int k = 0; k < 3; ++k) hf[t * b->fstride + k * HW + q] = f3[k];
       }
+    std::vector<int32_t> hr((size_t)n_tumors * 8, 0);
+    for (int32_t t = 0; t < n_tumors; ++t)
+      template_roi(&hs[(size_t)t * b->sstride], height, width, &hr[(size_t)t * 8]);
+    EMT6_CUDA(b->tpl_roi.alloc(hr.size()));
+    EMT6_CUDA(cudaMemcpy(b->tpl_roi.p, hr.data(), hr.size() * 4, cudaMemcpyHostToDevice));
     EMT6_CUDA(cudaMemcpy(b->tpl_fld.p, hf.data(), hf.size() * 4, cudaMemcpyHostToDevice));
     EMT6_CUDA(cudaMemcpy(b->tpl_st.p, hs.data(), hs.size(), cudaMemcpyHostToDevice));
     EMT6_CUDA(cudaMemcpy(b->tpl_cell.p, hc.data(), hc.size() * 16, cudaMemcpyHostToDevice));
@@ -806,6 +885,7 @@ int emt6_batch_create(const emt6_params *p, const emt6_site *tumors, int32_t n_t
   }
   // launch order, rebuilt on the device before every chunk (emt6::launch_order)
   EMT6_CUDA(b->order.alloc((size_t)n_sims));
+  EMT6_CUDA(b->tier.alloc((size_t)n_sims));
   EMT6_CUDA(b->order_hist.alloc(emt6::kOrderKeys));
   b->h_doses.assign((size_t)n_protocols * std::max<uint32_t>(protocol_bins, 1), 0.f);
   b->epoch = 0;
@@ -1331,7 +1411,7 @@ int emt6_test_order(const int32_t *roi, const uint32_t *step, const uint32_t *ho
   a.step = st.p;
   a.horizon = horizon ? hz.p : nullptr;
   a.nsims = nsims;
-  EMT6_CUDA(emt6::launch_order(a, t_end, hist.p, out.p, 0));
+  EMT6_CUDA(emt6::launch_order(a, t_end, hist.p, out.p, nullptr, 0));
   EMT6_CUDA(cudaMemcpy(order, out.p, nsims * sizeof(int64_t), cudaMemcpyDeviceToHost));
   return EMT6_OK;
 }

@@ -726,6 +726,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
       if (item >= a.nsims) break;
       sim = a.order ? a.order[item] : item;
     }
+    if (a.tier_of && a.tier_of[sim] != tier) continue;  // another concurrent launch's
     const uint32_t horizon = a.horizon ? a.horizon[sim] : 0xFFFFFFFFu;
     const uint32_t t_stop = t_end < horizon ? t_end : horizon;
     const uint32_t step0 = a.step[sim];
@@ -1085,11 +1086,24 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t *hist) {
   for (int k = 0; k < 4; ++k) hist[4 * t + k] = base + v[k];
 }
 
+// The tier expected to hold a simulation, from its stored region and list
+// (or, after a reset, its tumour's): a wrong guess only costs time, the launch
+// after the concurrent ones takes what they leave.
+__device__ __forceinline__ uint8_t expected_tier(const RunArgs &a, int64_t sim) {
+  const int *roi = a.roi + sim * 8;
+  const int h = roi[2], w = roi[3], d = roi[4], n = max(a.meta[sim].x, roi[5]) + 64;
+  const bool narrow = (h == 2 * d + 1 && w == h) ? d <= 16 : h + 2 <= 32 && w + 2 <= 32;
+  if (narrow && n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierNarrow).entries) return kTierNarrow;
+  return n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierWide).entries ? kTierWide : kTierFull;
+}
+
 __global__ void order_scatter_kernel(const RunArgs a, uint32_t t_end, uint32_t *hist,
-                                     int64_t *out) {
+                                     int64_t *out, uint8_t *tier) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.nsims;
-       i += (int64_t)gridDim.x * blockDim.x)
+       i += (int64_t)gridDim.x * blockDim.x) {
     out[atomicAdd(&hist[order_key(a, i, t_end)], 1u)] = i;
+    if (tier) tier[i] = expected_tier(a, i);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1109,7 +1123,7 @@ __global__ void reset_kernel(const ResetArgs a) {
     for (int q = threadIdx.x; q < a.HW * 3; q += blockDim.x) dc[q] = sc[q];
     if (threadIdx.x == 0) {
       a.meta[sim] = make_int4(0, 0, 0, 0);
-      for (int k = 0; k < 8; ++k) a.roi[sim * 8 + k] = 0;
+      for (int k = 0; k < 8; ++k) a.roi[sim * 8 + k] = a.tpl_roi[t * 8 + k];
       a.step[sim] = 0;
     }
   }
@@ -1282,6 +1296,10 @@ static cudaError_t ensure_smem(bool wide, size_t smem) {
                                   (int)smem)
            : cudaFuncSetAttribute(run_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem);
+  // both kernels ask for the same split of the L1, so their CTAs share SMs
+  if (e == cudaSuccess)
+    e = wide ? cudaFuncSetAttribute(run_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100)
+             : cudaFuncSetAttribute(run_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e == cudaSuccess) g_smem_set[wide][dev] = smem;
   return e;
 }
@@ -1298,7 +1316,7 @@ cudaError_t launch_run(const RunArgs &a, uint32_t t_end, int tier, int grid, cud
 }
 
 cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64_t *out,
-                         cudaStream_t stream) {
+                         uint8_t *tier, cudaStream_t stream) {
   if (a.nsims < 1) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(hist, 0, kOrderKeys * sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
@@ -1306,7 +1324,7 @@ cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64
   const int grid = (int)(blocks < 4096 ? blocks : 4096);
   order_count_kernel<<<grid, 256, 0, stream>>>(a, t_end, hist);
   order_scan_kernel<<<1, 1024, 0, stream>>>(hist);
-  order_scatter_kernel<<<grid, 256, 0, stream>>>(a, t_end, hist, out);
+  order_scatter_kernel<<<grid, 256, 0, stream>>>(a, t_end, hist, out, tier);
   return cudaGetLastError();
 }
 

@@ -12,7 +12,7 @@ namespace emt6 {
 // Device-resident batch, simulation-major.  Per simulation: fields
 // [3][H*W] FP32 (stride fstride floats), state bytes (sstride), cell records
 // [H*W][3] float4, occupied list (lstride u16), meta = (n, n0, multi, -),
-// roi[8] = (r0, c0, h, w, dist, -, -, -), step counter.
+// roi[8] = (r0, c0, h, w, dist, cells at the last reset, -, -), step counter.
 struct RunArgs {
   KParams p;
   float *fld;
@@ -33,6 +33,7 @@ struct RunArgs {
   int queue;  // 1: persistent CTAs take simulations from order[] via *ticket
   uint32_t *ticket;
   const int64_t *order;  // simulation of each CTA or ticket (null: the identity)
+  const uint8_t *tier_of;  // tier of each simulation (null: this launch takes any)
 };
 
 struct ResetArgs {
@@ -45,14 +46,15 @@ struct ResetArgs {
   const float *tpl_fld;
   const uint8_t *tpl_st;
   const float4 *tpl_cell;
+  const int32_t *tpl_roi;  // [templates][8]: where a simulation starts
   const int32_t *sim_tumor;
   uint32_t fstride, sstride;
   int HW;
   int64_t nsims;
 };
 
-// Tiers of a step launch, in this order: each takes the simulations that the
-// ones before left short of the target step (regions too wide, lists too long
+// Tiers of a step launch.  Run one after another without tier_of, each takes
+// the simulations that the ones before left short of the target step (regions too wide, lists too long
 // for the shared memory that lets 5 or 4 CTAs share an SM).  kTierFull holds any;
 // kTierWide may be skipped.
 enum { kTierNarrow = 0, kTierWide = 1, kTierFull = 2, kTiers = 3 };
@@ -62,10 +64,11 @@ int max_ctas_per_sm(const KParams &p, int tier);
 cudaError_t launch_run(const RunArgs &a, uint32_t t_end, int tier, int grid, cudaStream_t stream);
 cudaError_t launch_reset(const ResetArgs &a, cudaStream_t stream);
 // simulations sorted largest region first into out[0 .. a.nsims) for the
-// launches of a chunk ending at t_end; hist holds kOrderKeys counters
+// launches of a chunk ending at t_end, and (unless null) the tier expected to
+// hold each; hist holds kOrderKeys counters
 constexpr uint32_t kOrderKeys = 4096;
 cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64_t *out,
-                         cudaStream_t stream);
+                         uint8_t *tier, cudaStream_t stream);
 cudaError_t instr_read(unsigned long long counts[4], double *sum_dp, unsigned long long *hist);
 cudaError_t instr_reset();
 cudaError_t fp32_peak(int device, double *tflops);
