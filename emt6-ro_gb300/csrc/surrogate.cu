@@ -1,23 +1,20 @@
 // surrogate.cu -- the protocol-outcome surrogate: a 100 -> 512 -> 512 -> 512 -> 1
 // GELU MLP trained and evaluated on the GPU with hand-written kernels.
 //
-// GEMMs run on the 5th-generation tensor cores: one CTA of 512 threads owns a
-// 128 x 128 FP32 accumulator in tensor memory (TMEM, 128 columns); thread 0
-// streams 128 x 64 BF16 tiles of both operands into a 4-stage shared-memory
-// ring with TMA (128-byte swizzle), thread 32 issues tcgen05.mma (M = 128,
-// N = 128, K = 16, BF16 in, FP32 accumulate) and frees each stage with
-// tcgen05.commit; after the last k-block the 16 warps read the accumulator
-// back with tcgen05.ld (warp w: TMEM lanes 32(w % 4)..+31 = tile rows,
-// columns 32(w / 4)..+31) and run a fused epilogue:
-//   EPI_STORE_F32  C = A B^T in FP32 (tests, gradient export)
-//   EPI_BIAS_GELU  forward hidden layer: Z = acc + b, A = gelu(Z); stores Z, A
-//                  and A^T (BF16) so every later GEMM reads K-major operands
-//   EPI_GELU_BWD   dZ = acc * gelu'(Z) for the layer below; stores dZ, dZ^T
-//   EPI_ADAM       the accumulator is dW: Adam update of the FP32 master
-//                  weights, moments, and the BF16 copies W and W^T
-// Both operands are K-major ("TN": C[M,N] = sum_k A[m,k] B[n,k]), so a layer
-// keeps W [out, in] and W^T [in, out] in BF16 and activations in both
-// orientations; no transposes run between GEMMs.
+// All matrix products run on the 5th-generation tensor cores (tcgen05.mma, M =
+// 128, N = 128, K = 16, BF16 in, FP32 accumulators in tensor memory); operands
+// are K-major 64-column blocks in shared memory with the 128-byte swizzle.  A
+// training step is two launches, a prediction one:
+//   mlp_rows_kernel   everything that stays within a row: a cluster of 4 CTAs
+//     owns 128 rows, each CTA 128 of the 512 columns of every layer.  It packs
+//     the inputs, runs the hidden layers, the head, and (training) the error
+//     back through the layers.  A layer's activations go from a CTA's
+//     accumulator into its shared memory and from there, by bulk copies, into
+//     its three peers', where the next product reads them; weights stream in by
+//     TMA.
+//   mlp_grads_kernel  the weight gradients (products over the batch), split
+//     over a cluster's CTAs and summed in a fixed order through their shared
+//     memory, with Adam on the spot; the vectors' gradients beside them.
 //
 // Every wait on an mbarrier is bounded (kWaitLimitNs); a wait that runs out
 // sets an error flag, the CTA stops issuing work, waits (bounded) for its own
@@ -52,26 +49,8 @@ constexpr int BM = 128, BN = 128, BK = 64, STAGES = 4, GEMM_THREADS = 512;
 constexpr int TILE_BYTES = BM * BK * 2;  // 16 KB per operand per stage
 constexpr int GEMM_SMEM = 1024 + STAGES * 2 * TILE_BYTES + 256;
 constexpr uint64_t kWaitLimitNs = 1000000000ull;  // 1 s
-
-enum { EPI_STORE_F32 = 0, EPI_BIAS_GELU = 1, EPI_GELU_BWD = 2, EPI_ADAM = 3 };
-
-struct EpiArgs {
-  int M, N;
-  float *c_out;                 // STORE_F32: [M][N]
-  const float *bias;            // BIAS_GELU: [N]
-  __nv_bfloat16 *z_out;         // BIAS_GELU: [M][N]
-  __nv_bfloat16 *a_out;         // BIAS_GELU: A [M][N]; GELU_BWD: dZ [M][N]
-  __nv_bfloat16 *a_out_t;       // BIAS_GELU: A^T [N][M]; GELU_BWD: dZ^T [N][M]
-  const __nv_bfloat16 *z_in;    // GELU_BWD: Z of the layer below [M][N]
-  float *w, *m, *v;             // ADAM: master weights and moments [M][N]
-  __nv_bfloat16 *w_bf, *w_bf_t; // ADAM: BF16 W [M][N] and W^T [N][M]
-  float lr, beta1, beta2, eps, bc1, bc2;
-  int *err;
-  // test hook (emt6_test_mlp_gemm_timeout): when nonzero, the MMA issuer
-  // first waits this many ns on a barrier nothing arrives on, so it gives up
-  // exactly as a timed-out pipeline wait would
-  uint32_t stall_ns;
-};
+constexpr int IN = EMT6_MLP_IN, INP = EMT6_MLP_IN_PAD, HID = EMT6_MLP_HIDDEN;
+constexpr int CLUSTER = HID / BN;  // CTAs that share a tile of 128 rows
 
 // ---- PTX wrappers ----------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -148,6 +127,55 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// Clusters.  Every CTA of a cluster reaches every barrier, also after a wait
+// that gave up.
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// the address of shared-memory address `addr` in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
+// The same without ordering any data: the CTAs have all come this far.
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.relaxed;\n\tbarrier.cluster.wait;" ::: "memory");
+}
+
+// `bytes` of this CTA's shared memory at `src` to shared-memory address `dst` of a
+// peer, counted on the peer's mbarrier `bar` (both from peer_addr)
+__device__ __forceinline__ void peer_copy(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+      "r"(src), "r"(bytes), "r"(bar)
+      : "memory");
+}
+
+__device__ __forceinline__ void peer_store4(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+
+__device__ __forceinline__ float4 peer_load16(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+// orders this thread's shared-memory writes before later reads of the tensor cores
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
 // Programmatic dependent launch: the kernels of a training step are launched
 // with programmatic stream serialisation, so each one's launch and prologue
 // overlap the tail of the one before.  pdl_wait() blocks until the previous
@@ -197,6 +225,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 8 consecutive FP32 columns (see tmem_ld32)
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 // Shared-memory matrix descriptor: K-major tile written by TMA with the
 // 128-byte swizzle (rows of 64 BF16 = 128 B, 8-row atoms of 1024 B).
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
@@ -213,78 +255,57 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) |
                             (static_cast<uint32_t>(BN >> 3) << 17) |
                             (static_cast<uint32_t>(BM >> 4) << 24);
 
+// GELU and its derivative.  With u = |z|, the normal tail Phi(-u) is evaluated
+// as 2^-(1 + u P(u)): u P(u) = -log2(2 Phi(-u)) is smooth, and P is the weighted
+// minimax polynomial of degree 8 on [0, 6] (Lawson's iteration on Chebyshev
+// nodes, scipy's log_ndtr as the reference), within 2.4e-9 of Phi; the rounding
+// of the FP32 evaluation adds 2e-8, a third of an ulp of 1.  13 and 19
+// instructions in place of about 35 and 60 with erff and expf, on which the
+// epilogues spent most of their issue slots.
+__device__ __forceinline__ float exp2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Phi(-u), u = min(|z|, 6): beyond that it is below 1e-9
+__device__ __forceinline__ float normal_tail(float u) {
+  float p = -3.9834051790421654e-07f;
+  p = fmaf(p, u, 8.099371370917652e-06f);
+  p = fmaf(p, u, -6.745159771526232e-05f);
+  p = fmaf(p, u, 0.0002641645260155201f);
+  p = fmaf(p, u, 1.5400924894493073e-05f);
+  p = fmaf(p, u, -0.0069568706676363945f);
+  p = fmaf(p, u, 0.0524463951587677f);
+  p = fmaf(p, u, 0.4592190086841583f);
+  p = fmaf(p, u, 1.15110445022583f);
+  return exp2_approx(fmaf(-p, u, -1.0f));
+}
+
 __device__ __forceinline__ float gelu(float z) {
-  return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
+  // z Phi(z) = max(z, 0) - u Phi(-u).  NaN stays NaN (max.NaN), +inf is +inf, and
+  // -inf, which the product form makes -inf * 0, NaN.
+  float m;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(m) : "f"(z));
+  const float u = fminf(fabsf(z), 6.0f);
+  return fmaf(-fmaf(fminf(z, 0.0f), 0.0f, u), normal_tail(u), m);
 }
 
 __device__ __forceinline__ float gelu_grad(float z) {
-  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) +
-         z * 0.39894228040143268f * expf(-0.5f * z * z);
+  // Phi(z) + z phi(z), phi(z) = 2^(-z^2 / (2 ln 2)) / sqrt(2 pi)
+  const float h = normal_tail(fminf(fabsf(z), 6.0f));
+  const float phi = 0.39894228040143268f * exp2_approx(z * z * -0.72134752044448170f);
+  return fmaf(z, phi, z > 0.0f ? 1.0f - h : h);
 }
 
-// ---- epilogues ---------------------------------------------------------------
-template <int EPI>
-__device__ __forceinline__ void epilogue(const EpiArgs &ep, int row, int col0, const float (&v)[32]) {
-  const int M = ep.M, N = ep.N;
-  if constexpr (EPI == EPI_STORE_F32) {
-    float4 *dst = reinterpret_cast<float4 *>(ep.c_out + static_cast<size_t>(row) * N + col0);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-  } else if constexpr (EPI == EPI_BIAS_GELU) {
-    alignas(16) __nv_bfloat16 zb[32], ab[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float z = v[i] + __ldg(ep.bias + col0 + i);
-      zb[i] = __float2bfloat16_rn(z);
-      ab[i] = __float2bfloat16_rn(gelu(z));
-    }
-    uint4 *zd = reinterpret_cast<uint4 *>(ep.z_out + static_cast<size_t>(row) * N + col0);
-    uint4 *ad = reinterpret_cast<uint4 *>(ep.a_out + static_cast<size_t>(row) * N + col0);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      zd[i] = reinterpret_cast<const uint4 *>(zb)[i];
-      ad[i] = reinterpret_cast<const uint4 *>(ab)[i];
-    }
-#pragma unroll
-    for (int i = 0; i < 32; ++i) ep.a_out_t[static_cast<size_t>(col0 + i) * M + row] = ab[i];
-  } else if constexpr (EPI == EPI_GELU_BWD) {
-    alignas(16) __nv_bfloat16 zin[32], db[32];
-    const uint4 *zs = reinterpret_cast<const uint4 *>(ep.z_in + static_cast<size_t>(row) * N + col0);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) reinterpret_cast<uint4 *>(zin)[i] = zs[i];
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      db[i] = __float2bfloat16_rn(v[i] * gelu_grad(__bfloat162float(zin[i])));
-    uint4 *dd = reinterpret_cast<uint4 *>(ep.a_out + static_cast<size_t>(row) * N + col0);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dd[i] = reinterpret_cast<const uint4 *>(db)[i];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) ep.a_out_t[static_cast<size_t>(col0 + i) * M + row] = db[i];
-  } else {  // EPI_ADAM
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const size_t k = static_cast<size_t>(row) * N + col0 + i;
-      const float g = v[i];
-      const float m = ep.beta1 * ep.m[k] + (1.0f - ep.beta1) * g;
-      const float s = ep.beta2 * ep.v[k] + (1.0f - ep.beta2) * g * g;
-      const float w = ep.w[k] - ep.lr * (m / ep.bc1) / (sqrtf(s / ep.bc2) + ep.eps);
-      ep.m[k] = m;
-      ep.v[k] = s;
-      ep.w[k] = w;
-      const __nv_bfloat16 wb = __float2bfloat16_rn(w);
-      ep.w_bf[k] = wb;
-      ep.w_bf_t[static_cast<size_t>(col0 + i) * M + row] = wb;
-    }
-  }
-}
-
-// C tile (blockIdx.y, blockIdx.x) of C[M,N] = A[M,K] B[N,K]^T over the
-// k-blocks [blockIdx.z * nk, (blockIdx.z + 1) * nk) (split K: each z writes
-// its own FP32 partial tile, EPI_STORE_F32 only).
-template <int EPI>
+// C tile (blockIdx.y, blockIdx.x) of C[M,N] = A[M,K] B[N,K]^T in FP32: the
+// building block of the two kernels below on its own, for tests.  stall_ns
+// (emt6_test_mlp_gemm_timeout): when nonzero, the MMA issuer first waits this
+// many ns on a barrier nothing arrives on, so it gives up exactly as a
+// timed-out pipeline wait would.
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     mlp_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    int nk, EpiArgs ep) {
+                    int nk, int N, float *c_out, int *err, uint32_t stall_ns) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                               ~static_cast<uintptr_t>(1023));
@@ -299,8 +320,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                  done = smem_u32(bars + 2 * STAGES), never = smem_u32(bars + 2 * STAGES + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int kb0 = blockIdx.z * nk;
-  if (EPI == EPI_STORE_F32 && blockIdx.z) ep.c_out += static_cast<size_t>(blockIdx.z) * ep.M * ep.N;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -319,7 +338,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  pdl_wait();  // operands and epilogue inputs come from the previous kernel
 
   bool failed = false;
   int issued = 0;  // k-blocks whose loads thread 0 issued
@@ -333,13 +351,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         break;
       }
       mbar_expect_tx(full0 + 8 * s, 2 * TILE_BYTES);
-      tma_load_2d(smem_u32(sA + s * TILE_BYTES), &tmA, full0 + 8 * s, (kb0 + kb) * BK, m0);
-      tma_load_2d(smem_u32(sB + s * TILE_BYTES), &tmB, full0 + 8 * s, (kb0 + kb) * BK, n0);
+      tma_load_2d(smem_u32(sA + s * TILE_BYTES), &tmA, full0 + 8 * s, kb * BK, m0);
+      tma_load_2d(smem_u32(sB + s * TILE_BYTES), &tmB, full0 + 8 * s, kb * BK, n0);
       ++issued;
     }
   } else if (threadIdx.x == 32) {
     // MMA issuer
-    if (ep.stall_ns && !mbar_wait(never, 0, abort, ep.stall_ns)) {
+    if (stall_ns && !mbar_wait(never, 0, abort, stall_ns)) {
       failed = true;
       *abort = 1;
       __threadfence_block();
@@ -378,11 +396,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int quarter = warp & 3, group = warp >> 2;
     float v[32];
     tmem_ld32(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + group * 32, v);
-    epilogue<EPI>(ep, m0 + quarter * 32 + lane, n0 + group * 32, v);
+    float4 *dst = reinterpret_cast<float4 *>(
+        c_out + static_cast<size_t>(m0 + quarter * 32 + lane) * N + n0 + group * 32);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
   } else if (lane == 0) {
-    atomicOr(ep.err, 1);
+    atomicOr(err, 1);
   }
-  pdl_trigger();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -391,160 +411,595 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   }
 }
 
-// ---- small kernels -------------------------------------------------------------
-// fp32 features [B][in] -> BF16 X [B][in_pad] (zero padded) and X^T
-// [in_pad][B]; one block per 32 rows, the transpose through shared memory.
-__global__ void __launch_bounds__(256) pack_input_kernel(const float *x, int B, int in, int in_pad,
-                                                         __nv_bfloat16 *X, __nv_bfloat16 *XT,
-                                                         float *loss) {
-  __shared__ __nv_bfloat16 tile[128][34];
-  const int r0 = blockIdx.x * 32;
-  pdl_wait();
-  if (loss && blockIdx.x == 0 && threadIdx.x == 0) *loss = 0.0f;  // this step's loss sum
-  for (int i = threadIdx.x; i < 32 * in_pad; i += 256) {
-    const int rr = i / in_pad, c = i % in_pad;
-    const __nv_bfloat16 v =
-        __float2bfloat16_rn(c < in ? x[static_cast<size_t>(r0 + rr) * in + c] : 0.0f);
-    X[static_cast<size_t>(r0 + rr) * in_pad + c] = v;
-    tile[c][rr] = v;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 32 * in_pad; i += 256) {
-    const int c = i / 32, rr = i % 32;
-    XT[static_cast<size_t>(c) * B + r0 + rr] = tile[c][rr];
-  }
-  pdl_trigger();
+// ---- rows: forward, head, error ---------------------------------------------------
+struct RowsArgs {
+  const float *x;            // [n][100]
+  int n;                     // rows; training: a multiple of 128
+  int norm;                  // inputs are (x - mean) / std
+  float mean[IN], std[IN];
+  const float *b[3], *w4, *b4;
+  float *y;                  // prediction: [n]
+  // training
+  const float *target;
+  float *dy, *loss;
+  __nv_bfloat16 *z[3];                 // pre-activations, [n][512]
+  __nv_bfloat16 *xt, *at[3], *dzt[3];  // transposed, [columns][ld]
+  size_t ld;
+  int *err;
+};
+
+// shared memory of mlp_rows_kernel: the 8 blocks of the current operand, the
+// ring of weight tiles, barriers and the head's errors
+constexpr int ACT_BYTES = (HID / BK) * TILE_BYTES, RING = 6;
+constexpr int ROWS_SMEM = 1024 + ACT_BYTES + RING * TILE_BYTES + 2048;  // 227 KB: all there is
+
+// byte offset of the 16-byte chunk holding columns 8 * chunk .. of `row` in a
+// K-major operand of 128 rows (64-column blocks, 128-byte swizzle)
+__device__ __forceinline__ uint32_t act_chunk(int row, int chunk) {
+  return static_cast<uint32_t>((chunk >> 3) * TILE_BYTES + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
 }
 
-// Output layer and loss: y = A3 w4 + b4, one warp per row (8 BF16 per lane
-// per load); with targets, dy = 2 (y - t) / B and sum (y - t)^2 into *loss.
-__global__ void __launch_bounds__(256) head_y_kernel(const __nv_bfloat16 *A3, const float *w4,
-                                                     const float *b4, int B, int H,
-                                                     const float *target, float *y, float *dy,
-                                                     float *loss) {
-  __shared__ float s_loss[8];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // the grid covers B exactly
-  const uint4 *row = reinterpret_cast<const uint4 *>(A3 + static_cast<size_t>(r) * H);
-  pdl_wait();
-  float acc = 0.0f;
-  for (int j = lane; j < H / 8; j += 32) {
-    const uint4 u = row[j];
-    const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&u);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) acc += __bfloat162float(h[q]) * w4[8 * j + q];
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) {
-    const float yr = acc + b4[0];
-    y[r] = yr;
-    float e2 = 0.0f;
-    if (target) {
-      const float e = yr - target[r];
-      dy[r] = 2.0f * e / static_cast<float>(B);
-      e2 = e * e;
+// What bounds it, in cycles of a CTA per layer (4,096 rows): the weight tiles from
+// L2 and the products 5,800, the exchange 4,000, the epilogue 3,700, and training
+// 4,600 more for the transposed stores that the weight gradients need; the same
+// at 640 rows, so a latency chain of 57 us (43 us of it predicting: 20).  The
+// phases and the columns of an epilogue are loops, not unrolled: code that each
+// warp runs once is fetched as it goes.  With one launch per layer, and input,
+// head and error launches between, a step's rows took 75 us of GPU time.
+template <bool TRAIN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+    mlp_rows_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
+                    const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmT1,
+                    const __grid_constant__ CUtensorMap tmT2, const __grid_constant__ RowsArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                              ~static_cast<uintptr_t>(1023));
+  const uint32_t act = smem_u32(smem), ring = act + ACT_BYTES;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + ACT_BYTES + RING * TILE_BYTES);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * RING + 2);
+  volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  float *s_dy = reinterpret_cast<float *>(bars + 16);  // [128]
+  float *s_loss = s_dy + BM;                           // [16]
+  float *s_norm = s_loss + 16;                         // [2][100]
+  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + RING), done = smem_u32(bars + 2 * RING),
+                 in = smem_u32(bars + 2 * RING + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_rank();
+  const int m0 = static_cast<int>(blockIdx.x / CLUSTER) * BM, n0 = static_cast<int>(rank) * BN;
+  constexpr int PHASES = TRAIN ? 5 : 3;
+
+  if (tid == 0) {
+    for (int s = 0; s < RING; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
     }
-    s_loss[wid] = e2;
+    mbar_init(done, 1);
+    mbar_init(in, 1);
+    *abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (!target) return;
+  if (warp == 0) tmem_alloc(smem_u32(tmem_slot), BN);
+  tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.0f;
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();  // weights come from the previous kernel
+
+  // weight tiles of all phases in one sequence: layer 1 has 2 k-blocks, the
+  // others 8; the producer runs ahead of the products by the ring's 4 stages
+  int issued = 0;
+  bool failed = false;
+  auto load_tiles = [&](int phase, int from, int to) {  // thread 0
+    const CUtensorMap *map = phase == 0 ? &tmW0 : phase == 1 ? &tmW1 : phase == 2 ? &tmW2
+                             : phase == 3 ? &tmT2 : &tmT1;
+    for (int kb = from; kb < to && !*abort; ++kb) {
+      const int s = issued % RING;
+      if (issued >= RING && !mbar_wait(empty0 + 8 * s, ((issued / RING) - 1) & 1, abort)) {
+        *abort = 1;
+        break;
+      }
+      mbar_expect_tx(full0 + 8 * s, TILE_BYTES);
+      tma_load_2d(ring + s * TILE_BYTES, map, full0 + 8 * s, kb * BK, n0);
+      ++issued;
+    }
+  };
+  if (tid == 0) load_tiles(0, 0, 2);
+  if (!TRAIN && a.norm) {
+    if (tid < IN) {
+      s_norm[tid] = a.mean[tid];
+      s_norm[IN + tid] = a.std[tid];
+    }
+    __syncthreads();
+  }
+
+  // Exchange of operand blocks within the cluster: each CTA writes its own part
+  // of the next operand locally, then bulk copies take it to the three peers
+  // (scattered remote stores of the same values took 5 us a layer).  `in` counts
+  // what arrives from them.
+  int exchanges = 0;
+  const auto exchange = [&](uint32_t at, uint32_t bytes, int pieces, uint32_t pitch) {
+    fence_async();
+    __syncthreads();
+    if (tid == 0) {
+      mbar_expect_tx(in, (CLUSTER - 1) * bytes * pieces);
+      for (uint32_t p = 1; p < CLUSTER; ++p) {
+        const uint32_t to = (rank + p) % CLUSTER;
+        for (int i = 0; i < pieces; ++i)
+          peer_copy(peer_addr(act + at + i * pitch, to), act + at + i * pitch, bytes, peer_addr(in, to));
+      }
+    }
+    ++exchanges;
+  };
+  const auto arrived = [&]() -> bool { return mbar_wait(in, (exchanges - 1) & 1, nullptr); };
+  cluster_meet();  // every CTA runs, its barriers initialised
+
+  // ---- inputs: FP32 rows -> BF16 operand (zero columns 100..127, zero rows
+  // beyond n).  Each CTA packs a quarter of the rows: one 16-byte chunk per thread.
+  {
+    static_assert(BM / CLUSTER * (INP / 8) == GEMM_THREADS, "one chunk per thread");
+    const int r = static_cast<int>(rank) * (BM / CLUSTER) + tid / (INP / 8), chunk = tid % (INP / 8);
+    float f[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) t += s_loss[i];
-    atomicAdd(loss, t);
+    for (int q = 0; q < 8; ++q) f[q] = 0.0f;
+    if (m0 + r < a.n) {
+      const float *src = a.x + static_cast<size_t>(m0 + r) * IN + chunk * 8;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (chunk * 8 + q < IN) f[q] = src[q];
+      if (!TRAIN && a.norm) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (chunk * 8 + q < IN) f[q] = (f[q] - s_norm[chunk * 8 + q]) / s_norm[IN + chunk * 8 + q];
+      }
+    }
+    alignas(16) __nv_bfloat16 v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = __float2bfloat16_rn(f[q]);
+    *reinterpret_cast<uint4 *>(smem + act_chunk(r, chunk)) = *reinterpret_cast<const uint4 *>(v);
   }
-  pdl_trigger();
-}
+  // 32 rows of the 2 blocks
+  exchange(rank * (BM / CLUSTER) * 128, BM / CLUSTER * 128, INP / BK, TILE_BYTES);
+  const auto act_at = [&](int row, int col) -> __nv_bfloat16 {
+    return *reinterpret_cast<const __nv_bfloat16 *>(smem + act_chunk(row, col >> 3) + (col & 7) * 2);
+  };
+  if (TRAIN) {
+    // this CTA's quarter of X^T
+    if (!arrived()) failed = true;
+    for (int i = tid; i < (INP / CLUSTER) * BM; i += GEMM_THREADS) {
+      const int c = static_cast<int>(rank) * (INP / CLUSTER) + i / BM, r = i % BM;
+      a.xt[static_cast<size_t>(c) * a.ld + m0 + r] = act_at(r, c);
+    }
+  }
 
-// dZ3 = dy w4 * gelu'(Z3) for a 32-row x 64-column tile per block, stored in
-// both orientations (the transposed copy through shared memory).
-__global__ void __launch_bounds__(256) head_dz_kernel(const __nv_bfloat16 *Z3, const float *w4,
-                                                      const float *dy, int B, int H,
-                                                      __nv_bfloat16 *dZ3, __nv_bfloat16 *dZ3T) {
-  __shared__ __nv_bfloat16 tile[64][34];
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 64;
-  pdl_wait();
-  for (int i = threadIdx.x; i < 32 * 64; i += 256) {
-    const int rr = i / 64, cc = i % 64;
-    const int r = r0 + rr, c = c0 + cc;
-    const float z = __bfloat162float(Z3[static_cast<size_t>(r) * H + c]);
-    const __nv_bfloat16 g = __float2bfloat16_rn(dy[r] * w4[c] * gelu_grad(z));
-    dZ3[static_cast<size_t>(r) * H + c] = g;
-    tile[cc][rr] = g;
+  const int quarter = warp & 3, group = warp >> 2;
+  const int row = quarter * 32 + lane, col0 = n0 + group * 32;  // this thread's row, columns col0..+31
+  const uint32_t acc0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + group * 32;
+  // 8 BF16 values of this thread (columns col0 + 8 j ..) into the next operand
+  const auto publish = [&](int j, const uint4 &v) {
+    *reinterpret_cast<uint4 *>(smem + act_chunk(row, col0 / 8 + j)) = v;
+  };
+  const uint32_t own = rank * (BN / BK) * TILE_BYTES;  // this CTA's two blocks of it
+  const auto store_t = [&](__nv_bfloat16 *t, int j, const uint4 &v) {
+    const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[static_cast<size_t>(col0 + 8 * j + i) * a.ld + m0 + row] = e[i];
+  };
+  const auto z_at = [&](int l, int j) -> uint4 & {
+    return *reinterpret_cast<uint4 *>(a.z[l] + static_cast<size_t>(m0 + row) * HID + col0 + 8 * j);
+  };
+
+  int used = 0;  // weight tiles consumed by earlier phases
+#pragma unroll 1
+  for (int phase = 0; phase < PHASES; ++phase) {
+    const int nk = phase == 0 ? INP / BK : HID / BK;
+    // ---- product: accumulator = operand x this CTA's 128 weight rows
+    if (tid == 0) {
+      load_tiles(phase, phase == 0 ? 2 : RING, nk);
+    } else if (tid == 32) {
+      if (!arrived()) *abort = 1;
+      tc_fence_after();
+      for (int kb = 0; kb < nk && !*abort; ++kb) {
+        const int s = (used + kb) % RING;
+        if (!mbar_wait(full0 + 8 * s, ((used + kb) / RING) & 1, abort)) {
+          *abort = 1;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t pa = act + kb * TILE_BYTES, pb = ring + s * TILE_BYTES;
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          umma_bf16(tmem, sw128_desc(pa + 32 * k), sw128_desc(pb + 32 * k), kIdesc,
+                    (kb | k) != 0 ? 1u : 0u);
+        umma_commit(empty0 + 8 * s);
+      }
+      umma_commit(done);  // arrives once every product above has completed
+    }
+    __syncwarp();
+    if (!mbar_wait(done, phase & 1, nullptr)) failed = true;
+    tc_fence_after();
+    used += nk;
+    // the ring is free: the next phase's first tiles load during the epilogue
+    if (tid == 0 && phase + 1 < PHASES) load_tiles(phase + 1, 0, RING);
+    __syncwarp();
+    const bool last = TRAIN && phase == PHASES - 1;  // the lowest layer's error goes no further
+    if (!last) cluster_meet();  // every CTA's products have read the operand and its copies
+    // ---- epilogue
+    if (phase < 3) {
+      const float *bias = a.b[phase] + col0;
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        float v[8];
+        tmem_ld8(acc0 + 8 * j, v);
+        alignas(16) __nv_bfloat16 zb[8], h[8];
+        const float4 b0 = __ldg(reinterpret_cast<const float4 *>(bias + 8 * j)),
+                     b1 = __ldg(reinterpret_cast<const float4 *>(bias + 8 * j + 4));
+        const float bj[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float z = v[i] + bj[i];
+          zb[i] = __float2bfloat16_rn(z);
+          h[i] = __float2bfloat16_rn(gelu(z));
+        }
+        const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
+        publish(j, hv);
+        if (TRAIN) {
+          z_at(phase, j) = *reinterpret_cast<const uint4 *>(zb);
+          store_t(a.at[phase], j, hv);
+        }
+      }
+    } else {
+      const int l = phase == 3 ? 1 : 0;  // layer whose pre-activations the error passes
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        const uint4 zq = z_at(l, j);
+        const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zq);
+        float v[8];
+        tmem_ld8(acc0 + 8 * j, v);
+        alignas(16) __nv_bfloat16 h[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h[i] = __float2bfloat16_rn(v[i] * gelu_grad(__bfloat162float(zb[i])));
+        const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
+        if (!last) publish(j, hv);
+        store_t(a.dzt[l], j, hv);
+      }
+    }
+    if (last) break;
+    tc_fence_before();
+    exchange(own, BN / BK * TILE_BYTES, 1, 0);
+    if (phase == 2) {
+      if (!arrived()) failed = true;
+      // ---- head: y = A3 w4 + b4, one warp per row
+#pragma unroll 1
+      for (int k = 0; k < BM / CLUSTER / 16; ++k) {
+        const int r = static_cast<int>(rank) * (BM / CLUSTER) + warp * (BM / CLUSTER / 16) + k;
+        float acc = 0.0f;
+#pragma unroll
+        for (int j = lane; j < HID / 8; j += 32) {
+          const uint4 u = *reinterpret_cast<const uint4 *>(smem + act_chunk(r, j));
+          const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&u);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc += __bfloat162float(e[q]) * a.w4[8 * j + q];
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        const float yr = acc + a.b4[0];
+        if (!TRAIN) {
+          if (lane == 0 && m0 + r < a.n) a.y[m0 + r] = yr;
+        } else {
+          const float e = yr - a.target[m0 + r], d = 2.0f * e / static_cast<float>(a.n);
+          if (lane == 0) {
+            a.dy[m0 + r] = d;
+            s_loss[warp] = (k ? s_loss[warp] : 0.0f) + e * e;
+          }
+          if (lane < CLUSTER) peer_store4(peer_addr(smem_u32(s_dy + r), lane), d);
+        }
+      }
+      if (TRAIN) {
+        cluster_sync();  // dy is everywhere, and the operand may be overwritten
+        if (tid == 0) {
+          float t = 0.0f;
+#pragma unroll
+          for (int k = 0; k < 16; ++k) t += s_loss[k];
+          atomicAdd(a.loss, t);
+        }
+        const float d = s_dy[row];
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          const uint4 zq = z_at(2, j);
+          const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zq);
+          alignas(16) __nv_bfloat16 h[8];
+          const float4 w0 = __ldg(reinterpret_cast<const float4 *>(a.w4 + col0 + 8 * j)),
+                       w1 = __ldg(reinterpret_cast<const float4 *>(a.w4 + col0 + 8 * j + 4));
+          const float wj[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            h[i] = __float2bfloat16_rn(d * wj[i] * gelu_grad(__bfloat162float(zb[i])));
+          const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
+          publish(j, hv);
+          store_t(a.dzt[2], j, hv);
+        }
+        exchange(own, BN / BK * TILE_BYTES, 1, 0);
+      }
+    }
   }
+  // no CTA leaves while a peer may still read from or write to it
+  cluster_meet();
+  pdl_trigger();
+  if (*abort || failed) {
+    if (lane == 0) atomicOr(a.err, 1);
+    // loads still in flight (at most the last RING issued) land before the
+    // CTA frees its shared memory
+    if (tid == 0)
+      for (int k = issued - RING < 0 ? 0 : issued - RING; k < issued; ++k)
+        mbar_wait(full0 + 8 * (k % RING), (k / RING) & 1, nullptr);
+  }
+  tc_fence_before();
   __syncthreads();
-  for (int i = threadIdx.x; i < 32 * 64; i += 256) {
-    const int cc = i / 32, rr = i % 32;
-    dZ3T[static_cast<size_t>(c0 + cc) * B + r0 + rr] = tile[cc][rr];
+  if (warp == 0) {
+    __syncwarp();
+    tmem_dealloc(tmem, BN);
   }
-  pdl_trigger();
 }
 
+// ---- weight gradients and Adam -------------------------------------------------------
 struct VecAdam {
   float *w, *m, *v;
-  const __nv_bfloat16 *rows;  // [n][B] rows to sum (bias: dZ^T), or A3^T for w4
-  const float *dy;            // w4: weights of the row sum; null for biases
-  float *grad_out;            // optional: export of the gradient
+  const __nv_bfloat16 *rows;  // [n][ld] rows to sum (bias: dZ^T), or A3^T for w4; null: b4
+  float *grad_out;
   int n;
 };
 
-// Gradients and Adam updates of the vectors: b1, b2, b3 (row sums of dZ^T),
-// w4 (A3^T dy) and b4 (sum dy).  One warp per element.
-__global__ void vec_adam_kernel(VecAdam p0, VecAdam p1, VecAdam p2, VecAdam p3, VecAdam p4, int B,
-                                float lr, float beta1, float beta2, float eps, float bc1, float bc2,
-                                int apply) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  pdl_wait();
-  int idx = gw;
-  VecAdam p;
-  if (idx < p0.n) {
-    p = p0;
-  } else if ((idx -= p0.n) < p1.n) {
-    p = p1;
-  } else if ((idx -= p1.n) < p2.n) {
-    p = p2;
-  } else if ((idx -= p2.n) < p3.n) {
-    p = p3;
-  } else if ((idx -= p3.n) < p4.n) {
-    p = p4;
-  } else {
-    return;
+struct GradsArgs {
+  float *w[3], *m[3], *v[3];
+  __nv_bfloat16 *wb[3], *wbt[3];  // BF16 W and (null for the first layer) W^T
+  float *grad[3];                 // export instead of the update, or null
+  VecAdam vec[5];
+  const float *dy;
+  float *clear;  // the next step's loss sum
+  size_t ld;
+  int B, splits;
+  float lr, beta1, beta2, eps, bc1, bc2;
+  int *err;
+};
+
+// Gradients and Adam updates of elements e, e + stride, .. (VEC_U of them, below
+// VEC_ELEMS) of the vectors b1, b2, b3 (row sums of dZ^T), w4 (A3^T dy) and b4
+// (sum dy).  One warp; the elements' loads overlap, and lane u updates the u-th.
+constexpr int VEC_ELEMS = 4 * HID + 1, VEC_U = 4;
+__device__ __forceinline__ void vec_adam(const GradsArgs &a, int e, int stride, int lane) {
+  const uint4 *rows[VEC_U];
+  float g[VEC_U], mine = 0.0f;
+#pragma unroll
+  for (int u = 0; u < VEC_U; ++u) {
+    const int q = e + u * stride, k = q / HID;
+    g[u] = 0.0f;
+    rows[u] = k < 4 && q < VEC_ELEMS
+                  ? reinterpret_cast<const uint4 *>(a.vec[k].rows + static_cast<size_t>(q % HID) * a.ld)
+                  : nullptr;
   }
-  float g = 0.0f;
-  if (p.rows) {
-    // B is a multiple of 128: 8 BF16 (16 bytes) per lane per load
-    const uint4 *row = reinterpret_cast<const uint4 *>(p.rows + static_cast<size_t>(idx) * B);
-    for (int j = lane; j < B / 8; j += 32) {
-      const uint4 u = row[j];
-      const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&u);
-      if (p.dy) {
-        const float4 d0 = reinterpret_cast<const float4 *>(p.dy)[2 * j];
-        const float4 d1 = reinterpret_cast<const float4 *>(p.dy)[2 * j + 1];
-        g += __bfloat162float(h[0]) * d0.x + __bfloat162float(h[1]) * d0.y +
-             __bfloat162float(h[2]) * d0.z + __bfloat162float(h[3]) * d0.w +
-             __bfloat162float(h[4]) * d1.x + __bfloat162float(h[5]) * d1.y +
-             __bfloat162float(h[6]) * d1.z + __bfloat162float(h[7]) * d1.w;
+  // this lane's element (lanes 0 .. VEC_U - 1)
+  const int q = e + lane * stride, k = q / HID, idx = q % HID;
+  const bool own = lane < VEC_U && q < VEC_ELEMS;
+  const VecAdam &p = a.vec[own ? k : 0];
+  float m0 = 0.0f, v0 = 0.0f, w0 = 0.0f;
+  if (own && !p.grad_out) {
+    m0 = p.m[idx];
+    v0 = p.v[idx];
+    w0 = p.w[idx];
+  }
+  // B is a multiple of 128: 8 BF16 (16 bytes) per lane per load
+  for (int j = lane; j < a.B / 8; j += 32) {
+    uint4 r[VEC_U];
+#pragma unroll
+    for (int u = 0; u < VEC_U; ++u)
+      if (rows[u]) r[u] = rows[u][j];
+#pragma unroll
+    for (int u = 0; u < VEC_U; ++u) {
+      if (!rows[u]) continue;
+      const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&r[u]);
+      if ((e + u * stride) / HID == 3) {
+        const float4 d0 = reinterpret_cast<const float4 *>(a.dy)[2 * j];
+        const float4 d1 = reinterpret_cast<const float4 *>(a.dy)[2 * j + 1];
+        g[u] += __bfloat162float(h[0]) * d0.x + __bfloat162float(h[1]) * d0.y +
+                __bfloat162float(h[2]) * d0.z + __bfloat162float(h[3]) * d0.w +
+                __bfloat162float(h[4]) * d1.x + __bfloat162float(h[5]) * d1.y +
+                __bfloat162float(h[6]) * d1.z + __bfloat162float(h[7]) * d1.w;
       } else {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) g += __bfloat162float(h[q]);
+        for (int i = 0; i < 8; ++i) g[u] += __bfloat162float(h[i]);
       }
     }
-  } else {
-    for (int j = lane; j < B; j += 32) g += p.dy[j];
   }
 #pragma unroll
-  for (int o = 16; o; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-  if (lane != 0) return;
-  if (p.grad_out) p.grad_out[idx] = g;
-  if (!apply) return;
-  const float m = beta1 * p.m[idx] + (1.0f - beta1) * g;
-  const float s = beta2 * p.v[idx] + (1.0f - beta2) * g * g;
+  for (int u = 0; u < VEC_U; ++u) {
+    if (e + u * stride == VEC_ELEMS - 1)
+      for (int j = lane; j < a.B; j += 32) g[u] += a.dy[j];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) g[u] += __shfl_xor_sync(0xffffffffu, g[u], o);
+    if (lane == u) mine = g[u];
+  }
+  if (!own) return;
+  if (p.grad_out) {
+    p.grad_out[idx] = mine;
+    return;
+  }
+  const float m = a.beta1 * m0 + (1.0f - a.beta1) * mine;
+  const float s = a.beta2 * v0 + (1.0f - a.beta2) * mine * mine;
   p.m[idx] = m;
   p.v[idx] = s;
-  p.w[idx] -= lr * (m / bc1) / (sqrtf(s / bc2) + eps);
+  p.w[idx] = w0 - a.lr * (m / a.bc1) / (sqrtf(s / a.bc2) + a.eps);
+}
+
+// tiles of 128 x 128 weights: 16 of layer 3, 16 of layer 2, 4 of layer 1
+constexpr int GRAD_TILES = 36;
+constexpr int RED_BYTES = 2 * BM * BN * 4;  // two partial tiles, over the ring
+constexpr int TILE_T_BYTES = BN * (BM + 8) * 2;  // W^T on its way out, rows padded
+constexpr int GRADS_SMEM = 1024 + RED_BYTES + TILE_T_BYTES + 256;
+static_assert(RED_BYTES >= STAGES * 2 * TILE_BYTES, "the partial tiles replace the ring");
+
+// One cluster per tile of dW = dZ^T A (a product over the batch): its CTAs take
+// consecutive parts of the batch (`splits` parts in all, one or two per CTA,
+// each with an accumulator of its own), lay the partial tiles down in shared
+// memory, and each sums a share of the rows over all parts in order, applies
+// Adam and writes W and W^T.  Warps that do not feed the tensor cores compute
+// the vectors' gradients meanwhile.  Bound by L2 reads at 4,096 rows (75 MB of
+// operands in 9.5 us); 15 us in all, where the seven launches it replaces took
+// 40.
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+    mlp_grads_kernel(const __grid_constant__ CUtensorMap tmZ0, const __grid_constant__ CUtensorMap tmZ1,
+                     const __grid_constant__ CUtensorMap tmZ2, const __grid_constant__ CUtensorMap tmX,
+                     const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
+                     const __grid_constant__ GradsArgs a, int cluster) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                              ~static_cast<uintptr_t>(1023));
+  const uint32_t ringA = smem_u32(smem), ringB = ringA + STAGES * TILE_BYTES;
+  float *red = reinterpret_cast<float *>(smem);  // [part][128][128], columns swizzled
+  __nv_bfloat16 *tile_t = reinterpret_cast<__nv_bfloat16 *>(smem + RED_BYTES);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + RED_BYTES + TILE_T_BYTES);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 1);
+  volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES), done = smem_u32(bars + 2 * STAGES);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = static_cast<int>(cluster_rank());
+  const int t = static_cast<int>(blockIdx.x) / cluster;
+  const int l = t < 16 ? 2 : t < 32 ? 1 : 0, N = l ? HID : INP;
+  const int k = t < 16 ? t : t < 32 ? t - 16 : t - 32;
+  const int m0 = (l ? k / 4 : k) * BM, n0 = (l ? k % 4 : 0) * BN;
+  const int parts = a.splits / cluster, nkp = a.B / BK / a.splits, nk = parts * nkp;
+  const int kb0 = rank * nk;
+
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    mbar_init(done, 1);
+    *abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) tmem_alloc(smem_u32(tmem_slot), 2 * BN);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();  // operands come from the previous kernel
+
+  int issued = 0;
+  if (tid == 0) {
+    const CUtensorMap *ma = l == 2 ? &tmZ2 : l == 1 ? &tmZ1 : &tmZ0;
+    const CUtensorMap *mb = l == 2 ? &tmA1 : l == 1 ? &tmA0 : &tmX;
+    for (int kb = 0; kb < nk; ++kb) {
+      const int s = kb % STAGES;
+      if (kb >= STAGES && !mbar_wait(empty0 + 8 * s, ((kb / STAGES) - 1) & 1, abort)) {
+        *abort = 1;
+        break;
+      }
+      mbar_expect_tx(full0 + 8 * s, 2 * TILE_BYTES);
+      tma_load_2d(ringA + s * TILE_BYTES, ma, full0 + 8 * s, (kb0 + kb) * BK, m0);
+      tma_load_2d(ringB + s * TILE_BYTES, mb, full0 + 8 * s, (kb0 + kb) * BK, n0);
+      ++issued;
+    }
+  } else if (tid == 32) {
+    for (int kb = 0; kb < nk; ++kb) {
+      const int s = kb % STAGES;
+      if (!mbar_wait(full0 + 8 * s, (kb / STAGES) & 1, abort)) {
+        *abort = 1;
+        break;
+      }
+      tc_fence_after();
+      const uint32_t pa = ringA + s * TILE_BYTES, pb = ringB + s * TILE_BYTES;
+#pragma unroll
+      for (int q = 0; q < BK / 16; ++q)
+        umma_bf16(tmem + static_cast<uint32_t>(kb / nkp) * BN, sw128_desc(pa + 32 * q),
+                  sw128_desc(pb + 32 * q), kIdesc, (kb % nkp | q) != 0 ? 1u : 0u);
+      umma_commit(empty0 + 8 * s);
+    }
+    umma_commit(done);  // arrives once every product above has completed
+  } else if (warp >= 2) {
+    if (blockIdx.x == 0 && tid == 64) *a.clear = 0.0f;
+    const int stride = static_cast<int>(gridDim.x) * 14;
+    for (int e = static_cast<int>(blockIdx.x) * 14 + warp - 2; e < VEC_ELEMS; e += VEC_U * stride)
+      vec_adam(a, e, stride, lane);
+  }
+  __syncwarp();
+  bool failed = !mbar_wait(done, 0, nullptr);
+  if (tid == 0 && *abort)
+    for (int q = issued - STAGES < 0 ? 0 : issued - STAGES; q < issued; ++q)
+      mbar_wait(full0 + 8 * (q % STAGES), (q / STAGES) & 1, nullptr);
+  failed = failed || *abort;
+  tc_fence_after();
+  __syncthreads();  // (after an abort: nothing lands in the ring any more)
+  const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane;
+  for (int p = 0; p < parts; ++p) {
+    float v[32];
+    tmem_ld32(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + p * BN + group * 32, v);
+    // 16-byte columns of a row swizzled by the row: conflict-free both ways
+    float4 *dst = reinterpret_cast<float4 *>(red + p * BM * BN + row * BN);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      dst[(group * 8 + i) ^ (row & 31)] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  }
+  if (failed && lane == 0) atomicOr(a.err, 1);
+  tc_fence_before();
+  cluster_sync();
+  const int share = BM / cluster, r0 = rank * share;  // rows this CTA finishes
+  const uint32_t base = smem_u32(red);
+  for (int i = tid; i < share * 32; i += GEMM_THREADS) {
+    const int r = r0 + (i >> 5), c4 = i & 31;
+    const uint32_t at = base + static_cast<uint32_t>((r * 32 + (c4 ^ (r & 31))) * 16);
+    const size_t at_w = static_cast<size_t>(m0 + r) * N + n0 + 4 * c4;
+    float4 m4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = m4, w4 = m4;
+    if (!a.grad[l]) {
+      m4 = *reinterpret_cast<const float4 *>(a.m[l] + at_w);
+      v4 = *reinterpret_cast<const float4 *>(a.v[l] + at_w);
+      w4 = *reinterpret_cast<const float4 *>(a.w[l] + at_w);
+    }
+    float4 q[8];  // all parts' loads in flight, then summed in order
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+      if (p < a.splits)
+        q[p] = peer_load16(peer_addr(at + (parts == 2 ? p & 1 : 0) * (BM * BN * 4), parts == 2 ? p >> 1 : p));
+    float4 g = q[0];
+#pragma unroll
+    for (int p = 1; p < 8; ++p)
+      if (p < a.splits) {
+        g.x += q[p].x; g.y += q[p].y; g.z += q[p].z; g.w += q[p].w;
+      }
+    if (a.grad[l]) {
+      *reinterpret_cast<float4 *>(a.grad[l] + at_w) = g;
+      continue;
+    }
+    const float gg[4] = {g.x, g.y, g.z, g.w}, mo[4] = {m4.x, m4.y, m4.z, m4.w},
+                vo[4] = {v4.x, v4.y, v4.z, v4.w}, wo[4] = {w4.x, w4.y, w4.z, w4.w};
+    float mn[4], vn[4], wn[4];
+    alignas(8) __nv_bfloat16 wb[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      mn[q] = a.beta1 * mo[q] + (1.0f - a.beta1) * gg[q];
+      vn[q] = a.beta2 * vo[q] + (1.0f - a.beta2) * gg[q] * gg[q];
+      wn[q] = wo[q] - a.lr * (mn[q] / a.bc1) / (sqrtf(vn[q] / a.bc2) + a.eps);
+      wb[q] = __float2bfloat16_rn(wn[q]);
+      tile_t[(4 * c4 + q) * (share + 8) + ((((r - r0) >> 3) ^ ((c4 >> 1) & 3)) << 3) + (r & 7)] = wb[q];
+    }
+    *reinterpret_cast<float4 *>(a.m[l] + at_w) = make_float4(mn[0], mn[1], mn[2], mn[3]);
+    *reinterpret_cast<float4 *>(a.v[l] + at_w) = make_float4(vn[0], vn[1], vn[2], vn[3]);
+    *reinterpret_cast<float4 *>(a.w[l] + at_w) = make_float4(wn[0], wn[1], wn[2], wn[3]);
+    *reinterpret_cast<uint2 *>(a.wb[l] + at_w) = *reinterpret_cast<const uint2 *>(wb);
+  }
+  __syncthreads();
+  if (!a.grad[l] && a.wbt[l])
+    for (int i = tid; i < BN * share / 8; i += GEMM_THREADS) {
+      const int c = i / (share / 8), q = i % (share / 8);
+      *reinterpret_cast<uint4 *>(a.wbt[l] + static_cast<size_t>(n0 + c) * HID + m0 + r0 + 8 * q) =
+          *reinterpret_cast<const uint4 *>(tile_t + c * (share + 8) + ((q ^ ((c >> 3) & 3)) << 3));
+    }
   pdl_trigger();
+  cluster_sync();  // no CTA leaves while another reads its partial tiles
+  if (warp == 0) {
+    __syncwarp();
+    tmem_dealloc(tmem, 2 * BN);
+  }
 }
 
 __global__ void to_bf16_kernel(const float *src, __nv_bfloat16 *dst, __nv_bfloat16 *dst_t, int rows,
@@ -586,81 +1041,39 @@ bool make_map(CUtensorMap *map, const void *base, int rows, int cols) {
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Launch with programmatic stream serialisation (see pdl_wait / pdl_trigger).
+// Launch in clusters, with programmatic stream serialisation (see pdl_wait /
+// pdl_trigger).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                       cudaStream_t st, Args &&...args) {
+cudaError_t launch_clusters(void (*kernel)(KArgs...), int grid, int cluster, size_t smem,
+                            cudaStream_t st, const Args &...args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <int EPI>
-cudaError_t launch_gemm(const CUtensorMap &a, const CUtensorMap &b, int M, int N, int K,
-                        const EpiArgs &ep, cudaStream_t st, int splits = 1) {
-  static bool attr_set[64] = {};
+// Dynamic shared memory of a kernel, raised once per device.
+template <typename K>
+cudaError_t raise_smem(K kernel, int bytes, bool (&done)[64]) {
   int dev = 0;
-  cudaGetDevice(&dev);
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(mlp_gemm_kernel<EPI>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
-  }
-  return launch_pdl(mlp_gemm_kernel<EPI>, dim3(N / BN, M / BM, splits), dim3(GEMM_THREADS),
-                    GEMM_SMEM, st, a, b, K / BK / splits, ep);
-}
-
-// Sum of the split-K partial tiles of a weight gradient g[M][N] in a fixed
-// order, then either the Adam update (FP32 master, moments, BF16 W and W^T)
-// or, with grad_out, the gradient itself.  One element per thread, 32 x 32
-// tiles of 1024 threads; W^T goes through shared memory so both stores are
-// coalesced.
-__global__ void __launch_bounds__(1024) adam_reduce_kernel(const float *__restrict__ part,
-                                                           int splits, int M, int N, float *w,
-                                                           float *m, float *v,
-                                                           __nv_bfloat16 *w_bf,
-                                                           __nv_bfloat16 *w_bf_t, float *grad_out,
-                                                           float lr, float beta1, float beta2,
-                                                           float eps, float bc1, float bc2) {
-  __shared__ __nv_bfloat16 tile[32][34];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int r = blockIdx.y * 32 + ty, c = blockIdx.x * 32 + tx;
-  const size_t MN = static_cast<size_t>(M) * N;
-  const size_t k = static_cast<size_t>(r) * N + c;
-  pdl_wait();
-  float pz[8];
-#pragma unroll
-  for (int z = 0; z < 8; ++z) pz[z] = z < splits ? part[z * MN + k] : 0.0f;
-  float g = pz[0];
-#pragma unroll
-  for (int z = 1; z < 8; ++z)
-    if (z < splits) g += pz[z];
-  if (grad_out) {
-    grad_out[k] = g;
-    return;
-  }
-  const float mm = beta1 * m[k] + (1.0f - beta1) * g;
-  const float vv = beta2 * v[k] + (1.0f - beta2) * g * g;
-  const float ww = w[k] - lr * (mm / bc1) / (sqrtf(vv / bc2) + eps);
-  m[k] = mm;
-  v[k] = vv;
-  w[k] = ww;
-  const __nv_bfloat16 wb = __float2bfloat16_rn(ww);
-  w_bf[k] = wb;
-  tile[tx][ty] = wb;
-  __syncthreads();
-  w_bf_t[static_cast<size_t>(blockIdx.x * 32 + ty) * M + blockIdx.y * 32 + tx] = tile[ty][tx];
-  pdl_trigger();
+  if (done[dev]) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done[dev] = true;
+  return e;
 }
 
 template <typename T>
@@ -680,20 +1093,20 @@ struct DevArr {
 
 struct emt6_mlp {
   int device = 0, max_batch = 0;
-  int in = EMT6_MLP_IN, in_pad = EMT6_MLP_IN_PAD, H = EMT6_MLP_HIDDEN;
   cudaStream_t stream = nullptr;
   int64_t step = 0;
-  int cur_b = -1;
+  int slot = 0;  // of the running step's loss sum; the step clears the other
   float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
-  // parameters: FP32 masters, Adam moments, BF16 copies (W and W^T)
+  // parameters: FP32 masters, Adam moments, BF16 copies (W; W^T of layers 2, 3)
   DevArr<float> w[3], m[3], v[3], b[3], bm[3], bv[3], w4, m4, v4, b4, mb4, vb4;
   DevArr<__nv_bfloat16> wb[3], wbt[3];
-  // activations for max_batch rows
-  DevArr<__nv_bfloat16> X, XT, Z[3], A[3], AT[3], dZ[3], dZT[3];
-  DevArr<float> y, dy, loss, gradw[3], gradv[5], work;
+  // operands of the weight gradients, [columns][max_batch]
+  DevArr<__nv_bfloat16> XT, AT[3], dZT[3];
+  DevArr<__nv_bfloat16> Z[3];  // pre-activations, [max_batch][512]
+  DevArr<float> dy, loss, gradw[3], gradv[5];
   int split_override = 0;  // 0: choose per batch size
   DevArr<int> err;
-  CUtensorMap mX, mXT, mA[3], mAT[3], mW[3], mWT[3], mdZ[3], mdZT[3];
+  CUtensorMap mXT, mAT[2], mW[3], mWT[3], mdZT[3];
 };
 
 namespace {
@@ -705,30 +1118,6 @@ int fail(const std::string &m, int code = EMT6_ERR_DEVICE) { return emt6::set_er
 
 int cuda_fail(cudaError_t e, const char *what) {
   return fail(std::string(what) + ": " + cudaGetErrorString(e), EMT6_ERR_CUDA);
-}
-
-EpiArgs base_args(emt6_mlp *net, int M, int N) {
-  EpiArgs ep;
-  std::memset(&ep, 0, sizeof(ep));
-  ep.M = M;
-  ep.N = N;
-  ep.err = net->err.p;
-  return ep;
-}
-
-// forward hidden layers for B rows already packed into X / X^T
-int forward_hidden(emt6_mlp *net, int B) {
-  for (int l = 0; l < 3; ++l) {
-    EpiArgs ep = base_args(net, B, net->H);
-    ep.bias = net->b[l].p;
-    ep.z_out = net->Z[l].p;
-    ep.a_out = net->A[l].p;
-    ep.a_out_t = net->AT[l].p;
-    const CUtensorMap &a = l == 0 ? net->mX : net->mA[l - 1];
-    cudaError_t e = launch_gemm<EPI_BIAS_GELU>(a, net->mW[l], B, net->H, cols_of(l), ep, net->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "surrogate forward GEMM");
-  }
-  return EMT6_OK;
 }
 
 int check_batch(emt6_mlp *net, int B) {
@@ -747,17 +1136,14 @@ int read_err(emt6_mlp *net) {
   return EMT6_OK;
 }
 
-// maps depend on the batch size through the activation shapes
-bool build_maps(emt6_mlp *net, int B) {
-  bool ok = make_map(&net->mX, net->X.p, B, net->in_pad) &&
-            make_map(&net->mXT, net->XT.p, net->in_pad, B);
+// every map covers a whole allocation: batches use its first rows or columns
+bool build_maps(emt6_mlp *net) {
+  bool ok = make_map(&net->mXT, net->XT.p, INP, net->max_batch);
   for (int l = 0; l < 3 && ok; ++l) {
-    ok = make_map(&net->mA[l], net->A[l].p, B, net->H) &&
-         make_map(&net->mAT[l], net->AT[l].p, net->H, B) &&
-         make_map(&net->mW[l], net->wb[l].p, rows_of(l), cols_of(l)) &&
-         make_map(&net->mWT[l], net->wbt[l].p, cols_of(l), rows_of(l)) &&
-         make_map(&net->mdZ[l], net->dZ[l].p, B, net->H) &&
-         make_map(&net->mdZT[l], net->dZT[l].p, net->H, B);
+    ok = make_map(&net->mW[l], net->wb[l].p, rows_of(l), cols_of(l)) &&
+         make_map(&net->mdZT[l], net->dZT[l].p, HID, net->max_batch);
+    if (l < 2) ok = ok && make_map(&net->mAT[l], net->AT[l].p, HID, net->max_batch);
+    if (l > 0) ok = ok && make_map(&net->mWT[l], net->wbt[l].p, cols_of(l), rows_of(l));
   }
   return ok;
 }
@@ -772,90 +1158,105 @@ int weight_splits(const emt6_mlp *net, int B) {
   return 1;
 }
 
-int backward(emt6_mlp *net, int B, const float *d_target, bool apply, float lr) {
-  cudaStream_t st = net->stream;
-  cudaError_t e;
-  float *loss = net->loss.p;
-  // the loss sum was zeroed by the input packing of this step
-  e = launch_pdl(head_y_kernel, dim3(B / 8), dim3(256), 0, st, (const __nv_bfloat16 *)net->A[2].p,
-                 (const float *)net->w4.p, (const float *)net->b4.p, B, net->H, d_target,
-                 net->y.p, net->dy.p, loss);
-  if (e == cudaSuccess)
-    e = launch_pdl(head_dz_kernel, dim3(B / 32, net->H / 64), dim3(256), 0, st,
-                   (const __nv_bfloat16 *)net->Z[2].p, (const float *)net->w4.p,
-                   (const float *)net->dy.p, B, net->H, net->dZ[2].p, net->dZT[2].p);
-  if (e != cudaSuccess) return cuda_fail(e, "surrogate head");
-  ++net->step;
-  const float bc1 = 1.0f - std::pow(net->beta1, static_cast<float>(net->step));
-  const float bc2 = 1.0f - std::pow(net->beta2, static_cast<float>(net->step));
-  for (int l = 2; l >= 0; --l) {
-    // dA of the layer below (before W[l] changes), then dW[l]
-    if (l > 0) {
-      EpiArgs ep = base_args(net, B, net->H);
-      ep.z_in = net->Z[l - 1].p;
-      ep.a_out = net->dZ[l - 1].p;
-      ep.a_out_t = net->dZT[l - 1].p;
-      e = launch_gemm<EPI_GELU_BWD>(net->mdZ[l], net->mWT[l], B, net->H, net->H, ep, st);
-      if (e != cudaSuccess) return cuda_fail(e, "surrogate backward GEMM");
-    }
-    const CUtensorMap &bmap = l == 0 ? net->mXT : net->mAT[l - 1];
-    const int N = cols_of(l);
-    const int splits = weight_splits(net, B);
-    if (splits > 1) {
-      // K = B is long and M x N small: split K over `splits` CTAs per tile,
-      // then reduce the partial tiles in a fixed order (deterministic)
-      EpiArgs ep = base_args(net, net->H, N);
-      ep.c_out = net->work.p;
-      e = launch_gemm<EPI_STORE_F32>(net->mdZT[l], bmap, net->H, N, B, ep, st, splits);
-      if (e == cudaSuccess) {
-        e = launch_pdl(adam_reduce_kernel, dim3(N / 32, net->H / 32), dim3(1024), 0, st,
-                       (const float *)net->work.p, splits, net->H, N, net->w[l].p, net->m[l].p,
-                       net->v[l].p, net->wb[l].p, net->wbt[l].p,
-                       apply ? nullptr : net->gradw[l].p, lr, net->beta1, net->beta2, net->eps,
-                       bc1, bc2);
+// rows through the network: predictions, or (with targets) all that the weight
+// gradients need
+int run_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean, const float *std,
+             const float *d_target, float *d_y) {
+  static bool raised[2][64];
+  cudaError_t e = d_target ? raise_smem(mlp_rows_kernel<true>, ROWS_SMEM, raised[1])
+                           : raise_smem(mlp_rows_kernel<false>, ROWS_SMEM, raised[0]);
+  if (e != cudaSuccess) return cuda_fail(e, "surrogate rows");
+  // rows per launch: the kernel counts them in 32 bits
+  const int64_t most = int64_t(1) << 30;
+  for (int64_t at = 0; at < n; at += most) {
+    RowsArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.n = static_cast<int>(n - at < most ? n - at : most);
+    a.x = d_x + at * IN;
+    a.norm = mean != nullptr;
+    if (mean)
+      for (int c = 0; c < IN; ++c) {
+        a.mean[c] = mean[c];
+        a.std[c] = std[c];
       }
-    } else if (apply) {
-      EpiArgs ep = base_args(net, net->H, N);
-      ep.w = net->w[l].p;
-      ep.m = net->m[l].p;
-      ep.v = net->v[l].p;
-      ep.w_bf = net->wb[l].p;
-      ep.w_bf_t = net->wbt[l].p;
-      ep.lr = lr;
-      ep.beta1 = net->beta1;
-      ep.beta2 = net->beta2;
-      ep.eps = net->eps;
-      ep.bc1 = bc1;
-      ep.bc2 = bc2;
-      e = launch_gemm<EPI_ADAM>(net->mdZT[l], bmap, net->H, N, B, ep, st);
+    for (int l = 0; l < 3; ++l) a.b[l] = net->b[l].p;
+    a.w4 = net->w4.p;
+    a.b4 = net->b4.p;
+    a.err = net->err.p;
+    const int grid = (a.n + BM - 1) / BM * CLUSTER;
+    if (d_target) {
+      a.target = d_target;
+      a.dy = net->dy.p;
+      a.loss = net->loss.p + net->slot;
+      a.xt = net->XT.p;
+      for (int l = 0; l < 3; ++l) {
+        a.z[l] = net->Z[l].p;
+        a.at[l] = net->AT[l].p;
+        a.dzt[l] = net->dZT[l].p;
+      }
+      a.ld = static_cast<size_t>(net->max_batch);
+      e = launch_clusters(mlp_rows_kernel<true>, grid, CLUSTER, ROWS_SMEM, net->stream, net->mW[0],
+                          net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], a);
     } else {
-      EpiArgs ep = base_args(net, net->H, N);
-      ep.c_out = net->gradw[l].p;
-      e = launch_gemm<EPI_STORE_F32>(net->mdZT[l], bmap, net->H, N, B, ep, st);
+      a.y = d_y + at;
+      e = launch_clusters(mlp_rows_kernel<false>, grid, CLUSTER, ROWS_SMEM, net->stream, net->mW[0],
+                          net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], a);
     }
-    if (e != cudaSuccess) return cuda_fail(e, "surrogate weight-gradient GEMM");
+    if (e != cudaSuccess) return cuda_fail(e, "surrogate rows");
   }
-  VecAdam vp[5];
-  for (int l = 0; l < 3; ++l)
-    vp[l] = {net->b[l].p, net->bm[l].p, net->bv[l].p, net->dZT[l].p, nullptr,
-             apply ? nullptr : net->gradv[l].p, net->H};
-  vp[3] = {net->w4.p, net->m4.p, net->v4.p, net->AT[2].p, net->dy.p,
-           apply ? nullptr : net->gradv[3].p, net->H};
-  vp[4] = {net->b4.p, net->mb4.p, net->vb4.p, nullptr, net->dy.p,
-           apply ? nullptr : net->gradv[4].p, 1};
-  const int warps = 4 * net->H + 1;
-  e = launch_pdl(vec_adam_kernel, dim3((warps * 32 + 255) / 256), dim3(256), 0, st, vp[0], vp[1],
-                 vp[2], vp[3], vp[4], B, lr, net->beta1, net->beta2, net->eps, bc1, bc2,
-                 apply ? 1 : 0);
-  if (e != cudaSuccess) return cuda_fail(e, "surrogate vector Adam");
-  if (!apply) --net->step;
   return EMT6_OK;
 }
 
-int pack(emt6_mlp *net, const float *d_x, int B) {
-  cudaError_t e = launch_pdl(pack_input_kernel, dim3(B / 32), dim3(256), 0, net->stream, d_x, B,
-                             net->in, net->in_pad, net->X.p, net->XT.p, net->loss.p);
-  return e == cudaSuccess ? EMT6_OK : cuda_fail(e, "surrogate input");
+// weight gradients of the rows just run, with Adam or (apply false) exported
+int run_grads(emt6_mlp *net, int B, bool apply, float lr) {
+  static bool raised[64];
+  cudaError_t e = raise_smem(mlp_grads_kernel, GRADS_SMEM, raised);
+  if (e != cudaSuccess) return cuda_fail(e, "surrogate gradients");
+  GradsArgs a;
+  std::memset(&a, 0, sizeof(a));
+  const float step = static_cast<float>(net->step + 1);
+  for (int l = 0; l < 3; ++l) {
+    a.w[l] = net->w[l].p;
+    a.m[l] = net->m[l].p;
+    a.v[l] = net->v[l].p;
+    a.wb[l] = net->wb[l].p;
+    a.wbt[l] = net->wbt[l].p;
+    a.grad[l] = apply ? nullptr : net->gradw[l].p;
+    a.vec[l] = {net->b[l].p, net->bm[l].p, net->bv[l].p, net->dZT[l].p, apply ? nullptr : net->gradv[l].p, HID};
+  }
+  a.vec[3] = {net->w4.p, net->m4.p, net->v4.p, net->AT[2].p, apply ? nullptr : net->gradv[3].p, HID};
+  a.vec[4] = {net->b4.p, net->mb4.p, net->vb4.p, nullptr, apply ? nullptr : net->gradv[4].p, 1};
+  a.dy = net->dy.p;
+  a.clear = net->loss.p + (net->slot ^ 1);
+  a.ld = static_cast<size_t>(net->max_batch);
+  a.B = B;
+  a.splits = weight_splits(net, B);
+  a.lr = lr;
+  a.beta1 = net->beta1;
+  a.beta2 = net->beta2;
+  a.eps = net->eps;
+  a.bc1 = 1.0f - std::pow(net->beta1, step);
+  a.bc2 = 1.0f - std::pow(net->beta2, step);
+  a.err = net->err.p;
+  // at most two parts per CTA (two accumulators, two tiles of shared memory),
+  // and clusters of 4, 36 of which are resident at once
+  const int cluster = a.splits < 4 ? a.splits : 4;
+  e = launch_clusters(mlp_grads_kernel, GRAD_TILES * cluster, cluster, GRADS_SMEM, net->stream,
+                      net->mdZT[0], net->mdZT[1], net->mdZT[2], net->mXT, net->mAT[0], net->mAT[1], a,
+                      cluster);
+  if (e != cudaSuccess) return cuda_fail(e, "surrogate gradients");
+  if (apply) ++net->step;
+  return EMT6_OK;
+}
+
+// The batch's mean squared error; the next batch sums into the other slot.
+int read_loss(emt6_mlp *net, int B, int slot, float *h_loss) {
+  float s = 0.0f;
+  cudaError_t e = cudaMemcpyAsync(&s, net->loss.p + slot, 4, cudaMemcpyDeviceToHost, net->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(net->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "surrogate loss");
+  *h_loss = s / static_cast<float>(B);
+  return EMT6_OK;
 }
 
 int refresh_bf16(emt6_mlp *net) {
@@ -874,20 +1275,22 @@ void param_arrays(emt6_mlp *net, float *dev[8], size_t cnt[8]) {
     dev[2 * l] = net->w[l].p;
     cnt[2 * l] = static_cast<size_t>(rows_of(l)) * cols_of(l);
     dev[2 * l + 1] = net->b[l].p;
-    cnt[2 * l + 1] = net->H;
+    cnt[2 * l + 1] = HID;
   }
   dev[6] = net->w4.p;
-  cnt[6] = net->H;
+  cnt[6] = HID;
   dev[7] = net->b4.p;
   cnt[7] = 1;
 }
 
-// Batch-size-dependent maps are rebuilt when B changes.
-int ensure_maps(emt6_mlp *net, int B) {
-  if (net->cur_b == B) return EMT6_OK;
-  if (!build_maps(net, B)) return fail("surrogate: cuTensorMapEncodeTiled failed");
-  net->cur_b = B;
-  return EMT6_OK;
+cudaError_t launch_test_gemm(const CUtensorMap &ma, const CUtensorMap &mb, float *c, int M, int N,
+                             int K, int *err, uint32_t stall_ns, cudaStream_t st) {
+  static bool raised[64];
+  cudaError_t e = raise_smem(mlp_gemm_kernel, GEMM_SMEM, raised);
+  if (e != cudaSuccess) return e;
+  mlp_gemm_kernel<<<dim3(N / BN, M / BM), GEMM_THREADS, GEMM_SMEM, st>>>(ma, mb, K / BK, N, c, err,
+                                                                        stall_ns);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -905,24 +1308,21 @@ int emt6_mlp_create(int max_batch, uint64_t seed, int device, emt6_mlp **out) {
   auto *net = new emt6_mlp();
   net->device = device;
   net->max_batch = max_batch;
-  const int H = net->H;
+  const int H = HID;
   bool ok = cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking) == cudaSuccess;
   for (int l = 0; l < 3 && ok; ++l) {
     const size_t n = static_cast<size_t>(rows_of(l)) * cols_of(l);
     ok = net->w[l].alloc(n) && net->m[l].alloc(n) && net->v[l].alloc(n) && net->b[l].alloc(H) &&
          net->bm[l].alloc(H) && net->bv[l].alloc(H) && net->wb[l].alloc(n) &&
-         net->wbt[l].alloc(n) && net->gradw[l].alloc(n);
+         (l == 0 || net->wbt[l].alloc(n)) && net->gradw[l].alloc(n);
   }
   const size_t BH = static_cast<size_t>(max_batch) * H;
   ok = ok && net->w4.alloc(H) && net->m4.alloc(H) && net->v4.alloc(H) && net->b4.alloc(1) &&
-       net->mb4.alloc(1) && net->vb4.alloc(1) && net->X.alloc(static_cast<size_t>(max_batch) * net->in_pad) &&
-       net->XT.alloc(static_cast<size_t>(max_batch) * net->in_pad) && net->y.alloc(max_batch) &&
-       net->dy.alloc(max_batch) && net->loss.alloc(1) && net->err.alloc(1);
-  for (int l = 0; l < 3 && ok; ++l)
-    ok = net->Z[l].alloc(BH) && net->A[l].alloc(BH) && net->AT[l].alloc(BH) &&
-         net->dZ[l].alloc(BH) && net->dZT[l].alloc(BH);
+       net->mb4.alloc(1) && net->vb4.alloc(1) &&
+       net->XT.alloc(static_cast<size_t>(max_batch) * INP) && net->dy.alloc(max_batch) &&
+       net->loss.alloc(2) && net->err.alloc(1);
+  for (int l = 0; l < 3 && ok; ++l) ok = net->AT[l].alloc(BH) && net->dZT[l].alloc(BH) && net->Z[l].alloc(BH);
   for (int i = 0; i < 5 && ok; ++i) ok = net->gradv[i].alloc(i < 4 ? H : 1);
-  ok = ok && net->work.alloc(static_cast<size_t>(8) * H * H);
   if (!ok) {
     if (net->stream) cudaStreamDestroy(net->stream);
     delete net;
@@ -934,12 +1334,12 @@ int emt6_mlp_create(int max_batch, uint64_t seed, int device, emt6_mlp **out) {
   e = cudaSuccess;
   for (int l = 0; l < 4 && e == cudaSuccess; ++l) {
     const int rows = l < 3 ? rows_of(l) : 1, cols = l < 3 ? cols_of(l) : H;
-    const int fan_in = l == 0 ? net->in : H;
+    const int fan_in = l == 0 ? IN : H;
     std::normal_distribution<float> nd(0.0f, std::sqrt(2.0f / static_cast<float>(fan_in)));
     host.assign(static_cast<size_t>(rows) * cols, 0.0f);
     for (int r = 0; r < rows; ++r)
       for (int c = 0; c < cols; ++c)
-        if (l != 0 || c < net->in) host[static_cast<size_t>(r) * cols + c] = nd(rng);
+        if (l != 0 || c < IN) host[static_cast<size_t>(r) * cols + c] = nd(rng);
     float *dst = l < 3 ? net->w[l].p : net->w4.p;
     e = cudaMemcpy(dst, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice);
   }
@@ -954,11 +1354,12 @@ int emt6_mlp_create(int max_batch, uint64_t seed, int device, emt6_mlp **out) {
   for (size_t i = 0; i < sizeof(zero) / sizeof(zero[0]) && e == cudaSuccess; ++i)
     e = cudaMemset(zero[i], 0, zn[i] * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(net->err.p, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(net->loss.p, 0, 2 * sizeof(float));
   if (e != cudaSuccess) {
     emt6_mlp_destroy(net);
     return cuda_fail(e, "emt6_mlp_create");
   }
-  int rc = refresh_bf16(net);
+  int rc = build_maps(net) ? refresh_bf16(net) : fail("emt6_mlp_create: cuTensorMapEncodeTiled failed");
   if (rc == EMT6_OK) {
     e = cudaStreamSynchronize(net->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "emt6_mlp_create");
@@ -1012,16 +1413,16 @@ int emt6_mlp_get_params(emt6_mlp *net, float *const *host) {
 int emt6_mlp_predict(emt6_mlp *net, const float *d_x, int B, float *d_y) {
   if (!net || !d_x || !d_y) return fail("emt6_mlp_predict: null argument", EMT6_ERR_INVALID);
   cudaSetDevice(net->device);
-  int rc = check_batch(net, B);
-  if (rc == EMT6_OK) rc = ensure_maps(net, B);
-  if (rc == EMT6_OK) rc = pack(net, d_x, B);
-  if (rc == EMT6_OK) rc = forward_hidden(net, B);
-  if (rc != EMT6_OK) return rc;
-  cudaError_t e = launch_pdl(head_y_kernel, dim3(B / 8), dim3(256), 0, net->stream,
-                             (const __nv_bfloat16 *)net->A[2].p, (const float *)net->w4.p,
-                             (const float *)net->b4.p, B, net->H, (const float *)nullptr, d_y,
-                             (float *)nullptr, (float *)nullptr);
-  return e == cudaSuccess ? EMT6_OK : cuda_fail(e, "emt6_mlp_predict");
+  const int rc = check_batch(net, B);
+  return rc == EMT6_OK ? run_rows(net, d_x, B, nullptr, nullptr, nullptr, d_y) : rc;
+}
+
+int emt6_mlp_predict_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean,
+                          const float *std, float *d_y) {
+  if (!net || n < 0 || (n > 0 && (!d_x || !d_y)) || !mean != !std)
+    return fail("emt6_mlp_predict_rows: null or negative argument", EMT6_ERR_INVALID);
+  cudaSetDevice(net->device);
+  return run_rows(net, d_x, n, mean, std, nullptr, d_y);
 }
 
 int emt6_mlp_train_step(emt6_mlp *net, const float *d_x, const float *d_target, int B, float lr,
@@ -1029,20 +1430,14 @@ int emt6_mlp_train_step(emt6_mlp *net, const float *d_x, const float *d_target, 
   if (!net || !d_x || !d_target) return fail("emt6_mlp_train_step: null argument", EMT6_ERR_INVALID);
   cudaSetDevice(net->device);
   int rc = check_batch(net, B);
-  if (rc == EMT6_OK) rc = ensure_maps(net, B);
-  if (rc == EMT6_OK) rc = pack(net, d_x, B);
-  if (rc == EMT6_OK) rc = forward_hidden(net, B);
-  if (rc == EMT6_OK) rc = backward(net, B, d_target, true, lr);
+  const int slot = net->slot;
+  if (rc == EMT6_OK) rc = run_rows(net, d_x, B, nullptr, nullptr, d_target, nullptr);
+  if (rc == EMT6_OK) rc = run_grads(net, B, true, lr);
   if (rc != EMT6_OK) return rc;
-  if (h_loss) {
-    float s = 0.0f;
-    cudaError_t e = cudaMemcpyAsync(&s, net->loss.p, 4, cudaMemcpyDeviceToHost, net->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(net->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "emt6_mlp_train_step");
-    *h_loss = s / static_cast<float>(B);
-    return read_err(net);
-  }
-  return EMT6_OK;
+  net->slot ^= 1;
+  if (!h_loss) return EMT6_OK;
+  rc = read_loss(net, B, slot, h_loss);
+  return rc == EMT6_OK ? read_err(net) : rc;
 }
 
 int emt6_mlp_gradients(emt6_mlp *net, const float *d_x, const float *d_target, int B,
@@ -1051,11 +1446,11 @@ int emt6_mlp_gradients(emt6_mlp *net, const float *d_x, const float *d_target, i
     return fail("emt6_mlp_gradients: null argument", EMT6_ERR_INVALID);
   cudaSetDevice(net->device);
   int rc = check_batch(net, B);
-  if (rc == EMT6_OK) rc = ensure_maps(net, B);
-  if (rc == EMT6_OK) rc = pack(net, d_x, B);
-  if (rc == EMT6_OK) rc = forward_hidden(net, B);
-  if (rc == EMT6_OK) rc = backward(net, B, d_target, false, 0.0f);
+  const int slot = net->slot;
+  if (rc == EMT6_OK) rc = run_rows(net, d_x, B, nullptr, nullptr, d_target, nullptr);
+  if (rc == EMT6_OK) rc = run_grads(net, B, false, 0.0f);
   if (rc != EMT6_OK) return rc;
+  net->slot ^= 1;
   if ((rc = read_err(net)) != EMT6_OK) return rc;
   const float *grad[8] = {net->gradw[0].p, net->gradv[0].p, net->gradw[1].p, net->gradv[1].p,
                           net->gradw[2].p, net->gradv[2].p, net->gradv[3].p, net->gradv[4].p};
@@ -1065,12 +1460,8 @@ int emt6_mlp_gradients(emt6_mlp *net, const float *d_x, const float *d_target, i
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < 8 && e == cudaSuccess; ++i)
     e = cudaMemcpy(host_grads[i], grad[i], cnt[i] * sizeof(float), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && h_loss) {
-    float s = 0.0f;
-    e = cudaMemcpy(&s, net->loss.p, 4, cudaMemcpyDeviceToHost);
-    *h_loss = s / static_cast<float>(B);
-  }
-  return e == cudaSuccess ? EMT6_OK : cuda_fail(e, "emt6_mlp_gradients");
+  if (e != cudaSuccess) return cuda_fail(e, "emt6_mlp_gradients");
+  return h_loss ? read_loss(net, B, slot, h_loss) : EMT6_OK;
 }
 
 int emt6_mlp_set_splitk(emt6_mlp *net, int splits) {
@@ -1101,13 +1492,7 @@ int emt6_test_mlp_gemm(const void *d_a, const void *d_b, float *d_c, int M, int 
   cudaError_t e = cudaMallocAsync(&err, sizeof(int), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
   if (e != cudaSuccess) return cuda_fail(e, "emt6_test_mlp_gemm");
-  EpiArgs ep;
-  std::memset(&ep, 0, sizeof(ep));
-  ep.M = M;
-  ep.N = N;
-  ep.c_out = d_c;
-  ep.err = err;
-  e = launch_gemm<EPI_STORE_F32>(ma, mb, M, N, K, ep, st);
+  e = launch_test_gemm(ma, mb, d_c, M, N, K, err, 0u, st);
   int h = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1134,14 +1519,7 @@ int emt6_test_mlp_gemm_timeout(const void *d_a, const void *d_b, float *d_c, int
   cudaError_t e = cudaMallocAsync(&err, sizeof(int), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
   if (e != cudaSuccess) return cuda_fail(e, "emt6_test_mlp_gemm_timeout");
-  EpiArgs ep;
-  std::memset(&ep, 0, sizeof(ep));
-  ep.M = M;
-  ep.N = N;
-  ep.c_out = d_c;
-  ep.err = err;
-  ep.stall_ns = stall_us * 1000u;
-  e = launch_gemm<EPI_STORE_F32>(ma, mb, M, N, K, ep, st);
+  e = launch_test_gemm(ma, mb, d_c, M, N, K, err, stall_us * 1000u, st);
   int h = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -129,6 +129,7 @@ _SIGNATURES = {
     "emt6_mlp_set_params": (_c.c_int, [_VP, _P(_VP)]),
     "emt6_mlp_get_params": (_c.c_int, [_VP, _P(_VP)]),
     "emt6_mlp_predict": (_c.c_int, [_VP, _VP, _c.c_int32, _VP]),
+    "emt6_mlp_predict_rows": (_c.c_int, [_VP, _VP, _c.c_int64, _VP, _VP, _VP]),
     "emt6_mlp_train_step": (_c.c_int, [_VP, _VP, _VP, _c.c_int32, _c.c_float,
                                        _P(_c.c_float)]),
     "emt6_mlp_gradients": (_c.c_int, [_VP, _VP, _VP, _c.c_int32, _P(_VP), _P(_c.c_float)]),

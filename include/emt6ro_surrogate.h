@@ -52,6 +52,12 @@ int emt6_mlp_get_params(emt6_mlp *net, float *const *host);
 /* d_y[B] = network(d_x[B][100]); asynchronous. */
 int emt6_mlp_predict(emt6_mlp *net, const float *d_x, int B, float *d_y);
 
+/* d_y[n] = network(rows of d_x[n][100]) for any number of rows, in one launch;
+ * with host arrays mean[100] and std[100] (both or neither) the rows are raw
+ * and enter the network as (x - mean) / std in FP32.  Asynchronous. */
+int emt6_mlp_predict_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean,
+                          const float *std, float *d_y);
+
 /* One Adam step (beta1 0.9, beta2 0.999, eps 1e-8, learning rate lr) on the
  * mean squared error of d_x[B][100] against d_target[B].  When h_loss is not
  * NULL, waits and stores the batch's loss (before the update) there. */
