@@ -160,32 +160,34 @@ class Surrogate:
                                             ctypes.byref(loss)))
         return loss.value
 
-    def predict_std(self, x_std) -> np.ndarray:
-        """Network output for standardised rows (any count; padded to 128)."""
+    def _predict_rows(self, x: np.ndarray, mean=None, std=None) -> np.ndarray:
+        """Network output for rows of 100 FP32 features: one upload, one launch
+        for all rows, one read-back; with `mean` and `std` the rows are raw and
+        standardised on the device."""
         torch = self._torch
-        x = np.ascontiguousarray(x_std, np.float32)
         n = len(x)
         out = np.zeros(n, np.float32)
         if n == 0:
             return out
-        xd_all = self._to_dev(x)
+        xd = self._to_dev(x)
         with torch.cuda.stream(self._stream()):
-            yd = torch.empty(self.max_batch, dtype=torch.float32, device=f"cuda:{self.device}")
-            pad = torch.zeros((self.max_batch, N_FEATURES), dtype=torch.float32,
-                              device=f"cuda:{self.device}")
-            for lo in range(0, n, self.max_batch):
-                hi = min(n, lo + self.max_batch)
-                rows = hi - lo
-                B = (rows + 127) // 128 * 128
-                if rows == B:
-                    src = xd_all[lo:hi]
-                else:
-                    pad[:rows].copy_(xd_all[lo:hi])
-                    pad[rows:B].zero_()
-                    src = pad
-                N.check(N.lib().emt6_mlp_predict(self._h, src.data_ptr(), B, yd.data_ptr()))
-                out[lo:hi] = yd[:rows].cpu().numpy()
+            yd = torch.empty(n, dtype=torch.float32, device=f"cuda:{self.device}")
+            N.check(N.lib().emt6_mlp_predict_rows(self._h, xd.data_ptr(), n, N.ptr(mean),
+                                                  N.ptr(std), yd.data_ptr()))
+            torch.from_numpy(out).copy_(yd)
         return out
+
+    def predict_std(self, x_std) -> np.ndarray:
+        """Network output for standardised rows (any count)."""
+        x = np.ascontiguousarray(x_std, np.float32)
+        n = len(x)
+        if n == 0:
+            return np.zeros(0, np.float32)
+        if x.size == n * N_FEATURES:
+            x = x.reshape(n, N_FEATURES)
+        else:
+            x = np.ascontiguousarray(np.broadcast_to(x, (n, N_FEATURES)))
+        return self._predict_rows(x)
 
     # ---- training / inference in living cells -------------------------------
     def fit(self, x, y, epochs: int = 60, lr: float = 1e-3, batch: int = 4096, seed: int = 0,
@@ -264,7 +266,16 @@ class Surrogate:
 
     def predict(self, x) -> np.ndarray:
         """Predicted mean final living-cell count per raw feature row."""
-        return self.predict_std(self._norm_x(x)).astype(np.float64) * self.y_std + self.y_mean
+        x = np.asarray(x, np.float32)
+        m, s = np.asarray(self.x_mean), np.asarray(self.x_std)
+        if x.shape[1:] == m.shape == s.shape == (N_FEATURES,) and \
+                m.dtype == s.dtype == np.float32:
+            # (x - mean) / std on the device, rounded as numpy rounds it
+            y = self._predict_rows(np.ascontiguousarray(x), np.ascontiguousarray(m),
+                                   np.ascontiguousarray(s))
+        else:
+            y = self.predict_std(self._norm_x(x))
+        return y.astype(np.float64) * self.y_std + self.y_mean
 
 
 class SurrogateEnsemble:
