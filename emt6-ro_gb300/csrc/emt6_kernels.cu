@@ -37,6 +37,7 @@ __device__ unsigned long long g_instr_hist[600];  // irradiation bins, then time
 constexpr int kThreads = 96;  // one warp per field
 
 struct Misc {
+  float4 met[4];  // consumption by metabolic mode
   int roi[5];  // r0, c0, h, w, dist
   uint32_t n, n0;
   int has_multi;
@@ -685,6 +686,14 @@ __device__ __forceinline__ uint32_t occurrence(const uint16_t *list, const uint8
   return k;
 }
 
+// diffused site-substeps of `steps` steps with the current ROI: free sites x free
+// substeps + the final ROI pass
+__device__ __forceinline__ void count_diffused(Misc *m, const KParams &p, uint32_t steps) {
+  if (m->roi[2] > 0)
+    m->diffused += steps * (m->nfs * (unsigned long long)p.nfree +
+                            (unsigned long long)m->roi[2] * (unsigned long long)m->roi[3]);
+}
+
 // ---------------------------------------------------------------------------
 // the fused step kernel
 // ---------------------------------------------------------------------------
@@ -712,6 +721,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int plane = L.plane, rows = L.rows, tiles = WIDE ? kNumTiles : kNarrowTiles;
 
+  if (tid < 4) m->met[tid] = make_float4(p.met[tid][0], p.met[tid][1], p.met[tid][2], 0.f);
   for (int64_t item = blockIdx.x;; item += gridDim.x) {
     int64_t sim;
     if (a.queue) {
@@ -762,6 +772,8 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
     uint32_t t = step0;
     bool dirty = true;    // site states changed since the last vacancy snapshot
     bool onchip = false;  // the hot entries hold the cells' clocks
+    uint32_t bin = t / p.res, in_bin = t % p.res;  // dose bin of step t, steps into it
+    uint32_t since = t;   // steps before it are in m->diffused
     for (; t < t_stop; ++t) {
       if (t % 128 == 0) {
         if (onchip) scatter_cells<NT>(list, cells, hot, m->n);
@@ -771,6 +783,8 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
         dirty = true;
       }
       if (t % 32 == 0 || t == step0) {
+        if (tid == 0) count_diffused(m, p, t - since);
+        since = t;
         if (t % 32 == 0) {
           compute_roi<NT>(st, list, colmask, m, H, W);
         } else {
@@ -827,10 +841,6 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
         }
       dirty = false;
       diffuse_step<WIDE>(fld, plane, masks, edge, m, p);
-      // diffused site-substeps: free sites x free substeps + the final ROI pass
-      if (tid == 0 && m->roi[2] > 0)
-        m->diffused += m->nfs * (unsigned long long)p.nfree +
-                       (unsigned long long)m->roi[2] * (unsigned long long)m->roi[3];
       __syncthreads();
 
       // ---- cell update (simulation.cu:84-96) ----
@@ -840,21 +850,25 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
       // sites only after the arbitration), so the arbitration runs only when
       // a ready cell had a vacant neighbour or some cell died.
       bool may_divide = false;
-      const float dose =
-          (t < p.length && t % p.res == 0 && t / p.res < p.bins) ? doses[t / p.res] : 0.f;
+      const float dose = (in_bin == 0 && t < p.length && bin < p.bins) ? doses[bin] : 0.f;
+      if (++in_bin == p.res) {
+        in_bin = 0;
+        ++bin;
+      }
       {
-        // a thread steps the entries it gathered: no other thread touches them
-        // before the barrier below
+        // A thread steps the entries it gathered: no other thread touches them
+        // before the barrier below.  The loop is what the kernel issues most
+        // outside the substeps, so conditions are combined without branches and
+        // a mode's consumption comes from a table on chip.
         for (uint32_t e = tid; e < n; e += NT) {
-          const uint32_t f = hot.fl[e], cls = f & kClass;
-          if (cls == kGone) continue;
-          const uint32_t le = list[e], vac = le >> kSiteBits;
+          const uint32_t f = hot.fl[e], cls = f & kClass, le = list[e];
           const int s = le & kSiteMask;
           float *lv = fld + (s - fo);  // the site in the field window
-          if (cls == kSlow || dose > 0) {
-            const uint32_t r = step_entry(p, m, lv, plane, cells + 3 * s, st + s, hot, e, s, vac, dose,
-                                          t, (uint32_t)sim, a.epoch);
-            may_divide |= ((r & 1u) && vac != 0) || (r & 2u);
+          if (cls >= kSlow || dose > 0) {
+            if (cls == kGone) continue;
+            const uint32_t r = step_entry(p, m, lv, plane, cells + 3 * s, st + s, hot, e, s,
+                                          le >> kSiteBits, dose, t, (uint32_t)sim, a.epoch);
+            may_divide |= ((r & 1u) && (le >> kSiteBits) != 0) || (r & 2u);
             continue;
           }
           const float clk = hot.h0[e], thr = hot.h1[e];
@@ -862,17 +876,24 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
           // update_state, progress_clock and repair_pre (emt6_device.cuh)
           const bool rep = (f & kT) != 0;
           const bool late = rep ? (f & kG) != 0 : clk > thr - p.dt2_h;
-          const bool g1s = late & (cls == 0) & (vac <= 1);
-          uint32_t mode;
-          const bool alive = !(f & kOld) & metabolic_mode(p, l0, l1, l2, g1s, cls == 0 || cls == 8, mode);
+          const bool g1s = late & (cls == 0) & (le < (2u << kSiteBits));
+          const bool q = (l2 < p.quiescence_gi) & !g1s;
+          const bool d = (l2 < p.death_gi) & ((cls & (4u | 16u)) == 0);  // phases G1, G2 only
+          const bool a0 = (l0 >= p.met[0][0]) & (l1 >= p.met[0][1]) & q;
+          const bool a1 = (l0 >= p.met[1][0]) & (l1 >= p.met[1][1]) & q;
+          const bool a2 = (l0 >= p.met[2][0]) & (l1 >= p.met[2][1]) & d;
+          const bool a3 = (l0 >= p.met[3][0]) & (l1 >= p.met[3][1]) & d;
+          const bool grows = a0 | a1, alive = (grows | a2 | a3) & !(f & kOld);
+          const uint32_t mode = grows ? (a0 ? 0u : 1u) : (a2 ? 2u : 3u);
+          const float4 use = m->met[mode];
           const float next = clk + p.dt_h;
-          const bool moves = rep ? clk > 0 : mode < 2;
+          const bool moves = rep ? clk > 0 : grows;
           if (alive) {
-            lv[0] = l0 - met_of(p, mode, 0);
-            lv[plane] = l1 - met_of(p, mode, 1);
-            lv[2 * plane] = l2 - met_of(p, mode, 2);
+            lv[0] = l0 - use.x;
+            lv[plane] = l1 - use.y;
+            lv[2 * plane] = l2 - use.z;
+            hot.fl[e] = (uint8_t)((f & ~3u) | mode);
             if (moves) hot.h0[e] = next;
-            if (mode != (f & 3u)) hot.fl[e] = (uint8_t)((f & ~3u) | mode);
           }
           bool ready = alive & (cls == 16);
           if (!alive | (moves & (next >= thr))) {
@@ -881,7 +902,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
             ready = hot.ready(e) != 0;
             may_divide |= died;
           }
-          may_divide |= ready & (vac != 0);
+          may_divide |= ready & (le >= (1u << kSiteBits));
         }
       }
       if (m->has_multi && wid == 0) {
@@ -1005,6 +1026,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
       __syncthreads();
       continue;
     }
+    if (tid == 0) count_diffused(m, p, t - since);
     if (onchip) scatter_cells<NT>(list, cells, hot, m->n);
     if (m->w0 >= 0) store_window<NT>(fld, gfld, m->w0, plane, W, HW, a.fstride);
     uint4 *os = reinterpret_cast<uint4 *>(a.st + sim * a.sstride);
