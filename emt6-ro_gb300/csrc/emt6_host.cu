@@ -293,7 +293,7 @@ struct emt6_batch {
   bool use_graph = false;
   bool occ_known = false;
   bool resident = false;
-  int sms = 0, per_sm[emt6::kTiers] = {1, 1, 1};
+  int sms = 0, per_sm[emt6::kTiers] = {1, 1};
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_key[5] = {0, 0, 0, 0, 0};
   unsigned long long graph_kernels = 0;
@@ -306,8 +306,8 @@ struct emt6_batch {
   DevBuf<int4> meta;
   DevBuf<int32_t> roi, sim_tumor, sim_protocol, tpl_roi;
   DevBuf<uint8_t> tier;  // per chunk: the launch tier of each simulation
-  cudaStream_t side[2] = {nullptr, nullptr};  // the wide tiers', beside `stream`
-  cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
+  cudaStream_t side = nullptr;  // the wide tier's, beside `stream`
+  cudaEvent_t fork = nullptr, join = nullptr;
   DevBuf<uint32_t> step, horizon, counts, err, ticket, order_hist;
   DevBuf<int64_t> order;  // per chunk: simulations by region, largest first
   DevBuf<unsigned long long> diffused;
@@ -318,11 +318,9 @@ struct emt6_batch {
       DeviceGuard g(device);
       cudaStreamSynchronize(stream);
       if (graph_exec) cudaGraphExecDestroy(graph_exec);
-      for (int k = 0; k < 2; ++k) {
-        if (side[k]) cudaStreamSynchronize(side[k]);
-        if (join[k]) cudaEventDestroy(join[k]);
-        if (side[k]) cudaStreamDestroy(side[k]);
-      }
+      if (side) cudaStreamSynchronize(side);
+      if (join) cudaEventDestroy(join);
+      if (side) cudaStreamDestroy(side);
       if (fork) cudaEventDestroy(fork);
       cudaStreamDestroy(stream);
     }
@@ -411,12 +409,10 @@ struct emt6_batch {
       per_sm[tier] = std::max(emt6::max_ctas_per_sm(kp, tier), 1);
     // A batch that is resident at once needs neither an order nor a queue: its
     // CTAs all start together, at the tier with the fewest per SM too.
-    resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierFull]) * sms;
+    resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierWide]) * sms;
     if (!resident) {
-      for (int k = 0; k < 2; ++k) {
-        EMT6_CUDA(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
-        EMT6_CUDA(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming));
-      }
+      EMT6_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+      EMT6_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
       EMT6_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     }
     occ_known = true;
@@ -444,15 +440,15 @@ struct emt6_batch {
       if (has_horizon && t >= max_horizon) break;
       if (resident) {
         a.order = nullptr;
-        for (int tier : {emt6::kTierNarrow, emt6::kTierFull}) {
+        for (int tier : {emt6::kTierNarrow, emt6::kTierWide}) {
           const int rc = launch(a, end, tier, stream, count);
           if (rc) return rc;
         }
       } else {
-        // The tiers side by side, the largest simulations' first, each on the
-        // simulations expected to fit it: three launches in a row would leave
-        // most SMs idle at the end of each.  What outgrows its tier meanwhile is
-        // finished by the last launch.
+        // The tiers side by side, the larger simulations' first, each on the
+        // simulations expected to fit it: one after the other would leave most
+        // SMs idle at the end of each.  What outgrows the narrow tier meanwhile
+        // is finished by the last launch.
         EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, tier.p, stream));
         *count += 3;
         if (sched == 1)
@@ -460,17 +456,14 @@ struct emt6_batch {
         EMT6_CUDA(cudaEventRecord(fork, stream));
         emt6::RunArgs b = a;
         b.tier_of = tier.p;
-        const int order_of[2] = {emt6::kTierFull, emt6::kTierWide};
-        for (int k = 0; k < 2; ++k) {
-          EMT6_CUDA(cudaStreamWaitEvent(side[k], fork, 0));
-          const int rc = launch(b, end, order_of[k], side[k], count);
-          if (rc) return rc;
-          EMT6_CUDA(cudaEventRecord(join[k], side[k]));
-        }
-        int rc = launch(b, end, emt6::kTierNarrow, stream, count);
+        EMT6_CUDA(cudaStreamWaitEvent(side, fork, 0));
+        int rc = launch(b, end, emt6::kTierWide, side, count);
         if (rc) return rc;
-        for (int k = 0; k < 2; ++k) EMT6_CUDA(cudaStreamWaitEvent(stream, join[k], 0));
-        rc = launch(a, end, emt6::kTierFull, stream, count);
+        EMT6_CUDA(cudaEventRecord(join, side));
+        rc = launch(b, end, emt6::kTierNarrow, stream, count);
+        if (rc) return rc;
+        EMT6_CUDA(cudaStreamWaitEvent(stream, join, 0));
+        rc = launch(a, end, emt6::kTierWide, stream, count);
         if (rc) return rc;
       }
       t = end;

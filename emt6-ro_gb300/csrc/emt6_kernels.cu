@@ -6,8 +6,8 @@
 // stay in global memory, where the few hundred live cells of each resident
 // simulation stay L2-resident.  Two kernels: run_kernel<false> (5 CTAs/SM, a
 // window of at most 40 lattice rows on chip) for regions that fit a tile of 32
-// slots per lane, and run_kernel<true> (4 CTAs/SM, the whole lattice; 3 CTAs/SM
-// for lists longer than 1,500 entries) for larger ones.  Per step (reference cadence,
+// slots per lane, and run_kernel<true> (4 CTAs/SM, the whole lattice) for
+// larger ones.  Per step (reference cadence,
 // src/emt6ro/simulation/simulation.cu:153-166):
 //   t % 128 == 0  rebuild the occupied list        (simulation.cu:41-64)
 //   t % 32  == 0  ROI + circular fixed-value mask   (diffusion.cu:65-100)
@@ -56,18 +56,20 @@ struct Misc {
 __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
 // Rows of the field window and entries of the occupied list on chip, by tier of
-// launch.  kTierNarrow holds the region's rows (35 at most) with room to move, and
-// as many list entries as leave 5 CTAs on an SM; fewer rows or entries would
-// only park simulations.  kTierWide holds the whole lattice and the entries that
-// leave 4 CTAs (12 warps, 3 on each quarter of the SM; with 3 CTAs one quarter
-// has 3 warps and the CTAs wait for it: 23% slower diffusion); longer lists are
-// kTierFull's, 3 CTAs.
+// launch.  kTierNarrow holds the region's rows (35 at most) with room to move,
+// and as many list entries as leave 5 CTAs on an SM; fewer rows or entries would
+// only park simulations.  kTierWide holds the whole lattice and 4 CTAs (12 warps,
+// 3 on each quarter of the SM; with 3 CTAs one quarter has 3 warps and the CTAs
+// wait for it: 23% slower diffusion).  Its list may hold every interior site;
+// what does not fit of the entries' clocks lies in the padding of the cell
+// records, entry by entry (`held` of them are on chip).
 constexpr int kWindowRows = 40;
 constexpr uint32_t kEntryBytes = 4 + 4 + 2 + 1, kMinEntries = 1024;
 
 struct SmemLayout {
   uint32_t fld, st, colmask, masks, edge, misc, h0, h1, list, fl, total;
-  int rows, plane, entries;  // window rows, floats of a field's window, list capacity
+  int rows, plane;    // window rows, floats of a field's window
+  int entries, held;  // list capacity, entries with their clocks on chip
 };
 
 __host__ __device__ inline SmemLayout smem_layout(int H, int W, int lcap, int tier) {
@@ -87,19 +89,23 @@ __host__ __device__ inline SmemLayout smem_layout(int H, int W, int lcap, int ti
   L.edge = o; o += 3u * (wide ? kEdgeWide : kEdgeNarrow) * 4u;
   L.misc = o; o += align_up(sizeof(Misc), 16);
   // a rebuilt list holds at most the interior, and 128 divisions can follow
-  L.entries = lcap - 128;
-  if (tier != kTierFull) {
-    const uint32_t room = tier == kTierNarrow ? 44u * 1024u : 55u * 1024u + 512u;
-    const uint32_t left = o < room ? (room - o) / kEntryBytes : 0u;
-    const uint32_t fit = left > kMinEntries ? left : kMinEntries;
-    if (fit < (uint32_t)L.entries) L.entries = (int)fit;
+  const uint32_t all = align_up((uint32_t)lcap - 128u, 16), room = (wide ? 111u : 88u) * 512u;
+  const uint32_t left = o < room ? room - o : 0u;
+  uint32_t entries = all, held;
+  if (wide) {
+    held = left > 3u * all ? (left - 3u * all) / 8u : 0u;
+  } else {
+    held = left / kEntryBytes;
   }
-  L.entries &= ~15;  // keeps the arrays aligned
-  if (tier == kTierFull) L.entries = (lcap - 128 + 15) & ~15;
-  L.h0 = o; o += (uint32_t)L.entries * 4u;
-  L.h1 = o; o += (uint32_t)L.entries * 4u;
-  L.list = o; o += (uint32_t)L.entries * 2u;
-  L.fl = o; o += (uint32_t)L.entries;
+  held = held > kMinEntries ? held & ~15u : kMinEntries;
+  if (held > all) held = all;
+  if (!wide) entries = held;
+  L.entries = (int)entries;
+  L.held = (int)held;
+  L.h0 = o; o += held * 4u;
+  L.h1 = o; o += held * 4u;
+  L.list = o; o += entries * 2u;
+  L.fl = o; o += entries;
   L.total = o;
   return L;
 }
@@ -531,14 +537,28 @@ constexpr uint32_t kClass = 7u << 2, kSlow = 6u << 2, kGone = 7u << 2;
 struct Hot {
   float *h0, *h1;
   uint8_t *fl;
+  float4 *cells;  // the simulation's records
+  uint32_t held;  // entries from here on have their clocks in the records' padding
+  __device__ __forceinline__ float2 *spill(uint32_t e) const {
+    return reinterpret_cast<float2 *>(cells + 3 * e + 2) + 1;
+  }
+  __device__ __forceinline__ float clock(uint32_t e) const { return e < held ? h0[e] : spill(e)->x; }
+  __device__ __forceinline__ void set(uint32_t e, float clk, float thr) const {
+    if (e < held) {
+      h0[e] = clk;
+      h1[e] = thr;
+    } else {
+      *spill(e) = make_float2(clk, thr);
+    }
+  }
   __device__ __forceinline__ void idle(uint32_t e, uint32_t cls, uint32_t ready) const {
     fl[e] = (uint8_t)cls;
-    h0[e] = __uint_as_float(ready);
+    set(e, __uint_as_float(ready), 0.f);
   }
   // kReady | occurrence of a cell that is ready to divide, else 0
   __device__ __forceinline__ uint32_t ready(uint32_t e) const {
     const uint32_t cls = fl[e] & kClass;
-    return cls < kSlow ? (cls == 16u ? kReady : 0u) : __float_as_uint(h0[e]);
+    return cls < kSlow ? (cls == 16u ? kReady : 0u) : __float_as_uint(clock(e));
   }
 };
 
@@ -547,22 +567,22 @@ __device__ __forceinline__ void classify(const KParams &p, const DCell &c, const
   const float lim = c.t4 - p.dt_h;
   const bool old = c.prolif >= lim;
   uint32_t f = kSlow;
-  float h0 = 0.f;
+  float h0 = 0.f, h1 = 0.f;
   if (c.mode <= 3 && c.phase <= 4) {
     if (c.tir == 0) {
       // (the G1/S check reads the end of phase 0 itself)
       if (c.phase != 0 || tc <= lim) {
         f = c.mode | (c.phase << 2) | (old ? kOld : 0u);
         h0 = c.prolif;
-        h.h1[e] = fminf(tc, lim);
+        h1 = fminf(tc, lim);
       }
     } else if (!old) {
       f = c.mode | (c.phase << 2) | kT | (c.prolif > c.t0 - p.dt2_h ? kG : 0u);
       h0 = c.tir;
-      h.h1[e] = c.delay;
+      h1 = c.delay;
     }
   }
-  h.h0[e] = h0;
+  h.set(e, h0, h1);
   h.fl[e] = (uint8_t)f;
 }
 
@@ -571,7 +591,7 @@ __device__ __forceinline__ DCell merged_cell(const float4 *rec, const Hot &h, ui
   DCell c = load_cell(rec);
   const uint32_t f = h.fl[e];
   if ((f & kClass) < kSlow) {
-    (f & kT ? c.tir : c.prolif) = h.h0[e];
+    (f & kT ? c.tir : c.prolif) = h.clock(e);
     c.mode = f & 3u;
     c.phase = (f & kClass) >> 2;
   }
@@ -582,6 +602,13 @@ __device__ __forceinline__ DCell merged_cell(const float4 *rec, const Hot &h, ui
 __device__ __forceinline__ void store_clocks(float4 *rec, const DCell &c) {
   rec[0] = make_float4(c.prolif, c.tir, c.irr, c.delay);
   reinterpret_cast<uint32_t *>(rec + 2)[1] = c.mode | (c.phase << 8);
+}
+
+// a new cell's record; the padding may hold an entry's clocks
+__device__ __forceinline__ void store_fresh(float4 *rec, const DCell &c) {
+  store_clocks(rec, c);
+  rec[1] = make_float4(c.t0, c.t1, c.t2, c.t3);
+  reinterpret_cast<float *>(rec + 2)[0] = c.t4;
 }
 
 template <int NT>
@@ -615,7 +642,7 @@ __device__ __noinline__ void scatter_cells(const uint16_t *list, float4 *cells, 
     const uint32_t f = h.fl[e];
     if ((f & kClass) >= kSlow) continue;
     float *rec = reinterpret_cast<float *>(cells + 3 * (list[e] & kSiteMask));
-    rec[f & kT ? 1 : 0] = h.h0[e];
+    rec[f & kT ? 1 : 0] = h.clock(e);
     reinterpret_cast<uint32_t *>(rec)[9] = (f & 3u) | ((f & kClass) << 6);
   }
 }
@@ -700,20 +727,20 @@ __device__ __forceinline__ void count_diffused(Misc *m, const KParams &p, uint32
 // WIDE = false: regions that fit a tile of at most 32 slots per lane (discs up
 // to distance 16, clipped regions up to 32 x 32), 5 CTAs/SM.  A simulation it
 // cannot hold (region, window or list) is parked at the start of that step for
-// the WIDE = true kernel: any region, 4 CTAs/SM (3 as kTierFull).
+// the WIDE = true kernel: any simulation, 4 CTAs/SM.
 template <bool WIDE>
-__global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __grid_constant__ RunArgs a, uint32_t t_end, int tier) {
+__global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __grid_constant__ RunArgs a, uint32_t t_end) {
   constexpr int NT = kThreads;
   extern __shared__ __align__(16) uint8_t sm[];
   const KParams &p = a.p;
   const int H = p.H, W = p.W, HW = p.HW;
-  const SmemLayout L = smem_layout(H, W, p.lcap, WIDE ? tier : kTierNarrow);
-  const bool last = WIDE && tier == kTierFull;  // holds every simulation
+  constexpr int TIER = WIDE ? kTierWide : kTierNarrow;
+  const SmemLayout L = smem_layout(H, W, p.lcap, TIER);
   float *fld = reinterpret_cast<float *>(sm + L.fld);
   uint8_t *st = sm + L.st;
   uint16_t *list = reinterpret_cast<uint16_t *>(sm + L.list);
-  const Hot hot = {reinterpret_cast<float *>(sm + L.h0), reinterpret_cast<float *>(sm + L.h1),
-                   sm + L.fl};
+  Hot hot = {reinterpret_cast<float *>(sm + L.h0), reinterpret_cast<float *>(sm + L.h1), sm + L.fl,
+             nullptr, (uint32_t)L.held};
   uint64_t *colmask = reinterpret_cast<uint64_t *>(sm + L.colmask);
   uint32_t *masks = reinterpret_cast<uint32_t *>(sm + L.masks);
   float *edge = reinterpret_cast<float *>(sm + L.edge);
@@ -736,14 +763,14 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
       if (item >= a.nsims) break;
       sim = a.order ? a.order[item] : item;
     }
-    if (a.tier_of && a.tier_of[sim] != tier) continue;  // another concurrent launch's
+    if (a.tier_of && a.tier_of[sim] != TIER) continue;  // another concurrent launch's
     const uint32_t horizon = a.horizon ? a.horizon[sim] : 0xFFFFFFFFu;
     const uint32_t t_stop = t_end < horizon ? t_end : horizon;
     const uint32_t step0 = a.step[sim];
     // nothing to do for a simulation already at its target step
     if (step0 >= t_stop) continue;
     const int4 meta = a.meta[sim];
-    if (!last && meta.x >= L.entries) continue;  // the list does not fit: a later tier's
+    if (!WIDE && meta.x >= L.entries) continue;  // the list does not fit: the wide tier's
 
     // ---- load the simulation into shared memory (its fields when the window
     //      is known) ----
@@ -765,6 +792,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
     }
     cp_async_wait();
     float4 *cells = a.cell + sim * (int64_t)HW * 3;
+    hot.cells = cells;
     const int32_t prot = a.sim_protocol[sim];
     const float *doses = a.doses + (int64_t)prot * p.bins;
     __syncthreads();
@@ -794,13 +822,13 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
         }
         if (wid == 0) tile_mapping(colmask, m, p.layouts, tiles, H, rows);
         __syncthreads();
-        if (last || !m->park) build_masks<WIDE>(masks, colmask, m);
+        if (WIDE || !m->park) build_masks<WIDE>(masks, colmask, m);
         const int w0 = m->w0, need = m->wneed;
         if (w0 != need) {
           // (another) window of the fields; a parked simulation needs none
           if (w0 >= 0) store_window<NT>(fld, gfld, w0, plane, W, HW, a.fstride);
           __syncthreads();
-          if (last || !m->park) {
+          if (WIDE || !m->park) {
             load_window<NT>(fld, gfld, need, plane, W, HW, a.fstride);
             if (tid == 0) m->w0 = need;
           } else if (tid == 0) {
@@ -819,10 +847,10 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
         }
         __syncthreads();
       }
-      // a simulation this launch cannot hold is left for a later tier; the
+      // a simulation the narrow tier cannot hold is left for the wide one; the
       // state stored is the state at the start of step t (the list rebuild and
       // ROI above are recomputed identically there)
-      if (!last && (m->park || m->n >= (uint32_t)L.entries)) break;
+      if (!WIDE && (m->park || m->n >= (uint32_t)L.entries)) break;
       const uint32_t n = m->n;
       const int fo = m->w0 * W;
       if (!onchip) gather_cells<NT>(p, st, list, cells, hot, n);
@@ -860,7 +888,15 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
         // before the barrier below.  The loop is what the kernel issues most
         // outside the substeps, so conditions are combined without branches and
         // a mode's consumption comes from a table on chip.
+        float2 ahead = make_float2(0.f, 0.f);  // clocks of the next entry, if not on chip
         for (uint32_t e = tid; e < n; e += NT) {
+          float clk = ahead.x, thr = ahead.y;
+          const bool here = !WIDE || e < hot.held;
+          if (here) {
+            clk = hot.h0[e];
+            thr = hot.h1[e];
+          }
+          if (WIDE && e + NT >= hot.held && e + NT < n) ahead = *hot.spill(e + NT);
           const uint32_t f = hot.fl[e], cls = f & kClass, le = list[e];
           const int s = le & kSiteMask;
           float *lv = fld + (s - fo);  // the site in the field window
@@ -871,7 +907,6 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
             may_divide |= ((r & 1u) && (le >> kSiteBits) != 0) || (r & 2u);
             continue;
           }
-          const float clk = hot.h0[e], thr = hot.h1[e];
           const float l0 = lv[0], l1 = lv[plane], l2 = lv[2 * plane];
           // update_state, progress_clock and repair_pre (emt6_device.cuh)
           const bool rep = (f & kT) != 0;
@@ -893,7 +928,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
             lv[plane] = l1 - use.y;
             lv[2 * plane] = l2 - use.z;
             hot.fl[e] = (uint8_t)((f & ~3u) | mode);
-            if (moves) hot.h0[e] = next;
+            if (moves) *(here ? hot.h0 + e : &hot.spill(e)->x) = next;
           }
           bool ready = alive & (cls == 16);
           if (!alive | (moves & (next >= thr))) {
@@ -995,10 +1030,10 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
           DCell pc = merged_cell(cells + 3 * parent, hot, pe);
           pc.phase = 0;
           pc.prolif = 0.f;
-          store_cell(cells + 3 * parent, pc);
+          store_clocks(cells + 3 * parent, pc);
           if ((hot.fl[pe] & kClass) != kGone) classify(p, pc, hot, pe);
           const DCell cc = make_child(pc, z, p);
-          store_cell(cells + 3 * child, cc);
+          store_fresh(cells + 3 * child, cc);
           const uint8_t sv = st[child];
           const bool listed = (sv & (kStRebuilt | kStTail)) != 0;
           st[child] = (uint8_t)((sv & (kStRebuilt | kStTail | kStMulti)) | kStTail |
@@ -1022,7 +1057,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
     }
 
     // ---- write the simulation back (nothing changed when the first step parks) ----
-    if (!last && t == step0) {
+    if (!WIDE && t == step0) {
       __syncthreads();
       continue;
     }
@@ -1110,13 +1145,15 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t *hist) {
 
 // The tier expected to hold a simulation, from its stored region and list
 // (or, after a reset, its tumour's): a wrong guess only costs time, the launch
-// after the concurrent ones takes what they leave.
+// after the concurrent ones takes what they leave.  A region at the narrow
+// tiles' limit is given to the wide tier, which runs it nearly as fast: it may
+// grow in the next steps, and what is left for the last launch runs alone.
 __device__ __forceinline__ uint8_t expected_tier(const RunArgs &a, int64_t sim) {
   const int *roi = a.roi + sim * 8;
   const int h = roi[2], w = roi[3], d = roi[4], n = max(a.meta[sim].x, roi[5]) + 64;
-  const bool narrow = (h == 2 * d + 1 && w == h) ? d <= 16 : h + 2 <= 32 && w + 2 <= 32;
+  const bool narrow = (h == 2 * d + 1 && w == h) ? d <= 15 : h + 2 <= 30 && w + 2 <= 30;
   if (narrow && n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierNarrow).entries) return kTierNarrow;
-  return n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierWide).entries ? kTierWide : kTierFull;
+  return kTierWide;
 }
 
 __global__ void order_scatter_kernel(const RunArgs a, uint32_t t_end, uint32_t *hist,
@@ -1247,7 +1284,7 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5)
   constexpr int NT = kThreads;
   extern __shared__ __align__(16) uint8_t sm[];
   const int HW = p.HW;
-  const SmemLayout L = smem_layout(p.H, p.W, p.lcap, WIDE ? kTierFull : kTierNarrow);
+  const SmemLayout L = smem_layout(p.H, p.W, p.lcap, WIDE ? kTierWide : kTierNarrow);
   float *fld = reinterpret_cast<float *>(sm + L.fld);
   uint8_t *st = sm + L.st;
   uint16_t *list = reinterpret_cast<uint16_t *>(sm + L.list);
@@ -1331,9 +1368,9 @@ cudaError_t launch_run(const RunArgs &a, uint32_t t_end, int tier, int grid, cud
   cudaError_t e = ensure_smem(tier != kTierNarrow, smem);
   if (e != cudaSuccess) return e;
   if (tier != kTierNarrow)
-    run_kernel<true><<<grid, kThreads, smem, stream>>>(a, t_end, tier);
+    run_kernel<true><<<grid, kThreads, smem, stream>>>(a, t_end);
   else
-    run_kernel<false><<<grid, kThreads, smem, stream>>>(a, t_end, tier);
+    run_kernel<false><<<grid, kThreads, smem, stream>>>(a, t_end);
   return cudaGetLastError();
 }
 
@@ -1472,7 +1509,7 @@ cudaError_t launch_test_block(const KParams &p, int mode, bool wide, float *fld,
                               const uint8_t *st, int32_t *roi, uint8_t *mask, uint16_t *list,
                               uint32_t *n) {
   wide = wide || mode < 2;  // lists and ROIs of any size
-  const size_t smem = run_kernel_smem(p.H, p.W, p.lcap, wide ? kTierFull : kTierNarrow);
+  const size_t smem = run_kernel_smem(p.H, p.W, p.lcap, wide ? kTierWide : kTierNarrow);
   cudaError_t e;
   if (wide) {
     e = cudaFuncSetAttribute(test_block_kernel<true>,

@@ -53,11 +53,11 @@ struct ResetArgs {
   int64_t nsims;
 };
 
-// Tiers of a step launch.  Run one after another without tier_of, each takes
-// the simulations that the ones before left short of the target step (regions too wide, lists too long
-// for the shared memory that lets 5 or 4 CTAs share an SM).  kTierFull holds any;
-// kTierWide may be skipped.
-enum { kTierNarrow = 0, kTierWide = 1, kTierFull = 2, kTiers = 3 };
+// Tiers of a step launch.  Run one after the other without tier_of, the wide one
+// takes the simulations that the narrow one left short of the target step
+// (regions too wide or lists too long for the shared memory that lets 5 CTAs
+// share an SM); it holds any.
+enum { kTierNarrow = 0, kTierWide = 1, kTiers = 2 };
 size_t run_kernel_smem(int H, int W, int lcap, int tier);
 int max_ctas_per_sm(const KParams &p, int tier);
 // Advance the simulations that `tier` holds to step min(t_end, horizon).

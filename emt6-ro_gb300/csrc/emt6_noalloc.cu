@@ -270,7 +270,7 @@ int emt6_simulate_noalloc(const emt6_params *p, const emt6_site *d_tumors, int32
   if (e != cudaSuccess) return fail(EMT6_ERR_CUDA, cudaGetErrorString(e));
   for (uint32_t t = 0; t < nsteps;) {
     const uint32_t end = nsteps - t > 1200 ? t + 1200 : nsteps;
-    for (int tier : {emt6::kTierNarrow, emt6::kTierFull}) {
+    for (int tier : {emt6::kTierNarrow, emt6::kTierWide}) {
       e = emt6::launch_run(a, end, tier, (int)n_sims, s);
       if (e != cudaSuccess) return fail(EMT6_ERR_CUDA, cudaGetErrorString(e));
     }
