@@ -394,21 +394,27 @@ __device__ __forceinline__ void diffuse_step(float *fld, int plane, const uint32
     diffuse_tile<tile_shape(K).C, tile_shape(K).R, tile_shape(K).RE, tile_shape(K).CE>(           \
         f, masks, WIDE ? kWordsWide : kWordsNarrow, e, tm, r0, c0, w, p.W, ext, ca, cb, cd, p.nfree); \
     break;
+#define EMT6_LARGE(K)                                                                             \
+  case K:                                                                                         \
+    diffuse_large<tile_shape(K).C, tile_shape(K).R, tile_shape(K).RE, tile_shape(K).CE>(          \
+        f, masks, kWordsWide, e, &m->tm, r0, c0, w, p.W, ext, ca, cb, cd, p.nfree);               \
+    break;
   switch (tm.tile) {
     EMT6_TILE(0) EMT6_TILE(1) EMT6_TILE(2) EMT6_TILE(3) EMT6_TILE(4) EMT6_TILE(5)
     EMT6_TILE(6) EMT6_TILE(7) EMT6_TILE(8) EMT6_TILE(9) EMT6_TILE(10) EMT6_TILE(11)
     default:
       if constexpr (WIDE) {
         switch (tm.tile) {
-          EMT6_TILE(12) EMT6_TILE(13) EMT6_TILE(14) EMT6_TILE(15)
-          EMT6_TILE(16) EMT6_TILE(17) EMT6_TILE(18) EMT6_TILE(19)
+          EMT6_TILE(12) EMT6_TILE(13) EMT6_TILE(14) EMT6_TILE(15) EMT6_LARGE(16)
+          EMT6_LARGE(17) EMT6_LARGE(18) EMT6_LARGE(19) EMT6_LARGE(20)
           default: break;
         }
       }
       break;
   }
 #undef EMT6_TILE
-  static_assert(kNumTiles == 20 && kNarrowTiles == 12, "every tile has a case above");
+#undef EMT6_LARGE
+  static_assert(kNumTiles == 21 && kNarrowTiles == 12, "every tile has a case above");
 }
 
 // Field window (rows w0 .. w0 + rows - 1 of the three planes) from and to
