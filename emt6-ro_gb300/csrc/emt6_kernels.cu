@@ -1171,6 +1171,11 @@ __global__ void order_scatter_kernel(const RunArgs a, uint32_t t_end, uint32_t *
   }
 }
 
+__global__ void tier_kernel(const RunArgs a, uint8_t *tier) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < a.nsims) tier[i] = expected_tier(a, i);
+}
+
 // ---------------------------------------------------------------------------
 // reset: expand the initial tumours into every simulation
 // ---------------------------------------------------------------------------
@@ -1390,6 +1395,11 @@ cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64
   order_count_kernel<<<grid, 256, 0, stream>>>(a, t_end, hist);
   order_scan_kernel<<<1, 1024, 0, stream>>>(hist);
   order_scatter_kernel<<<grid, 256, 0, stream>>>(a, t_end, hist, out, tier);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, cudaStream_t stream) {
+  tier_kernel<<<(unsigned)((a.nsims + 127) / 128), 128, 0, stream>>>(a, tier);
   return cudaGetLastError();
 }
 

@@ -69,6 +69,8 @@ cudaError_t launch_reset(const ResetArgs &a, cudaStream_t stream);
 constexpr uint32_t kOrderKeys = 4096;
 cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64_t *out,
                          uint8_t *tier, cudaStream_t stream);
+// the tiers alone, for a batch that needs no order
+cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, cudaStream_t stream);
 cudaError_t instr_read(unsigned long long counts[4], double *sum_dp, unsigned long long *hist);
 cudaError_t instr_reset();
 cudaError_t fp32_peak(int device, double *tflops);
