@@ -255,47 +255,16 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) |
                             (static_cast<uint32_t>(BN >> 3) << 17) |
                             (static_cast<uint32_t>(BM >> 4) << 24);
 
-// GELU and its derivative.  With u = |z|, the normal tail Phi(-u) is evaluated
-// as 2^-(1 + u P(u)): u P(u) = -log2(2 Phi(-u)) is smooth, and P is the weighted
-// minimax polynomial of degree 8 on [0, 6] (Lawson's iteration on Chebyshev
-// nodes, scipy's log_ndtr as the reference), within 2.4e-9 of Phi; the rounding
-// of the FP32 evaluation adds 2e-8, a third of an ulp of 1.  13 and 19
-// instructions in place of about 35 and 60 with erff and expf, on which the
-// epilogues spent most of their issue slots.
-__device__ __forceinline__ float exp2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Phi(-u), u = min(|z|, 6): beyond that it is below 1e-9
-__device__ __forceinline__ float normal_tail(float u) {
-  float p = -3.9834051790421654e-07f;
-  p = fmaf(p, u, 8.099371370917652e-06f);
-  p = fmaf(p, u, -6.745159771526232e-05f);
-  p = fmaf(p, u, 0.0002641645260155201f);
-  p = fmaf(p, u, 1.5400924894493073e-05f);
-  p = fmaf(p, u, -0.0069568706676363945f);
-  p = fmaf(p, u, 0.0524463951587677f);
-  p = fmaf(p, u, 0.4592190086841583f);
-  p = fmaf(p, u, 1.15110445022583f);
-  return exp2_approx(fmaf(-p, u, -1.0f));
-}
-
+// GELU and its derivative, by erff and expf: they round as the library's do, which
+// a cheaper normal tail did not, and an activation that rounds to the other of two
+// BF16 values travels through every layer above.
 __device__ __forceinline__ float gelu(float z) {
-  // z Phi(z) = max(z, 0) - u Phi(-u).  NaN stays NaN (max.NaN), +inf is +inf, and
-  // -inf, which the product form makes -inf * 0, NaN.
-  float m;
-  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(m) : "f"(z));
-  const float u = fminf(fabsf(z), 6.0f);
-  return fmaf(-fmaf(fminf(z, 0.0f), 0.0f, u), normal_tail(u), m);
+  return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
 }
 
 __device__ __forceinline__ float gelu_grad(float z) {
-  // Phi(z) + z phi(z), phi(z) = 2^(-z^2 / (2 ln 2)) / sqrt(2 pi)
-  const float h = normal_tail(fminf(fabsf(z), 6.0f));
-  const float phi = 0.39894228040143268f * exp2_approx(z * z * -0.72134752044448170f);
-  return fmaf(z, phi, z > 0.0f ? 1.0f - h : h);
+  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) +
+         z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
 // C tile (blockIdx.y, blockIdx.x) of C[M,N] = A[M,K] B[N,K]^T in FP32: the
@@ -440,7 +409,7 @@ __device__ __forceinline__ uint32_t act_chunk(int row, int chunk) {
 }
 
 // What bounds it, in cycles of a CTA per layer (4,096 rows): the weight tiles from
-// L2 and the products 5,800, the exchange 4,000, the epilogue 3,700, and training
+// L2 and the products 5,800, the exchange 4,000, the epilogue 5,900, and training
 // 4,600 more for the transposed stores that the weight gradients need; the same
 // at 640 rows, so a latency chain of 57 us (43 us of it predicting: 20).  The
 // phases and the columns of an epilogue are loops, not unrolled: code that each
