@@ -3,8 +3,9 @@
 //
 // All matrix products run on the 5th-generation tensor cores (tcgen05.mma, M =
 // 128, N = 128, K = 16, BF16 in, FP32 accumulators in tensor memory); operands
-// are K-major 64-column blocks in shared memory with the 128-byte swizzle.  A
-// training step is two launches, a prediction one:
+// are 64-column blocks in shared memory with the 128-byte swizzle, K-major for
+// the layers, rows of the batch (MN-major) for the weight gradients.  A training
+// step is two launches, a prediction one:
 //   mlp_rows_kernel   everything that stays within a row: a cluster of 4 CTAs
 //     owns 128 rows, each CTA 128 of the 512 columns of every layer.  It packs
 //     the inputs, runs the hidden layers, the head, and (training) the error
@@ -106,6 +107,17 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+
+// a box from shared memory to global; wait for the reads of it, or for its writes
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
+               ::"l"(map), "r"(x), "r"(y), "r"(src)
+               : "memory");
+}
+
+__device__ __forceinline__ void store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void store_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot),
@@ -255,6 +267,17 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) |
                             (static_cast<uint32_t>(BN >> 3) << 17) |
                             (static_cast<uint32_t>(BM >> 4) << 24);
 
+// The same for operands stored with their reduction dimension outermost (weight
+// gradients: rows of the batch): boxes of 64 columns x 64 rows with the 128-byte
+// swizzle, two of them for 128 columns (leading offset), 8-row atoms (stride).
+constexpr int BOX_BYTES = BK * 64 * 2;
+__device__ __forceinline__ uint64_t mn_desc(uint32_t saddr) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) |
+         (static_cast<uint64_t>(BOX_BYTES >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+         (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
+}
+constexpr uint32_t kIdescMN = kIdesc | (1u << 15) | (1u << 16);
+
 // GELU and its derivative, by erff and expf: they round as the library's do, which
 // a cheaper normal tail did not, and an activation that rounds to the other of two
 // BF16 values travels through every layer above.
@@ -391,10 +414,16 @@ struct RowsArgs {
   // training
   const float *target;
   float *dy, *loss;
-  __nv_bfloat16 *z[3];                 // pre-activations, [n][512]
-  __nv_bfloat16 *xt, *at[3], *dzt[3];  // transposed, [columns][ld]
+  uint4 *z[3];         // pre-activations, 8 columns of a row each (z_at)
+  __nv_bfloat16 *x16;  // [n][128]
+  float *part;         // sums of 32 rows: [dZ1, dZ2, dZ3, A3 dy][512][ld]
   size_t ld;
   int *err;
+};
+
+// where training's operands of the weight gradients go, [n][512]
+struct RowsMaps {
+  CUtensorMap a[2], dz[3];
 };
 
 // shared memory of mlp_rows_kernel: the 8 blocks of the current operand, the
@@ -409,9 +438,10 @@ __device__ __forceinline__ uint32_t act_chunk(int row, int chunk) {
 }
 
 // What bounds it, in cycles of a CTA per layer (4,096 rows): the weight tiles from
-// L2 and the products 5,800, the exchange 4,000, the epilogue 5,900, and training
-// 4,600 more for the transposed stores that the weight gradients need; the same
-// at 640 rows, so a latency chain of 57 us (43 us of it predicting: 20).  The
+// L2 and the products 5,800, the exchange 4,000, the epilogue 5,900: a latency
+// chain, as long at 640 rows.  Training's operands of the weight gradients leave
+// by bulk copies of the operand blocks that the exchange needs anyway, as rows;
+// transposed from registers they took 4,600 a layer.  The
 // phases and the columns of an epilogue are loops, not unrolled: code that each
 // warp runs once is fetched as it goes.  With one launch per layer, and input,
 // head and error launches between, a step's rows took 75 us of GPU time.
@@ -419,7 +449,8 @@ template <bool TRAIN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     mlp_rows_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                     const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmT1,
-                    const __grid_constant__ CUtensorMap tmT2, const __grid_constant__ RowsArgs a) {
+                    const __grid_constant__ CUtensorMap tmT2, const __grid_constant__ RowsMaps out,
+                    const __grid_constant__ RowsArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                               ~static_cast<uintptr_t>(1023));
@@ -525,21 +556,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
     for (int q = 0; q < 8; ++q) v[q] = __float2bfloat16_rn(f[q]);
     *reinterpret_cast<uint4 *>(smem + act_chunk(r, chunk)) = *reinterpret_cast<const uint4 *>(v);
+    if (TRAIN)
+      *reinterpret_cast<uint4 *>(a.x16 + static_cast<size_t>(m0 + r) * INP + 8 * chunk) =
+          *reinterpret_cast<const uint4 *>(v);
   }
   // 32 rows of the 2 blocks
   exchange(rank * (BM / CLUSTER) * 128, BM / CLUSTER * 128, INP / BK, TILE_BYTES);
-  const auto act_at = [&](int row, int col) -> __nv_bfloat16 {
-    return *reinterpret_cast<const __nv_bfloat16 *>(smem + act_chunk(row, col >> 3) + (col & 7) * 2);
-  };
-  if (TRAIN) {
-    // this CTA's quarter of X^T
-    if (!arrived()) failed = true;
-    for (int i = tid; i < (INP / CLUSTER) * BM; i += GEMM_THREADS) {
-      const int c = static_cast<int>(rank) * (INP / CLUSTER) + i / BM, r = i % BM;
-      a.xt[static_cast<size_t>(c) * a.ld + m0 + r] = act_at(r, c);
-    }
-  }
-
   const int quarter = warp & 3, group = warp >> 2;
   const int row = quarter * 32 + lane, col0 = n0 + group * 32;  // this thread's row, columns col0..+31
   const uint32_t acc0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + group * 32;
@@ -548,13 +570,38 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     *reinterpret_cast<uint4 *>(smem + act_chunk(row, col0 / 8 + j)) = v;
   };
   const uint32_t own = rank * (BN / BK) * TILE_BYTES;  // this CTA's two blocks of it
-  const auto store_t = [&](__nv_bfloat16 *t, int j, const uint4 &v) {
-    const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
+  // these two blocks at shared address `from` to rows of global memory
+  const auto store_rows = [&](const CUtensorMap *map, uint32_t from) {  // thread 0
 #pragma unroll
-    for (int i = 0; i < 8; ++i) t[static_cast<size_t>(col0 + 8 * j + i) * a.ld + m0 + row] = e[i];
+    for (int i = 0; i < 4; ++i)
+      tma_store_2d(map, from + i * BOX_BYTES, n0 + (i >> 1) * BK, m0 + (i & 1) * 64);
+    store_commit();
   };
+  // each thread reads back what it wrote: laid out so that a warp's are adjacent
   const auto z_at = [&](int l, int j) -> uint4 & {
-    return *reinterpret_cast<uint4 *>(a.z[l] + static_cast<size_t>(m0 + row) * HID + col0 + 8 * j);
+    return a.z[l][(static_cast<size_t>(blockIdx.x) * 16 + group * 4 + j) * BM + row];
+  };
+  // sums of the warp's 32 rows of 8 columns: 4 lanes end up with the same column
+  const auto sum_rows = [&](int k, int j, float (&v)[8]) {
+#pragma unroll
+    for (int n = 4, o = 16; n; n >>= 1, o >>= 1)
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float keep = lane & o ? v[i + n] : v[i], send = lane & o ? v[i] : v[i + n];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    if (!(lane & 3))
+      a.part[static_cast<size_t>(k * HID + col0 + 8 * j + (lane >> 4 & 1) * 4 + (lane >> 3 & 1) * 2 +
+                                 (lane >> 2 & 1)) * a.ld + m0 / 32 + quarter] = v[0];
+  };
+  const auto sum_dz = [&](int l, int j, const uint4 &v) {
+    const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
+    float f[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(e[i]);
+    sum_rows(l, j, f);
   };
 
   int used = 0;  // weight tiles consumed by earlier phases
@@ -591,6 +638,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (tid == 0 && phase + 1 < PHASES) load_tiles(phase + 1, 0, RING);
     __syncwarp();
     const bool last = TRAIN && phase == PHASES - 1;  // the lowest layer's error goes no further
+    if (TRAIN && tid == 0) store_read();  // the operand's own blocks are overwritten next
     if (!last) cluster_meet();  // every CTA's products have read the operand and its copies
     // ---- epilogue
     if (phase < 3) {
@@ -611,10 +659,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
         const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
         publish(j, hv);
-        if (TRAIN) {
-          z_at(phase, j) = *reinterpret_cast<const uint4 *>(zb);
-          store_t(a.at[phase], j, hv);
-        }
+        if (TRAIN) z_at(phase, j) = *reinterpret_cast<const uint4 *>(zb);
       }
     } else {
       const int l = phase == 3 ? 1 : 0;  // layer whose pre-activations the error passes
@@ -628,13 +673,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
         for (int i = 0; i < 8; ++i) h[i] = __float2bfloat16_rn(v[i] * gelu_grad(__bfloat162float(zb[i])));
         const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
-        if (!last) publish(j, hv);
-        store_t(a.dzt[l], j, hv);
+        if (!last)
+          publish(j, hv);
+        else  // the ring is free; a peer's copy of this CTA's operand blocks may not be done
+          *reinterpret_cast<uint4 *>(smem + ACT_BYTES + act_chunk(row, group * 4 + j)) = hv;
+        sum_dz(l, j, hv);
       }
     }
-    if (last) break;
+    if (last) {
+      fence_async();
+      __syncthreads();
+      if (tid == 0) store_rows(&out.dz[0], ring);
+      break;
+    }
     tc_fence_before();
     exchange(own, BN / BK * TILE_BYTES, 1, 0);
+    if (TRAIN && phase != 2 && tid == 0) store_rows(phase < 2 ? &out.a[phase] : &out.dz[1], act + own);
     if (phase == 2) {
       if (!arrived()) failed = true;
       // ---- head: y = A3 w4 + b4, one warp per row
@@ -680,18 +734,26 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
           const float4 w0 = __ldg(reinterpret_cast<const float4 *>(a.w4 + col0 + 8 * j)),
                        w1 = __ldg(reinterpret_cast<const float4 *>(a.w4 + col0 + 8 * j + 4));
           const float wj[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+          const uint4 aq = *reinterpret_cast<const uint4 *>(smem + act_chunk(row, col0 / 8 + j));
+          const __nv_bfloat16 *ab = reinterpret_cast<const __nv_bfloat16 *>(&aq);
+          float gw[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) gw[i] = __bfloat162float(ab[i]) * d;
+          sum_rows(3, j, gw);
 #pragma unroll
           for (int i = 0; i < 8; ++i)
             h[i] = __float2bfloat16_rn(d * wj[i] * gelu_grad(__bfloat162float(zb[i])));
           const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
           publish(j, hv);
-          store_t(a.dzt[2], j, hv);
+          sum_dz(2, j, hv);
         }
         exchange(own, BN / BK * TILE_BYTES, 1, 0);
+        if (tid == 0) store_rows(&out.dz[2], act + own);
       }
     }
   }
   // no CTA leaves while a peer may still read from or write to it
+  if (TRAIN && tid == 0) store_wait();
   cluster_meet();
   pdl_trigger();
   if (*abort || failed) {
@@ -713,7 +775,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 // ---- weight gradients and Adam -------------------------------------------------------
 struct VecAdam {
   float *w, *m, *v;
-  const __nv_bfloat16 *rows;  // [n][ld] rows to sum (bias: dZ^T), or A3^T for w4; null: b4
+  const float *rows;  // [n][ld] partial sums; null: b4
   float *grad_out;
   int n;
 };
@@ -732,18 +794,19 @@ struct GradsArgs {
 };
 
 // Gradients and Adam updates of elements e, e + stride, .. (VEC_U of them, below
-// VEC_ELEMS) of the vectors b1, b2, b3 (row sums of dZ^T), w4 (A3^T dy) and b4
-// (sum dy).  One warp; the elements' loads overlap, and lane u updates the u-th.
+// VEC_ELEMS) of the vectors b1, b2, b3, w4 (sums over the batch from the rows
+// kernel's sums of 32 rows) and b4 (sum dy).  One warp; the elements' loads
+// overlap, and lane u updates the u-th.
 constexpr int VEC_ELEMS = 4 * HID + 1, VEC_U = 4;
 __device__ __forceinline__ void vec_adam(const GradsArgs &a, int e, int stride, int lane) {
-  const uint4 *rows[VEC_U];
+  const float4 *rows[VEC_U];
   float g[VEC_U], mine = 0.0f;
 #pragma unroll
   for (int u = 0; u < VEC_U; ++u) {
     const int q = e + u * stride, k = q / HID;
     g[u] = 0.0f;
     rows[u] = k < 4 && q < VEC_ELEMS
-                  ? reinterpret_cast<const uint4 *>(a.vec[k].rows + static_cast<size_t>(q % HID) * a.ld)
+                  ? reinterpret_cast<const float4 *>(a.vec[k].rows + static_cast<size_t>(q % HID) * a.ld)
                   : nullptr;
   }
   // this lane's element (lanes 0 .. VEC_U - 1)
@@ -756,28 +819,15 @@ __device__ __forceinline__ void vec_adam(const GradsArgs &a, int e, int stride, 
     v0 = p.v[idx];
     w0 = p.w[idx];
   }
-  // B is a multiple of 128: 8 BF16 (16 bytes) per lane per load
-  for (int j = lane; j < a.B / 8; j += 32) {
-    uint4 r[VEC_U];
+  // B is a multiple of 128: 4 sums (16 bytes) per lane per load
+  for (int j = lane; j < a.B / 128; j += 32) {
+    float4 r[VEC_U];
 #pragma unroll
     for (int u = 0; u < VEC_U; ++u)
       if (rows[u]) r[u] = rows[u][j];
 #pragma unroll
-    for (int u = 0; u < VEC_U; ++u) {
-      if (!rows[u]) continue;
-      const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&r[u]);
-      if ((e + u * stride) / HID == 3) {
-        const float4 d0 = reinterpret_cast<const float4 *>(a.dy)[2 * j];
-        const float4 d1 = reinterpret_cast<const float4 *>(a.dy)[2 * j + 1];
-        g[u] += __bfloat162float(h[0]) * d0.x + __bfloat162float(h[1]) * d0.y +
-                __bfloat162float(h[2]) * d0.z + __bfloat162float(h[3]) * d0.w +
-                __bfloat162float(h[4]) * d1.x + __bfloat162float(h[5]) * d1.y +
-                __bfloat162float(h[6]) * d1.z + __bfloat162float(h[7]) * d1.w;
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) g[u] += __bfloat162float(h[i]);
-      }
-    }
+    for (int u = 0; u < VEC_U; ++u)
+      if (rows[u]) g[u] += (r[u].x + r[u].y) + (r[u].z + r[u].w);
   }
 #pragma unroll
   for (int u = 0; u < VEC_U; ++u) {
@@ -811,7 +861,8 @@ static_assert(RED_BYTES >= STAGES * 2 * TILE_BYTES, "the partial tiles replace t
 // each with an accumulator of its own), lay the partial tiles down in shared
 // memory, and each sums a share of the rows over all parts in order, applies
 // Adam and writes W and W^T.  Warps that do not feed the tensor cores compute
-// the vectors' gradients meanwhile.  Bound by L2 reads at 4,096 rows (75 MB of
+// the vectors' gradients meanwhile, from the rows kernel's sums of 32 rows (they
+// read every operand once more before).  Bound by L2 reads at 4,096 rows (75 MB of
 // operands in 9.5 us); 15 us in all, where the seven launches it replaces took
 // 40.
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -865,8 +916,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         break;
       }
       mbar_expect_tx(full0 + 8 * s, 2 * TILE_BYTES);
-      tma_load_2d(ringA + s * TILE_BYTES, ma, full0 + 8 * s, (kb0 + kb) * BK, m0);
-      tma_load_2d(ringB + s * TILE_BYTES, mb, full0 + 8 * s, (kb0 + kb) * BK, n0);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t at = s * TILE_BYTES + i * BOX_BYTES;
+        tma_load_2d(ringA + at, ma, full0 + 8 * s, m0 + 64 * i, (kb0 + kb) * BK);
+        tma_load_2d(ringB + at, mb, full0 + 8 * s, n0 + 64 * i, (kb0 + kb) * BK);
+      }
       ++issued;
     }
   } else if (tid == 32) {
@@ -880,8 +935,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       const uint32_t pa = ringA + s * TILE_BYTES, pb = ringB + s * TILE_BYTES;
 #pragma unroll
       for (int q = 0; q < BK / 16; ++q)
-        umma_bf16(tmem + static_cast<uint32_t>(kb / nkp) * BN, sw128_desc(pa + 32 * q),
-                  sw128_desc(pb + 32 * q), kIdesc, (kb % nkp | q) != 0 ? 1u : 0u);
+        umma_bf16(tmem + static_cast<uint32_t>(kb / nkp) * BN, mn_desc(pa + 2048 * q),
+                  mn_desc(pb + 2048 * q), kIdescMN, (kb % nkp | q) != 0 ? 1u : 0u);
       umma_commit(empty0 + 8 * s);
     }
     umma_commit(done);  // arrives once every product above has completed
@@ -997,13 +1052,13 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// K-major BF16 matrix [rows][cols] (cols = K contiguous), boxes of 128 rows x 64 columns.
-bool make_map(CUtensorMap *map, const void *base, int rows, int cols) {
+// BF16 matrix [rows][cols], boxes of 64 columns x `high` rows.
+bool make_map(CUtensorMap *map, const void *base, int rows, int cols, int high = BM) {
   auto fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
-  cuuint32_t box[2] = {BK, BM};
+  cuuint32_t box[2] = {BK, static_cast<cuuint32_t>(high)};
   cuuint32_t estr[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box,
             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1069,13 +1124,14 @@ struct emt6_mlp {
   // parameters: FP32 masters, Adam moments, BF16 copies (W; W^T of layers 2, 3)
   DevArr<float> w[3], m[3], v[3], b[3], bm[3], bv[3], w4, m4, v4, b4, mb4, vb4;
   DevArr<__nv_bfloat16> wb[3], wbt[3];
-  // operands of the weight gradients, [columns][max_batch]
-  DevArr<__nv_bfloat16> XT, AT[3], dZT[3];
-  DevArr<__nv_bfloat16> Z[3];  // pre-activations, [max_batch][512]
+  DevArr<__nv_bfloat16> X16, A[2], dZ[3];  // operands of the weight gradients, [max_batch][columns]
+  DevArr<uint4> Z[3];                      // pre-activations, 8 to an element
+  DevArr<float> part;                      // vector gradients' sums, [4][512][max_batch / 32]
   DevArr<float> dy, loss, gradw[3], gradv[5];
   int split_override = 0;  // 0: choose per batch size
   DevArr<int> err;
-  CUtensorMap mXT, mAT[2], mW[3], mWT[3], mdZT[3];
+  CUtensorMap mX, mW[3], mWT[3];
+  RowsMaps mRows;
 };
 
 namespace {
@@ -1107,11 +1163,11 @@ int read_err(emt6_mlp *net) {
 
 // every map covers a whole allocation: batches use its first rows or columns
 bool build_maps(emt6_mlp *net) {
-  bool ok = make_map(&net->mXT, net->XT.p, INP, net->max_batch);
+  bool ok = make_map(&net->mX, net->X16.p, net->max_batch, INP, 64);
   for (int l = 0; l < 3 && ok; ++l) {
     ok = make_map(&net->mW[l], net->wb[l].p, rows_of(l), cols_of(l)) &&
-         make_map(&net->mdZT[l], net->dZT[l].p, HID, net->max_batch);
-    if (l < 2) ok = ok && make_map(&net->mAT[l], net->AT[l].p, HID, net->max_batch);
+         make_map(&net->mRows.dz[l], net->dZ[l].p, net->max_batch, HID, 64);
+    if (l < 2) ok = ok && make_map(&net->mRows.a[l], net->A[l].p, net->max_batch, HID, 64);
     if (l > 0) ok = ok && make_map(&net->mWT[l], net->wbt[l].p, cols_of(l), rows_of(l));
   }
   return ok;
@@ -1157,19 +1213,16 @@ int run_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean, cons
       a.target = d_target;
       a.dy = net->dy.p;
       a.loss = net->loss.p + net->slot;
-      a.xt = net->XT.p;
-      for (int l = 0; l < 3; ++l) {
-        a.z[l] = net->Z[l].p;
-        a.at[l] = net->AT[l].p;
-        a.dzt[l] = net->dZT[l].p;
-      }
-      a.ld = static_cast<size_t>(net->max_batch);
+      a.x16 = net->X16.p;
+      for (int l = 0; l < 3; ++l) a.z[l] = net->Z[l].p;
+      a.part = net->part.p;
+      a.ld = static_cast<size_t>(net->max_batch / 32);
       e = launch_clusters(mlp_rows_kernel<true>, grid, CLUSTER, ROWS_SMEM, net->stream, net->mW[0],
-                          net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], a);
+                          net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], net->mRows, a);
     } else {
       a.y = d_y + at;
       e = launch_clusters(mlp_rows_kernel<false>, grid, CLUSTER, ROWS_SMEM, net->stream, net->mW[0],
-                          net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], a);
+                          net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], net->mRows, a);
     }
     if (e != cudaSuccess) return cuda_fail(e, "surrogate rows");
   }
@@ -1184,6 +1237,8 @@ int run_grads(emt6_mlp *net, int B, bool apply, float lr) {
   GradsArgs a;
   std::memset(&a, 0, sizeof(a));
   const float step = static_cast<float>(net->step + 1);
+  a.ld = static_cast<size_t>(net->max_batch / 32);
+  const size_t vec = HID * a.ld;
   for (int l = 0; l < 3; ++l) {
     a.w[l] = net->w[l].p;
     a.m[l] = net->m[l].p;
@@ -1191,13 +1246,12 @@ int run_grads(emt6_mlp *net, int B, bool apply, float lr) {
     a.wb[l] = net->wb[l].p;
     a.wbt[l] = net->wbt[l].p;
     a.grad[l] = apply ? nullptr : net->gradw[l].p;
-    a.vec[l] = {net->b[l].p, net->bm[l].p, net->bv[l].p, net->dZT[l].p, apply ? nullptr : net->gradv[l].p, HID};
+    a.vec[l] = {net->b[l].p, net->bm[l].p, net->bv[l].p, net->part.p + l * vec, apply ? nullptr : net->gradv[l].p, HID};
   }
-  a.vec[3] = {net->w4.p, net->m4.p, net->v4.p, net->AT[2].p, apply ? nullptr : net->gradv[3].p, HID};
+  a.vec[3] = {net->w4.p, net->m4.p, net->v4.p, net->part.p + 3 * vec, apply ? nullptr : net->gradv[3].p, HID};
   a.vec[4] = {net->b4.p, net->mb4.p, net->vb4.p, nullptr, apply ? nullptr : net->gradv[4].p, 1};
   a.dy = net->dy.p;
   a.clear = net->loss.p + (net->slot ^ 1);
-  a.ld = static_cast<size_t>(net->max_batch);
   a.B = B;
   a.splits = weight_splits(net, B);
   a.lr = lr;
@@ -1211,7 +1265,8 @@ int run_grads(emt6_mlp *net, int B, bool apply, float lr) {
   // and clusters of 4, 36 of which are resident at once
   const int cluster = a.splits < 4 ? a.splits : 4;
   e = launch_clusters(mlp_grads_kernel, GRAD_TILES * cluster, cluster, GRADS_SMEM, net->stream,
-                      net->mdZT[0], net->mdZT[1], net->mdZT[2], net->mXT, net->mAT[0], net->mAT[1], a,
+                      net->mRows.dz[0], net->mRows.dz[1], net->mRows.dz[2], net->mX, net->mRows.a[0],
+                      net->mRows.a[1], a,
                       cluster);
   if (e != cudaSuccess) return cuda_fail(e, "surrogate gradients");
   if (apply) ++net->step;
@@ -1288,9 +1343,10 @@ int emt6_mlp_create(int max_batch, uint64_t seed, int device, emt6_mlp **out) {
   const size_t BH = static_cast<size_t>(max_batch) * H;
   ok = ok && net->w4.alloc(H) && net->m4.alloc(H) && net->v4.alloc(H) && net->b4.alloc(1) &&
        net->mb4.alloc(1) && net->vb4.alloc(1) &&
-       net->XT.alloc(static_cast<size_t>(max_batch) * INP) && net->dy.alloc(max_batch) &&
-       net->loss.alloc(2) && net->err.alloc(1);
-  for (int l = 0; l < 3 && ok; ++l) ok = net->AT[l].alloc(BH) && net->dZT[l].alloc(BH) && net->Z[l].alloc(BH);
+       net->X16.alloc(static_cast<size_t>(max_batch) * INP) && net->dy.alloc(max_batch) &&
+       net->part.alloc(4 * BH / 32) && net->loss.alloc(2) && net->err.alloc(1);
+  for (int l = 0; l < 3 && ok; ++l)
+    ok = (l == 2 || net->A[l].alloc(BH)) && net->dZ[l].alloc(BH) && net->Z[l].alloc(BH / 8);
   for (int i = 0; i < 5 && ok; ++i) ok = net->gradv[i].alloc(i < 4 ? H : 1);
   if (!ok) {
     if (net->stream) cudaStreamDestroy(net->stream);
