@@ -44,9 +44,9 @@ struct KParams {
   uint32_t layouts;
 };
 
-// kLayoutBands: eight-lane bands for narrow regions up to 23 columns;
-// kLayoutWideBands: three-column half-warp bands for 41-48-row wide regions;
-// kLayoutRing: the ring mapping of 35 x 35 regions on the narrow kernel
+// kLayoutBands, kLayoutWideBands: a tile holds just the free block of unclipped
+// regions, up to distance 16 and above it; kLayoutRing: a region or block may
+// fill its tile to the last row and column (tile_mapping)
 constexpr uint32_t kLayoutBands = 1u, kLayoutWideBands = 2u, kLayoutRing = 4u,
                    kLayoutAll = 7u;
 

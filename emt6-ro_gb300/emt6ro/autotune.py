@@ -1,8 +1,8 @@
 """Launch and tile-shape autotuner for the batch engine.
 
-A CTA holds one simulation's lattice in shared memory (52 KB: an SM holds
-four whatever the grouping, so one simulation per CTA is fixed), and the
-kernels pick a register tiling per region.  Tuned per workload, in two
+A CTA holds one simulation (an SM holds five with small regions, else four,
+whatever the grouping, so one simulation per CTA is fixed),
+and the kernels pick a register tile per region.  Tuned per workload, in two
 stages on a stratified sample of the batch from identical initial states:
 
 1. how the step loop is launched: steps per launch (longer launches amortise
@@ -11,8 +11,8 @@ stages on a stratified sample of the batch from identical initial states:
    schedule (one CTA per simulation vs persistent CTAs over a device work
    queue ordered by horizon) and CUDA-graph replay of the launch sequence;
 2. with the fastest launch, which tile shapes the kernels may use
-   (Batch.LAYOUT_* bits: eight-lane bands for small regions, three-column
-   bands for 41-48-row wide regions, the 35 x 35 ring mapping).
+   (Batch.LAYOUT_* bits: tiles of just the free block of unclipped regions,
+   small and large ones, and tiles filled to their last row and column).
 
 Every candidate gives bit-identical results; only time differs.
 """

@@ -1,0 +1,97 @@
+"""The simulation kernel's register tiles and launch tiers where they end:
+regions that just fill or just miss a tile, batches larger than one wave whose
+simulations run on both tiers side by side, lists longer than the on-chip
+clocks, and cells in every class of the cell loop.  Exact throughout: the
+tiles, tiers, schedules and layouts only change where a site is computed, so
+nothing is to differ by a bit."""
+import numpy as np
+import pytest
+
+from test_gpu_units import _diffusion_parity
+
+pytestmark = pytest.mark.gpu
+
+# the tiles' columns and rows per lane; a tile holds 4R x 8C sites
+_TILES = [(1, 2), (2, 3), (2, 4), (3, 5), (3, 6), (4, 7), (4, 8), (5, 9), (5, 10), (6, 11),
+          (6, 12), (7, 13), (7, 14), (8, 14)]
+
+
+@pytest.mark.parametrize("tile", range(len(_TILES)))
+def test_regions_that_fill_a_tile(tile, params, oracle):
+    """One diffusion step on lattices that are one region: as large as the
+    tile, one row or column less, one more (the next tile), and flat ones."""
+    C, R = _TILES[tile]
+    rng = np.random.default_rng(4100 + tile)
+    for h, w in [(4 * R, 8 * C), (4 * R - 1, 8 * C), (4 * R, 8 * C - 1), (4 * R + 1, 8 * C),
+                 (4 * R, 8 * C + 1), (4 * R, 3), (3, 8 * C)]:
+        h, w = min(h, 56), min(w, 62)
+        st = np.full((h, w), 2, np.uint8)
+        st[1:-1, 1:-1] = rng.random((h - 2, w - 2)) < 0.9
+        st[1:-1:max(h - 3, 1), 1:-1:max(w - 3, 1)] = 1  # the corners
+        _diffusion_parity(st, rng, params, oracle)
+
+
+def _tumour(params, r, seed):
+    """A disc whose cells are in every phase and class: clocks before, at and
+    past the end of their phase or cycle, under repair, first phases longer
+    than the cycle."""
+    from emt6ro import workloads as wl
+    t = wl.disc_tumor(params, r, seed=seed)
+    s = t.sites
+    rng = np.random.default_rng(seed)
+    live = s["state"] == 1
+    n = int(live.sum())
+    ct = s["cycle_times"][live]
+    ct[rng.random(n) < 0.05, 0] = 40.0
+    s["cycle_times"][live] = ct
+    phase = rng.integers(0, 5, n)
+    s["phase"][live] = phase
+    s["mode"][live] = rng.integers(0, 4, n)
+    end = ct[np.arange(n), phase]
+    s["proliferation_time"][live] = np.where(rng.random(n) < 0.1, end, end * rng.random(n))
+    hurt = live & (rng.random(s.shape) < 0.2)
+    k = int(hurt.sum())
+    s["irradiation"][hurt] = rng.integers(1, 17, k).astype(np.float32) * np.float32(0.25)
+    s["repair_delay_time"][hurt] = 4.0
+    s["time_in_repair"][hurt] = 4.0 * rng.random(k)
+    return t
+
+
+@pytest.mark.parametrize("schedule,layouts", [(0, 7), (1, 7), (2, 7), (3, 0)])
+def test_tiers_side_by_side(schedule, layouts, params, oracle):
+    """1,400 simulations (more than one wave) of radii 1 to 24 on both tiers:
+    the first ones equal the oracle, others equal batches that are one wave,
+    whose runs are once short (tiers in turn), once long (side by side)."""
+    from emt6ro.batch import Batch
+    n, chunks, seed = 1400, [70, 20, 60], 71
+    tumors = [_tumour(params, r, 700 + r) for r in (1, 5, 9, 14, 15, 16, 17, 19, 21, 24)]
+    protocols = [[(0, 1.5)], [(0, 0.75)], []]
+    i = np.arange(n)
+    st, sp = (i % 10).astype(np.int32), (i % 3).astype(np.int32)
+    hz = np.where(i % 7 == 3, i % 97, 1000).astype(np.uint32)
+    b = Batch(params, tumors, protocols, st, sp, sim_horizon=hz, seed=seed)
+    b.set_schedule(schedule, 0)
+    b.set_layouts(layouts)
+    for c in chunks:
+        b.run(c)
+    counts = b.counts()
+
+    k = 20
+    ob = oracle.Batch(oracle.params_copy(params.native), k, seed)
+    for j in range(k):
+        ob.set(j, tumors[st[j]].sites, b.doses[sp[j]], resolution=300, length=144_000,
+               horizon=int(hz[j]))
+    ob.run(sum(chunks), nthreads=8)
+    assert (counts[:k] == ob.counts()).all()
+    for j in range(k):
+        assert b.state(j).sites.tobytes() == ob.get(j).tobytes(), j
+
+    for base, parts in ((600, chunks), (1300, [50, 50, 50])):
+        m = slice(base, base + 100)
+        small = Batch(params, tumors, protocols, st[m], sp[m], sim_horizon=hz[m], seed=seed)
+        small.set_index_base(base)
+        for c in parts:
+            small.run(c)
+        assert (small.counts() == counts[m]).all()
+        for j in range(0, 100, 9):
+            assert small.state(j).sites.tobytes() == b.state(base + j).sites.tobytes(), j
