@@ -273,10 +273,13 @@ struct DevBuf {
 
 }  // namespace
 
-// Launches of fewer steps run a resident batch's tiers one after the other: the
-// tier guess, the second stream and the launch after it cost about 8 us, a step 5
-// to 30; of more, side by side (100 discs of radius 16, 300 steps: 3.6 vs 5.9 ms).
-constexpr uint32_t kSplitSteps = 64;
+// Launches of fewer steps run a resident batch on the wide tier alone, which takes
+// any simulation: one launch instead of the tier guess and three launches.  The
+// narrow tier is 2 to 4 % faster where it fits.  600 discs of radius 6, both tiers
+// in turn and wide alone: 1 step 28 and 22 us, 20 steps 119 and 121, 40 steps 217
+// and 226; of radius 18: 67 and 58, 472 and 463.  Side by side costs what both in
+// turn do, and less where some simulations outgrow the narrow tier.
+constexpr uint32_t kSplitSteps = 24;
 
 struct emt6_batch {
   std::mutex mu;
@@ -443,10 +446,8 @@ struct emt6_batch {
       if (has_horizon && t >= max_horizon) break;
       if (resident && end - t < kSplitSteps) {
         a.order = nullptr;
-        for (int tier : {emt6::kTierNarrow, emt6::kTierWide}) {
-          const int rc = launch(a, end, tier, stream, count);
-          if (rc) return rc;
-        }
+        const int rc = launch(a, end, emt6::kTierWide, stream, count);
+        if (rc) return rc;
       } else {
         // The tiers side by side, the larger simulations' first, each on the
         // simulations expected to fit it: one after the other would leave most
