@@ -608,6 +608,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll 1
   for (int phase = 0; phase < PHASES; ++phase) {
     const int nk = phase == 0 ? INP / BK : HID / BK;
+    // what the epilogue reads from memory, ahead of the product: a lane's share of
+    // the warp's 32 biases, or the thread's pre-activations
+    const float bias = phase < 3 ? __ldg(a.b[phase < 3 ? phase : 0] + col0 + lane) : 0.0f;
+    uint4 zq[4];
+    if (TRAIN && phase >= 3)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) zq[j] = z_at(phase == 3 ? 1 : 0, j);
     // ---- product: accumulator = operand x this CTA's 128 weight rows
     if (tid == 0) {
       load_tiles(phase, phase == 0 ? 2 : RING, nk);
@@ -642,18 +649,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (!last) cluster_meet();  // every CTA's products have read the operand and its copies
     // ---- epilogue
     if (phase < 3) {
-      const float *bias = a.b[phase] + col0;
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
         float v[8];
         tmem_ld8(acc0 + 8 * j, v);
         alignas(16) __nv_bfloat16 zb[8], h[8];
-        const float4 b0 = __ldg(reinterpret_cast<const float4 *>(bias + 8 * j)),
-                     b1 = __ldg(reinterpret_cast<const float4 *>(bias + 8 * j + 4));
-        const float bj[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float z = v[i] + bj[i];
+          const float z = v[i] + __shfl_sync(0xffffffffu, bias, 8 * j + i);
           zb[i] = __float2bfloat16_rn(z);
           h[i] = __float2bfloat16_rn(gelu(z));
         }
@@ -665,8 +668,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       const int l = phase == 3 ? 1 : 0;  // layer whose pre-activations the error passes
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
-        const uint4 zq = z_at(l, j);
-        const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zq);
+        const uint4 zj = j == 0 ? zq[0] : j == 1 ? zq[1] : j == 2 ? zq[2] : zq[3];
+        const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zj);
         float v[8];
         tmem_ld8(acc0 + 8 * j, v);
         alignas(16) __nv_bfloat16 h[8];
@@ -690,6 +693,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     exchange(own, BN / BK * TILE_BYTES, 1, 0);
     if (TRAIN && phase != 2 && tid == 0) store_rows(phase < 2 ? &out.a[phase] : &out.dz[1], act + own);
     if (phase == 2) {
+      const float w4l = TRAIN ? __ldg(a.w4 + col0 + lane) : 0.0f;
+      float wh[HID / 256][8];  // the head's weights
+#pragma unroll
+      for (int j = 0; j < HID / 256; ++j)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) wh[j][q] = __ldg(a.w4 + 8 * (lane + 32 * j) + q);
+      if (TRAIN)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) zq[j] = z_at(2, j);
       if (!arrived()) failed = true;
       // ---- head: y = A3 w4 + b4, one warp per row
 #pragma unroll 1
@@ -697,11 +709,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const int r = static_cast<int>(rank) * (BM / CLUSTER) + warp * (BM / CLUSTER / 16) + k;
         float acc = 0.0f;
 #pragma unroll
-        for (int j = lane; j < HID / 8; j += 32) {
-          const uint4 u = *reinterpret_cast<const uint4 *>(smem + act_chunk(r, j));
+        for (int j = 0; j < HID / 256; ++j) {
+          const uint4 u = *reinterpret_cast<const uint4 *>(smem + act_chunk(r, lane + 32 * j));
           const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&u);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) acc += __bfloat162float(e[q]) * a.w4[8 * j + q];
+          for (int q = 0; q < 8; ++q) acc += __bfloat162float(e[q]) * wh[j][q];
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -728,12 +740,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const float d = s_dy[row];
 #pragma unroll 1
         for (int j = 0; j < 4; ++j) {
-          const uint4 zq = z_at(2, j);
-          const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zq);
+          const uint4 zj = j == 0 ? zq[0] : j == 1 ? zq[1] : j == 2 ? zq[2] : zq[3];
+          const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zj);
           alignas(16) __nv_bfloat16 h[8];
-          const float4 w0 = __ldg(reinterpret_cast<const float4 *>(a.w4 + col0 + 8 * j)),
-                       w1 = __ldg(reinterpret_cast<const float4 *>(a.w4 + col0 + 8 * j + 4));
-          const float wj[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+          float wj[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) wj[i] = __shfl_sync(0xffffffffu, w4l, 8 * j + i);
           const uint4 aq = *reinterpret_cast<const uint4 *>(smem + act_chunk(row, col0 / 8 + j));
           const __nv_bfloat16 *ab = reinterpret_cast<const __nv_bfloat16 *>(&aq);
           float gw[8];
