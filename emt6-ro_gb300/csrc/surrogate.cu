@@ -437,9 +437,11 @@ __device__ __forceinline__ uint32_t act_chunk(int row, int chunk) {
   return static_cast<uint32_t>((chunk >> 3) * TILE_BYTES + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
 }
 
-// What bounds it, in cycles of a CTA per layer (4,096 rows): the weight tiles from
-// L2 and the products 5,800, the exchange 4,000, the epilogue 5,900: a latency
-// chain, as long at 640 rows.  Training's operands of the weight gradients leave
+// What bounds it: a latency chain of product, epilogue and exchange per layer, as
+// long at 640 rows as at 4,096.  What an epilogue reads from memory is loaded ahead
+// of the product (scoring 200,000 rows 2.24 -> 2.08 ms), and a CTA's first block of
+// the next operand leaves while the second is computed (1.95 ms).
+// Training's operands of the weight gradients leave
 // by bulk copies of the operand blocks that the exchange needs anyway, as rows;
 // transposed from registers they took 4,600 a layer.  The
 // phases and the columns of an epilogue are loops, not unrolled: code that each
@@ -563,13 +565,30 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   // 32 rows of the 2 blocks
   exchange(rank * (BM / CLUSTER) * 128, BM / CLUSTER * 128, INP / BK, TILE_BYTES);
   const int quarter = warp & 3, group = warp >> 2;
-  const int row = quarter * 32 + lane, col0 = n0 + group * 32;  // this thread's row, columns col0..+31
-  const uint32_t acc0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + group * 32;
-  // 8 BF16 values of this thread (columns col0 + 8 j ..) into the next operand
+  // this thread's row, and its 4 x 8 columns: two of each of the CTA's blocks, the
+  // first block's first, so that it leaves while the second is computed
+  const int row = quarter * 32 + lane;
+  const auto col = [&](int j) { return (j >> 1) * BK + group * 16 + (j & 1) * 8; };
+  const int lane_col = n0 + col(lane >> 3) + (lane & 7);  // of the warp's 32, the lane's
+  const uint32_t acc0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+  // 8 BF16 values of this thread (columns n0 + col(j) ..) into the next operand
   const auto publish = [&](int j, const uint4 &v) {
-    *reinterpret_cast<uint4 *>(smem + act_chunk(row, col0 / 8 + j)) = v;
+    *reinterpret_cast<uint4 *>(smem + act_chunk(row, (n0 + col(j)) / 8)) = v;
   };
   const uint32_t own = rank * (BN / BK) * TILE_BYTES;  // this CTA's two blocks of it
+  const auto push = [&](int half) {  // one of them to the peers
+    fence_async();
+    __syncthreads();
+    if (tid == 0) {
+      if (half == 0) mbar_expect_tx(in, (CLUSTER - 1) * BN / BK * TILE_BYTES);
+      const uint32_t at = act + own + half * TILE_BYTES;
+      for (uint32_t p = 1; p < CLUSTER; ++p) {
+        const uint32_t to = (rank + p) % CLUSTER;
+        peer_copy(peer_addr(at, to), at, TILE_BYTES, peer_addr(in, to));
+      }
+    }
+    exchanges += half;
+  };
   // these two blocks at shared address `from` to rows of global memory
   const auto store_rows = [&](const CUtensorMap *map, uint32_t from) {  // thread 0
 #pragma unroll
@@ -593,7 +612,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
     v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
     if (!(lane & 3))
-      a.part[static_cast<size_t>(k * HID + col0 + 8 * j + (lane >> 4 & 1) * 4 + (lane >> 3 & 1) * 2 +
+      a.part[static_cast<size_t>(k * HID + n0 + col(j) + (lane >> 4 & 1) * 4 + (lane >> 3 & 1) * 2 +
                                  (lane >> 2 & 1)) * a.ld + m0 / 32 + quarter] = v[0];
   };
   const auto sum_dz = [&](int l, int j, const uint4 &v) {
@@ -610,7 +629,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int nk = phase == 0 ? INP / BK : HID / BK;
     // what the epilogue reads from memory, ahead of the product: a lane's share of
     // the warp's 32 biases, or the thread's pre-activations
-    const float bias = phase < 3 ? __ldg(a.b[phase < 3 ? phase : 0] + col0 + lane) : 0.0f;
+    const float bias = phase < 3 ? __ldg(a.b[phase < 3 ? phase : 0] + lane_col) : 0.0f;
     uint4 zq[4];
     if (TRAIN && phase >= 3)
 #pragma unroll
@@ -652,7 +671,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
         float v[8];
-        tmem_ld8(acc0 + 8 * j, v);
+        tmem_ld8(acc0 + col(j), v);
         alignas(16) __nv_bfloat16 zb[8], h[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -663,6 +682,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
         publish(j, hv);
         if (TRAIN) z_at(phase, j) = *reinterpret_cast<const uint4 *>(zb);
+        if (j == 1) push(0);
       }
     } else {
       const int l = phase == 3 ? 1 : 0;  // layer whose pre-activations the error passes
@@ -671,7 +691,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const uint4 zj = j == 0 ? zq[0] : j == 1 ? zq[1] : j == 2 ? zq[2] : zq[3];
         const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zj);
         float v[8];
-        tmem_ld8(acc0 + 8 * j, v);
+        tmem_ld8(acc0 + col(j), v);
         alignas(16) __nv_bfloat16 h[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) h[i] = __float2bfloat16_rn(v[i] * gelu_grad(__bfloat162float(zb[i])));
@@ -679,8 +699,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         if (!last)
           publish(j, hv);
         else  // the ring is free; a peer's copy of this CTA's operand blocks may not be done
-          *reinterpret_cast<uint4 *>(smem + ACT_BYTES + act_chunk(row, group * 4 + j)) = hv;
+          *reinterpret_cast<uint4 *>(smem + ACT_BYTES + act_chunk(row, col(j) / 8)) = hv;
         sum_dz(l, j, hv);
+        if (!last && j == 1) push(0);
       }
     }
     if (last) {
@@ -690,10 +711,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       break;
     }
     tc_fence_before();
-    exchange(own, BN / BK * TILE_BYTES, 1, 0);
+    push(1);
     if (TRAIN && phase != 2 && tid == 0) store_rows(phase < 2 ? &out.a[phase] : &out.dz[1], act + own);
     if (phase == 2) {
-      const float w4l = TRAIN ? __ldg(a.w4 + col0 + lane) : 0.0f;
+      const float w4l = TRAIN ? __ldg(a.w4 + lane_col) : 0.0f;
       float wh[HID / 256][8];  // the head's weights
 #pragma unroll
       for (int j = 0; j < HID / 256; ++j)
@@ -746,7 +767,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
           float wj[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) wj[i] = __shfl_sync(0xffffffffu, w4l, 8 * j + i);
-          const uint4 aq = *reinterpret_cast<const uint4 *>(smem + act_chunk(row, col0 / 8 + j));
+          const uint4 aq = *reinterpret_cast<const uint4 *>(smem + act_chunk(row, (n0 + col(j)) / 8));
           const __nv_bfloat16 *ab = reinterpret_cast<const __nv_bfloat16 *>(&aq);
           float gw[8];
 #pragma unroll
@@ -758,8 +779,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
           const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
           publish(j, hv);
           sum_dz(2, j, hv);
+          if (j == 1) push(0);
         }
-        exchange(own, BN / BK * TILE_BYTES, 1, 0);
+        push(1);
         if (tid == 0) store_rows(&out.dz[2], act + own);
       }
     }
