@@ -25,6 +25,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -467,7 +469,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                  in = smem_u32(bars + 2 * RING + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_rank();
-  const int m0 = static_cast<int>(blockIdx.x / CLUSTER) * BM, n0 = static_cast<int>(rank) * BN;
+  const int n0 = static_cast<int>(rank) * BN;
+  int m0 = static_cast<int>(blockIdx.x / CLUSTER) * BM;  // the cluster's rows, in turn
+  const int stride = static_cast<int>(gridDim.x / CLUSTER) * BM;
   constexpr int PHASES = TRAIN ? 5 : 3;
 
   if (tid == 0) {
@@ -535,35 +539,23 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   const auto arrived = [&]() -> bool { return mbar_wait(in, (exchanges - 1) & 1, nullptr); };
   cluster_meet();  // every CTA runs, its barriers initialised
 
-  // ---- inputs: FP32 rows -> BF16 operand (zero columns 100..127, zero rows
-  // beyond n).  Each CTA packs a quarter of the rows: one 16-byte chunk per thread.
-  {
-    static_assert(BM / CLUSTER * (INP / 8) == GEMM_THREADS, "one chunk per thread");
-    const int r = static_cast<int>(rank) * (BM / CLUSTER) + tid / (INP / 8), chunk = tid % (INP / 8);
-    float f[8];
+  // inputs: each CTA takes a quarter of the rows, a thread one 16-byte chunk of
+  // BF16 (zero columns 100..127, zero rows beyond n)
+  static_assert(BM / CLUSTER * (INP / 8) == GEMM_THREADS, "one chunk per thread");
+  const int xr = static_cast<int>(rank) * (BM / CLUSTER) + tid / (INP / 8), xc = tid % (INP / 8);
+  float f[8];
+  const auto load_x = [&](int from) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) f[q] = 0.0f;
-    if (m0 + r < a.n) {
-      const float *src = a.x + static_cast<size_t>(m0 + r) * IN + chunk * 8;
+    if (from + xr < a.n) {
+      const float *src = a.x + static_cast<size_t>(from + xr) * IN + xc * 8;
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        if (chunk * 8 + q < IN) f[q] = src[q];
-      if (!TRAIN && a.norm) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (chunk * 8 + q < IN) f[q] = (f[q] - s_norm[chunk * 8 + q]) / s_norm[IN + chunk * 8 + q];
-      }
+        if (xc * 8 + q < IN) f[q] = src[q];
     }
-    alignas(16) __nv_bfloat16 v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = __float2bfloat16_rn(f[q]);
-    *reinterpret_cast<uint4 *>(smem + act_chunk(r, chunk)) = *reinterpret_cast<const uint4 *>(v);
-    if (TRAIN)
-      *reinterpret_cast<uint4 *>(a.x16 + static_cast<size_t>(m0 + r) * INP + 8 * chunk) =
-          *reinterpret_cast<const uint4 *>(v);
-  }
-  // 32 rows of the 2 blocks
-  exchange(rank * (BM / CLUSTER) * 128, BM / CLUSTER * 128, INP / BK, TILE_BYTES);
+  };
+  load_x(m0);
+
   const int quarter = warp & 3, group = warp >> 2;
   // this thread's row, and its 4 x 8 columns: two of each of the CTA's blocks, the
   // first block's first, so that it leaves while the second is computed
@@ -623,168 +615,196 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     sum_rows(l, j, f);
   };
 
-  int used = 0;  // weight tiles consumed by earlier phases
-#pragma unroll 1
-  for (int phase = 0; phase < PHASES; ++phase) {
-    const int nk = phase == 0 ? INP / BK : HID / BK;
-    // what the epilogue reads from memory, ahead of the product: a lane's share of
-    // the warp's 32 biases, or the thread's pre-activations
-    const float bias = phase < 3 ? __ldg(a.b[phase < 3 ? phase : 0] + lane_col) : 0.0f;
-    uint4 zq[4];
-    if (TRAIN && phase >= 3)
+  int used = 0, products = 0;  // weight tiles consumed, products run
+  for (;;) {
+    // ---- inputs into the operand
+    if (!TRAIN && a.norm && m0 + xr < a.n)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) zq[j] = z_at(phase == 3 ? 1 : 0, j);
-    // ---- product: accumulator = operand x this CTA's 128 weight rows
-    if (tid == 0) {
-      load_tiles(phase, phase == 0 ? 2 : RING, nk);
-    } else if (tid == 32) {
-      if (!arrived()) *abort = 1;
-      tc_fence_after();
-      for (int kb = 0; kb < nk && !*abort; ++kb) {
-        const int s = (used + kb) % RING;
-        if (!mbar_wait(full0 + 8 * s, ((used + kb) / RING) & 1, abort)) {
-          *abort = 1;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t pa = act + kb * TILE_BYTES, pb = ring + s * TILE_BYTES;
+      for (int q = 0; q < 8; ++q)
+        if (xc * 8 + q < IN) f[q] = (f[q] - s_norm[xc * 8 + q]) / s_norm[IN + xc * 8 + q];
+    {
+      alignas(16) __nv_bfloat16 v[8];
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k)
-          umma_bf16(tmem, sw128_desc(pa + 32 * k), sw128_desc(pb + 32 * k), kIdesc,
-                    (kb | k) != 0 ? 1u : 0u);
-        umma_commit(empty0 + 8 * s);
-      }
-      umma_commit(done);  // arrives once every product above has completed
-    }
-    __syncwarp();
-    if (!mbar_wait(done, phase & 1, nullptr)) failed = true;
-    tc_fence_after();
-    used += nk;
-    // the ring is free: the next phase's first tiles load during the epilogue
-    if (tid == 0 && phase + 1 < PHASES) load_tiles(phase + 1, 0, RING);
-    __syncwarp();
-    const bool last = TRAIN && phase == PHASES - 1;  // the lowest layer's error goes no further
-    if (TRAIN && tid == 0) store_read();  // the operand's own blocks are overwritten next
-    if (!last) cluster_meet();  // every CTA's products have read the operand and its copies
-    // ---- epilogue
-    if (phase < 3) {
-#pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
-        float v[8];
-        tmem_ld8(acc0 + col(j), v);
-        alignas(16) __nv_bfloat16 zb[8], h[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float z = v[i] + __shfl_sync(0xffffffffu, bias, 8 * j + i);
-          zb[i] = __float2bfloat16_rn(z);
-          h[i] = __float2bfloat16_rn(gelu(z));
-        }
-        const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
-        publish(j, hv);
-        if (TRAIN) z_at(phase, j) = *reinterpret_cast<const uint4 *>(zb);
-        if (j == 1) push(0);
-      }
-    } else {
-      const int l = phase == 3 ? 1 : 0;  // layer whose pre-activations the error passes
-#pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
-        const uint4 zj = j == 0 ? zq[0] : j == 1 ? zq[1] : j == 2 ? zq[2] : zq[3];
-        const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zj);
-        float v[8];
-        tmem_ld8(acc0 + col(j), v);
-        alignas(16) __nv_bfloat16 h[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) h[i] = __float2bfloat16_rn(v[i] * gelu_grad(__bfloat162float(zb[i])));
-        const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
-        if (!last)
-          publish(j, hv);
-        else  // the ring is free; a peer's copy of this CTA's operand blocks may not be done
-          *reinterpret_cast<uint4 *>(smem + ACT_BYTES + act_chunk(row, col(j) / 8)) = hv;
-        sum_dz(l, j, hv);
-        if (!last && j == 1) push(0);
-      }
-    }
-    if (last) {
-      fence_async();
-      __syncthreads();
-      if (tid == 0) store_rows(&out.dz[0], ring);
-      break;
-    }
-    tc_fence_before();
-    push(1);
-    if (TRAIN && phase != 2 && tid == 0) store_rows(phase < 2 ? &out.a[phase] : &out.dz[1], act + own);
-    if (phase == 2) {
-      const float w4l = TRAIN ? __ldg(a.w4 + lane_col) : 0.0f;
-      float wh[HID / 256][8];  // the head's weights
-#pragma unroll
-      for (int j = 0; j < HID / 256; ++j)
-#pragma unroll
-        for (int q = 0; q < 8; ++q) wh[j][q] = __ldg(a.w4 + 8 * (lane + 32 * j) + q);
+      for (int q = 0; q < 8; ++q) v[q] = __float2bfloat16_rn(f[q]);
+      *reinterpret_cast<uint4 *>(smem + act_chunk(xr, xc)) = *reinterpret_cast<const uint4 *>(v);
       if (TRAIN)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) zq[j] = z_at(2, j);
-      if (!arrived()) failed = true;
-      // ---- head: y = A3 w4 + b4, one warp per row
+        *reinterpret_cast<uint4 *>(a.x16 + static_cast<size_t>(m0 + xr) * INP + 8 * xc) =
+            *reinterpret_cast<const uint4 *>(v);
+    }
+    // 32 rows of the 2 blocks
+    exchange(rank * (BM / CLUSTER) * 128, BM / CLUSTER * 128, INP / BK, TILE_BYTES);
+    const bool more = !TRAIN && m0 + stride < a.n;
 #pragma unroll 1
-      for (int k = 0; k < BM / CLUSTER / 16; ++k) {
-        const int r = static_cast<int>(rank) * (BM / CLUSTER) + warp * (BM / CLUSTER / 16) + k;
-        float acc = 0.0f;
+    for (int phase = 0; phase < PHASES; ++phase) {
+      const int nk = phase == 0 ? INP / BK : HID / BK;
+      // what the epilogue reads from memory, ahead of the product: a lane's share of
+      // the warp's 32 biases, or the thread's pre-activations
+      const float bias = phase < 3 ? __ldg(a.b[phase < 3 ? phase : 0] + lane_col) : 0.0f;
+      uint4 zq[4];
+      if (TRAIN && phase >= 3)
 #pragma unroll
-        for (int j = 0; j < HID / 256; ++j) {
-          const uint4 u = *reinterpret_cast<const uint4 *>(smem + act_chunk(r, lane + 32 * j));
-          const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&u);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) acc += __bfloat162float(e[q]) * wh[j][q];
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        const float yr = acc + a.b4[0];
-        if (!TRAIN) {
-          if (lane == 0 && m0 + r < a.n) a.y[m0 + r] = yr;
-        } else {
-          const float e = yr - a.target[m0 + r], d = 2.0f * e / static_cast<float>(a.n);
-          if (lane == 0) {
-            a.dy[m0 + r] = d;
-            s_loss[warp] = (k ? s_loss[warp] : 0.0f) + e * e;
+        for (int j = 0; j < 4; ++j) zq[j] = z_at(phase == 3 ? 1 : 0, j);
+      if (phase == 2 && more) load_x(m0 + stride);
+      // ---- product: accumulator = operand x this CTA's 128 weight rows
+      if (tid == 0) {
+        load_tiles(phase, phase == 0 ? 2 : RING, nk);
+      } else if (tid == 32) {
+        if (*abort || !arrived()) *abort = 1;
+        tc_fence_after();
+        for (int kb = 0; kb < nk && !*abort; ++kb) {
+          const int s = (used + kb) % RING;
+          if (!mbar_wait(full0 + 8 * s, ((used + kb) / RING) & 1, abort)) {
+            *abort = 1;
+            break;
           }
-          if (lane < CLUSTER) peer_store4(peer_addr(smem_u32(s_dy + r), lane), d);
-        }
-      }
-      if (TRAIN) {
-        cluster_sync();  // dy is everywhere, and the operand may be overwritten
-        if (tid == 0) {
-          float t = 0.0f;
+          tc_fence_after();
+          const uint32_t pa = act + kb * TILE_BYTES, pb = ring + s * TILE_BYTES;
 #pragma unroll
-          for (int k = 0; k < 16; ++k) t += s_loss[k];
-          atomicAdd(a.loss, t);
+          for (int k = 0; k < BK / 16; ++k)
+            umma_bf16(tmem, sw128_desc(pa + 32 * k), sw128_desc(pb + 32 * k), kIdesc,
+                      (kb | k) != 0 ? 1u : 0u);
+          umma_commit(empty0 + 8 * s);
         }
-        const float d = s_dy[row];
+        umma_commit(done);  // arrives once every product above has completed
+      }
+      __syncwarp();
+      // (after a wait ran out: no further ones)
+      if (!failed && !mbar_wait(done, products & 1, nullptr)) failed = true;
+      ++products;
+      tc_fence_after();
+      used += nk;
+      // the ring is free: the next phase's first tiles load during the epilogue
+      if (tid == 0) {
+        if (phase + 1 < PHASES) load_tiles(phase + 1, 0, RING);
+        else if (more) load_tiles(0, 0, INP / BK);
+      }
+      __syncwarp();
+      const bool last = TRAIN && phase == PHASES - 1;  // the lowest layer's error goes no further
+      if (TRAIN && tid == 0) store_read();  // the operand's own blocks are overwritten next
+      if (!last) cluster_meet();  // every CTA's products have read the operand and its copies
+      // ---- epilogue
+      if (phase < 3) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          float v[8];
+          tmem_ld8(acc0 + col(j), v);
+          alignas(16) __nv_bfloat16 zb[8], h[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float z = v[i] + __shfl_sync(0xffffffffu, bias, 8 * j + i);
+            zb[i] = __float2bfloat16_rn(z);
+            h[i] = __float2bfloat16_rn(gelu(z));
+          }
+          const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
+          publish(j, hv);
+          if (TRAIN) z_at(phase, j) = *reinterpret_cast<const uint4 *>(zb);
+          if (j == 1) push(0);
+        }
+      } else {
+        const int l = phase == 3 ? 1 : 0;  // layer whose pre-activations the error passes
 #pragma unroll 1
         for (int j = 0; j < 4; ++j) {
           const uint4 zj = j == 0 ? zq[0] : j == 1 ? zq[1] : j == 2 ? zq[2] : zq[3];
           const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zj);
+          float v[8];
+          tmem_ld8(acc0 + col(j), v);
           alignas(16) __nv_bfloat16 h[8];
-          float wj[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) wj[i] = __shfl_sync(0xffffffffu, w4l, 8 * j + i);
-          const uint4 aq = *reinterpret_cast<const uint4 *>(smem + act_chunk(row, (n0 + col(j)) / 8));
-          const __nv_bfloat16 *ab = reinterpret_cast<const __nv_bfloat16 *>(&aq);
-          float gw[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) gw[i] = __bfloat162float(ab[i]) * d;
-          sum_rows(3, j, gw);
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            h[i] = __float2bfloat16_rn(d * wj[i] * gelu_grad(__bfloat162float(zb[i])));
+          for (int i = 0; i < 8; ++i) h[i] = __float2bfloat16_rn(v[i] * gelu_grad(__bfloat162float(zb[i])));
           const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
-          publish(j, hv);
-          sum_dz(2, j, hv);
-          if (j == 1) push(0);
+          if (!last)
+            publish(j, hv);
+          else  // the ring is free; a peer's copy of this CTA's operand blocks may not be done
+            *reinterpret_cast<uint4 *>(smem + ACT_BYTES + act_chunk(row, col(j) / 8)) = hv;
+          sum_dz(l, j, hv);
+          if (!last && j == 1) push(0);
         }
-        push(1);
-        if (tid == 0) store_rows(&out.dz[2], act + own);
+      }
+      if (last) {
+        fence_async();
+        __syncthreads();
+        if (tid == 0) store_rows(&out.dz[0], ring);
+        break;
+      }
+      tc_fence_before();
+      push(1);
+      if (TRAIN && phase != 2 && tid == 0) store_rows(phase < 2 ? &out.a[phase] : &out.dz[1], act + own);
+      if (phase == 2) {
+        const float w4l = TRAIN ? __ldg(a.w4 + lane_col) : 0.0f;
+        float wh[HID / 256][8];  // the head's weights
+#pragma unroll
+        for (int j = 0; j < HID / 256; ++j)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) wh[j][q] = __ldg(a.w4 + 8 * (lane + 32 * j) + q);
+        if (TRAIN)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) zq[j] = z_at(2, j);
+        if (!failed && !arrived()) failed = true;
+        // ---- head: y = A3 w4 + b4, one warp per row
+#pragma unroll 1
+        for (int k = 0; k < BM / CLUSTER / 16; ++k) {
+          const int r = static_cast<int>(rank) * (BM / CLUSTER) + warp * (BM / CLUSTER / 16) + k;
+          float acc = 0.0f;
+#pragma unroll
+          for (int j = 0; j < HID / 256; ++j) {
+            const uint4 u = *reinterpret_cast<const uint4 *>(smem + act_chunk(r, lane + 32 * j));
+            const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&u);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc += __bfloat162float(e[q]) * wh[j][q];
+          }
+#pragma unroll
+          for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+          const float yr = acc + a.b4[0];
+          if (!TRAIN) {
+            if (lane == 0 && m0 + r < a.n) a.y[m0 + r] = yr;
+          } else {
+            const float e = yr - a.target[m0 + r], d = 2.0f * e / static_cast<float>(a.n);
+            if (lane == 0) {
+              a.dy[m0 + r] = d;
+              s_loss[warp] = (k ? s_loss[warp] : 0.0f) + e * e;
+            }
+            if (lane < CLUSTER) peer_store4(peer_addr(smem_u32(s_dy + r), lane), d);
+          }
+        }
+        if (TRAIN) {
+          cluster_sync();  // dy is everywhere, and the operand may be overwritten
+          if (tid == 0) {
+            float t = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) t += s_loss[k];
+            atomicAdd(a.loss, t);
+          }
+          const float d = s_dy[row];
+#pragma unroll 1
+          for (int j = 0; j < 4; ++j) {
+            const uint4 zj = j == 0 ? zq[0] : j == 1 ? zq[1] : j == 2 ? zq[2] : zq[3];
+            const __nv_bfloat16 *zb = reinterpret_cast<const __nv_bfloat16 *>(&zj);
+            alignas(16) __nv_bfloat16 h[8];
+            float wj[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) wj[i] = __shfl_sync(0xffffffffu, w4l, 8 * j + i);
+            const uint4 aq = *reinterpret_cast<const uint4 *>(smem + act_chunk(row, (n0 + col(j)) / 8));
+            const __nv_bfloat16 *ab = reinterpret_cast<const __nv_bfloat16 *>(&aq);
+            float gw[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) gw[i] = __bfloat162float(ab[i]) * d;
+            sum_rows(3, j, gw);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              h[i] = __float2bfloat16_rn(d * wj[i] * gelu_grad(__bfloat162float(zb[i])));
+            const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
+            publish(j, hv);
+            sum_dz(2, j, hv);
+            if (j == 1) push(0);
+          }
+          push(1);
+          if (tid == 0) store_rows(&out.dz[2], act + own);
+        }
       }
     }
+    if (!more) break;
+    m0 += stride;
+    cluster_sync();  // the heads have read the operand
   }
   // no CTA leaves while a peer may still read from or write to it
   if (TRAIN && tid == 0) store_wait();
@@ -1134,6 +1154,30 @@ cudaError_t raise_smem(K kernel, int bytes, bool (&done)[64]) {
   return e;
 }
 
+// Clusters of mlp_rows_kernel<false> that are resident at once, asked once per device.
+cudaError_t resident_clusters(int *out) {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  *out = known[dev].load();
+  if (*out) return cudaSuccess;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(CLUSTER);
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = ROWS_SMEM;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = CLUSTER;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  e = cudaOccupancyMaxActiveClusters(out, mlp_rows_kernel<false>, &cfg);
+  if (e == cudaSuccess) known[dev].store(*out = std::max(*out, 1));
+  return e;
+}
+
 template <typename T>
 struct DevArr {
   T *p = nullptr;
@@ -1242,7 +1286,7 @@ int run_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean, cons
     a.w4 = net->w4.p;
     a.b4 = net->b4.p;
     a.err = net->err.p;
-    const int grid = (a.n + BM - 1) / BM * CLUSTER;
+    int grid = (a.n + BM - 1) / BM * CLUSTER;
     if (d_target) {
       a.target = d_target;
       a.dy = net->dy.p;
@@ -1255,6 +1299,10 @@ int run_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean, cons
                           net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], net->mRows, a);
     } else {
       a.y = d_y + at;
+      int resident = 0;
+      e = resident_clusters(&resident);
+      if (e != cudaSuccess) return cuda_fail(e, "surrogate rows");
+      grid = std::min(grid, resident * CLUSTER);
       e = launch_clusters(mlp_rows_kernel<false>, grid, CLUSTER, ROWS_SMEM, net->stream, net->mW[0],
                           net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], net->mRows, a);
     }

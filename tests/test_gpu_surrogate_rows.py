@@ -53,6 +53,18 @@ def test_not_a_number_reaches_its_row_only():
     assert np.array_equal(y[keep], z[keep])
 
 
+@pytest.mark.parametrize("n", [4608, 4609, 5001, 19_999])
+def test_more_rows_than_run_at_once(n):
+    """Clusters that go over several tiles of rows give what short calls do."""
+    net = _net(128)
+    rng = np.random.default_rng(n)
+    x = (rng.normal(size=(n, 100)) * 3).astype(np.float32)
+    net.x_mean = rng.normal(size=100).astype(np.float32)
+    net.x_std = rng.uniform(0.5, 2, 100).astype(np.float32)
+    y = net.predict(x)
+    assert np.array_equal(y, np.concatenate([net.predict(x[i:i + 999]) for i in range(0, n, 999)]))
+
+
 # 128 and 384 rows: one part; 640: two; 1024: four; 2048: eight
 @pytest.mark.parametrize("batch", [128, 384, 640, 1024, 2048])
 def test_gradients_and_step_at_every_split(batch):
