@@ -418,14 +418,12 @@ struct RowsArgs {
   float *dy, *loss;
   uint4 *z[3];         // pre-activations, 8 columns of a row each (z_at)
   __nv_bfloat16 *x16;  // [n][128]
-  float *part;         // sums of 32 rows: [dZ1, dZ2, dZ3, A3 dy][512][ld]
-  size_t ld;
   int *err;
 };
 
 // where training's operands of the weight gradients go, [n][512]
 struct RowsMaps {
-  CUtensorMap a[2], dz[3];
+  CUtensorMap a[3], dz[3];
 };
 
 // shared memory of mlp_rows_kernel: the 8 blocks of the current operand, the
@@ -442,10 +440,11 @@ __device__ __forceinline__ uint32_t act_chunk(int row, int chunk) {
 // What bounds it: a latency chain of product, epilogue and exchange per layer, as
 // long at 640 rows as at 4,096.  What an epilogue reads from memory is loaded ahead
 // of the product (scoring 200,000 rows 2.24 -> 2.08 ms), and a CTA's first block of
-// the next operand leaves while the second is computed (1.95 ms).
-// Training's operands of the weight gradients leave
-// by bulk copies of the operand blocks that the exchange needs anyway, as rows;
-// transposed from registers they took 4,600 a layer.  The
+// the next operand leaves while the second is computed (1.93 ms).  Predicting, a
+// resident cluster goes over tiles of rows, the next one's inputs and first weights
+// on their way during the last layer (1.88 ms).  Training's operands of the weight
+// gradients leave by bulk copies of the operand blocks that the exchange needs
+// anyway, as rows; transposed from registers they took 4,600 cycles a layer.  The
 // phases and the columns of an epilogue are loops, not unrolled: code that each
 // warp runs once is fetched as it goes.  With one launch per layer, and input,
 // head and error launches between, a step's rows took 75 us of GPU time.
@@ -592,28 +591,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   const auto z_at = [&](int l, int j) -> uint4 & {
     return a.z[l][(static_cast<size_t>(blockIdx.x) * 16 + group * 4 + j) * BM + row];
   };
-  // sums of the warp's 32 rows of 8 columns: 4 lanes end up with the same column
-  const auto sum_rows = [&](int k, int j, float (&v)[8]) {
-#pragma unroll
-    for (int n = 4, o = 16; n; n >>= 1, o >>= 1)
-#pragma unroll
-      for (int i = 0; i < n; ++i) {
-        const float keep = lane & o ? v[i + n] : v[i], send = lane & o ? v[i] : v[i + n];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-      }
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    if (!(lane & 3))
-      a.part[static_cast<size_t>(k * HID + n0 + col(j) + (lane >> 4 & 1) * 4 + (lane >> 3 & 1) * 2 +
-                                 (lane >> 2 & 1)) * a.ld + m0 / 32 + quarter] = v[0];
-  };
-  const auto sum_dz = [&](int l, int j, const uint4 &v) {
-    const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&v);
-    float f[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(e[i]);
-    sum_rows(l, j, f);
-  };
 
   int used = 0, products = 0;  // weight tiles consumed, products run
   for (;;) {
@@ -716,7 +693,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             publish(j, hv);
           else  // the ring is free; a peer's copy of this CTA's operand blocks may not be done
             *reinterpret_cast<uint4 *>(smem + ACT_BYTES + act_chunk(row, col(j) / 8)) = hv;
-          sum_dz(l, j, hv);
           if (!last && j == 1) push(0);
         }
       }
@@ -728,7 +704,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       }
       tc_fence_before();
       push(1);
-      if (TRAIN && phase != 2 && tid == 0) store_rows(phase < 2 ? &out.a[phase] : &out.dz[1], act + own);
+      if (TRAIN && tid == 0) {
+        store_rows(phase < 3 ? &out.a[phase] : &out.dz[1], act + own);
+        if (phase == 2) store_read();  // dZ3 replaces A3 below
+      }
       if (phase == 2) {
         const float w4l = TRAIN ? __ldg(a.w4 + lane_col) : 0.0f;
         float wh[HID / 256][8];  // the head's weights
@@ -783,18 +762,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             float wj[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) wj[i] = __shfl_sync(0xffffffffu, w4l, 8 * j + i);
-            const uint4 aq = *reinterpret_cast<const uint4 *>(smem + act_chunk(row, (n0 + col(j)) / 8));
-            const __nv_bfloat16 *ab = reinterpret_cast<const __nv_bfloat16 *>(&aq);
-            float gw[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) gw[i] = __bfloat162float(ab[i]) * d;
-            sum_rows(3, j, gw);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
               h[i] = __float2bfloat16_rn(d * wj[i] * gelu_grad(__bfloat162float(zb[i])));
             const uint4 &hv = *reinterpret_cast<const uint4 *>(h);
             publish(j, hv);
-            sum_dz(2, j, hv);
             if (j == 1) push(0);
           }
           push(1);
@@ -829,9 +801,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 // ---- weight gradients and Adam -------------------------------------------------------
 struct VecAdam {
   float *w, *m, *v;
-  const float *rows;  // [n][ld] partial sums; null: b4
+  const __nv_bfloat16 *rows;  // [n][512]: dZ, or A3 for w4
   float *grad_out;
-  int n;
 };
 
 struct GradsArgs {
@@ -841,73 +812,86 @@ struct GradsArgs {
   VecAdam vec[5];
   const float *dy;
   float *clear;  // the next step's loss sum
-  size_t ld;
   int B, splits;
   float lr, beta1, beta2, eps, bc1, bc2;
   int *err;
 };
 
-// Gradients and Adam updates of elements e, e + stride, .. (VEC_U of them, below
-// VEC_ELEMS) of the vectors b1, b2, b3, w4 (sums over the batch from the rows
-// kernel's sums of 32 rows) and b4 (sum dy).  One warp; the elements' loads
-// overlap, and lane u updates the u-th.
-constexpr int VEC_ELEMS = 4 * HID + 1, VEC_U = 4;
-__device__ __forceinline__ void vec_adam(const GradsArgs &a, int e, int stride, int lane) {
-  const float4 *rows[VEC_U];
-  float g[VEC_U], mine = 0.0f;
-#pragma unroll
-  for (int u = 0; u < VEC_U; ++u) {
-    const int q = e + u * stride, k = q / HID;
-    g[u] = 0.0f;
-    rows[u] = k < 4 && q < VEC_ELEMS
-                  ? reinterpret_cast<const float4 *>(a.vec[k].rows + static_cast<size_t>(q % HID) * a.ld)
-                  : nullptr;
-  }
-  // this lane's element (lanes 0 .. VEC_U - 1)
-  const int q = e + lane * stride, k = q / HID, idx = q % HID;
-  const bool own = lane < VEC_U && q < VEC_ELEMS;
-  const VecAdam &p = a.vec[own ? k : 0];
-  float m0 = 0.0f, v0 = 0.0f, w0 = 0.0f;
-  if (own && !p.grad_out) {
-    m0 = p.m[idx];
-    v0 = p.v[idx];
-    w0 = p.w[idx];
-  }
-  // B is a multiple of 128: 4 sums (16 bytes) per lane per load
-  for (int j = lane; j < a.B / 128; j += 32) {
-    float4 r[VEC_U];
-#pragma unroll
-    for (int u = 0; u < VEC_U; ++u)
-      if (rows[u]) r[u] = rows[u][j];
-#pragma unroll
-    for (int u = 0; u < VEC_U; ++u)
-      if (rows[u]) g[u] += (r[u].x + r[u].y) + (r[u].z + r[u].w);
-  }
-#pragma unroll
-  for (int u = 0; u < VEC_U; ++u) {
-    if (e + u * stride == VEC_ELEMS - 1)
-      for (int j = lane; j < a.B; j += 32) g[u] += a.dy[j];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) g[u] += __shfl_xor_sync(0xffffffffu, g[u], o);
-    if (lane == u) mine = g[u];
-  }
-  if (!own) return;
+__device__ __forceinline__ void vec_update(const GradsArgs &a, const VecAdam &p, int idx, float g) {
   if (p.grad_out) {
-    p.grad_out[idx] = mine;
+    p.grad_out[idx] = g;
     return;
   }
-  const float m = a.beta1 * m0 + (1.0f - a.beta1) * mine;
-  const float s = a.beta2 * v0 + (1.0f - a.beta2) * mine * mine;
+  const float m = a.beta1 * p.m[idx] + (1.0f - a.beta1) * g;
+  const float s = a.beta2 * p.v[idx] + (1.0f - a.beta2) * g * g;
   p.m[idx] = m;
   p.v[idx] = s;
-  p.w[idx] = w0 - a.lr * (m / a.bc1) / (sqrtf(s / a.bc2) + a.eps);
+  p.w[idx] = p.w[idx] - a.lr * (m / a.bc1) / (sqrtf(s / a.bc2) + a.eps);
+}
+
+// Gradients and Adam updates of 16 elements of b1, b2, b3 (sums of dZ over the
+// batch) or w4 (A3^T dy), by 8 warps.  Rows 8 q .. 8 q + 7, and those 256 further
+// and so on, are summed in order by slot q = 8 (lane / 8) + w, a thread two
+// columns of it; then slots 16, 8, 4, 2 and 1 apart.  Latency bound, beside the
+// products: 32 bytes of 8 rows per load round.
+constexpr int VEC_COLS = 16, VEC_TASKS = 4 * HID / VEC_COLS, VEC_WARPS = 8;
+__device__ __forceinline__ void vec_adam(const GradsArgs &a, int task, float *part, int w, int lane) {
+  const int k = task / (HID / VEC_COLS), c0 = task % (HID / VEC_COLS) * VEC_COLS;
+  const uint32_t *src =
+      reinterpret_cast<const uint32_t *>(a.vec[k].rows + c0) + (lane & 7);
+  float g[2] = {0.0f, 0.0f};
+#pragma unroll 2
+  for (int r = 8 * (8 * (lane >> 3) + w); r < a.B; r += 256) {
+    uint32_t u[8];
+    float h[2][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) u[i] = src[static_cast<size_t>(r + i) * (HID / 2)];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      h[0][i] = __uint_as_float(u[i] << 16);
+      h[1][i] = __uint_as_float(u[i] & 0xffff0000u);
+    }
+    if (k == 3) {
+      const float4 d0 = *reinterpret_cast<const float4 *>(a.dy + r);
+      const float4 d1 = *reinterpret_cast<const float4 *>(a.dy + r + 4);
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        g[q] += h[q][0] * d0.x + h[q][1] * d0.y + h[q][2] * d0.z + h[q][3] * d0.w +
+                h[q][4] * d1.x + h[q][5] * d1.y + h[q][6] * d1.z + h[q][7] * d1.w;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) g[q] += h[q][i];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    g[q] += __shfl_xor_sync(0xffffffffu, g[q], 16);
+    g[q] += __shfl_xor_sync(0xffffffffu, g[q], 8);
+  }
+  if (lane < 8) *reinterpret_cast<float2 *>(part + w * VEC_COLS + 2 * lane) = make_float2(g[0], g[1]);
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * VEC_WARPS) : "memory");
+  if (w == 0 && lane < VEC_COLS) {
+    float t[VEC_WARPS];
+#pragma unroll
+    for (int q = 0; q < VEC_WARPS; ++q) t[q] = part[q * VEC_COLS + lane];
+#pragma unroll
+    for (int o = 4; o; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < o; ++q) t[q] += t[q + o];
+    vec_update(a, a.vec[k], c0 + lane, t[0]);
+  }
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * VEC_WARPS) : "memory");  // part is free again
 }
 
 // tiles of 128 x 128 weights: 16 of layer 3, 16 of layer 2, 4 of layer 1
 constexpr int GRAD_TILES = 36;
 constexpr int RED_BYTES = 2 * BM * BN * 4;  // two partial tiles, over the ring
 constexpr int TILE_T_BYTES = BN * (BM + 8) * 2;  // W^T on its way out, rows padded
-constexpr int GRADS_SMEM = 1024 + RED_BYTES + TILE_T_BYTES + 256;
+constexpr int GRADS_SMEM = 1024 + RED_BYTES + TILE_T_BYTES + 256 + VEC_WARPS * VEC_COLS * 4;
 static_assert(RED_BYTES >= STAGES * 2 * TILE_BYTES, "the partial tiles replace the ring");
 
 // One cluster per tile of dW = dZ^T A (a product over the batch): its CTAs take
@@ -915,8 +899,7 @@ static_assert(RED_BYTES >= STAGES * 2 * TILE_BYTES, "the partial tiles replace t
 // each with an accumulator of its own), lay the partial tiles down in shared
 // memory, and each sums a share of the rows over all parts in order, applies
 // Adam and writes W and W^T.  Warps that do not feed the tensor cores compute
-// the vectors' gradients meanwhile, from the rows kernel's sums of 32 rows (they
-// read every operand once more before).  Bound by L2 reads at 4,096 rows (75 MB of
+// the vectors' gradients meanwhile.  Bound by L2 reads at 4,096 rows (75 MB of
 // operands in 9.5 us); 15 us in all, where the seven launches it replaces took
 // 40.
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -933,6 +916,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + RED_BYTES + TILE_T_BYTES);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 1);
   volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  float *vec_part = reinterpret_cast<float *>(smem + RED_BYTES + TILE_T_BYTES + 256);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES), done = smem_u32(bars + 2 * STAGES);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = static_cast<int>(cluster_rank());
@@ -996,9 +980,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     umma_commit(done);  // arrives once every product above has completed
   } else if (warp >= 2) {
     if (blockIdx.x == 0 && tid == 64) *a.clear = 0.0f;
-    const int stride = static_cast<int>(gridDim.x) * 14;
-    for (int e = static_cast<int>(blockIdx.x) * 14 + warp - 2; e < VEC_ELEMS; e += VEC_U * stride)
-      vec_adam(a, e, stride, lane);
+    if (warp < 2 + VEC_WARPS) {
+      for (int task = blockIdx.x; task < VEC_TASKS; task += gridDim.x)
+        vec_adam(a, task, vec_part, warp - 2, lane);
+    } else if (blockIdx.x == gridDim.x - 1 && warp == 2 + VEC_WARPS) {  // b4: sum dy
+      float g = 0.0f;
+      for (int j = lane; j < a.B; j += 32) g += a.dy[j];
+#pragma unroll
+      for (int o = 16; o; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+      if (lane == 0) vec_update(a, a.vec[4], 0, g);
+    }
   }
   __syncwarp();
   bool failed = !mbar_wait(done, 0, nullptr);
@@ -1202,9 +1193,8 @@ struct emt6_mlp {
   // parameters: FP32 masters, Adam moments, BF16 copies (W; W^T of layers 2, 3)
   DevArr<float> w[3], m[3], v[3], b[3], bm[3], bv[3], w4, m4, v4, b4, mb4, vb4;
   DevArr<__nv_bfloat16> wb[3], wbt[3];
-  DevArr<__nv_bfloat16> X16, A[2], dZ[3];  // operands of the weight gradients, [max_batch][columns]
+  DevArr<__nv_bfloat16> X16, A[3], dZ[3];  // operands of the weight gradients, [max_batch][columns]
   DevArr<uint4> Z[3];                      // pre-activations, 8 to an element
-  DevArr<float> part;                      // vector gradients' sums, [4][512][max_batch / 32]
   DevArr<float> dy, loss, gradw[3], gradv[5];
   int split_override = 0;  // 0: choose per batch size
   DevArr<int> err;
@@ -1245,7 +1235,7 @@ bool build_maps(emt6_mlp *net) {
   for (int l = 0; l < 3 && ok; ++l) {
     ok = make_map(&net->mW[l], net->wb[l].p, rows_of(l), cols_of(l)) &&
          make_map(&net->mRows.dz[l], net->dZ[l].p, net->max_batch, HID, 64);
-    if (l < 2) ok = ok && make_map(&net->mRows.a[l], net->A[l].p, net->max_batch, HID, 64);
+    ok = ok && make_map(&net->mRows.a[l], net->A[l].p, net->max_batch, HID, 64);
     if (l > 0) ok = ok && make_map(&net->mWT[l], net->wbt[l].p, cols_of(l), rows_of(l));
   }
   return ok;
@@ -1293,8 +1283,6 @@ int run_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean, cons
       a.loss = net->loss.p + net->slot;
       a.x16 = net->X16.p;
       for (int l = 0; l < 3; ++l) a.z[l] = net->Z[l].p;
-      a.part = net->part.p;
-      a.ld = static_cast<size_t>(net->max_batch / 32);
       e = launch_clusters(mlp_rows_kernel<true>, grid, CLUSTER, ROWS_SMEM, net->stream, net->mW[0],
                           net->mW[1], net->mW[2], net->mWT[1], net->mWT[2], net->mRows, a);
     } else {
@@ -1319,8 +1307,6 @@ int run_grads(emt6_mlp *net, int B, bool apply, float lr) {
   GradsArgs a;
   std::memset(&a, 0, sizeof(a));
   const float step = static_cast<float>(net->step + 1);
-  a.ld = static_cast<size_t>(net->max_batch / 32);
-  const size_t vec = HID * a.ld;
   for (int l = 0; l < 3; ++l) {
     a.w[l] = net->w[l].p;
     a.m[l] = net->m[l].p;
@@ -1328,10 +1314,10 @@ int run_grads(emt6_mlp *net, int B, bool apply, float lr) {
     a.wb[l] = net->wb[l].p;
     a.wbt[l] = net->wbt[l].p;
     a.grad[l] = apply ? nullptr : net->gradw[l].p;
-    a.vec[l] = {net->b[l].p, net->bm[l].p, net->bv[l].p, net->part.p + l * vec, apply ? nullptr : net->gradv[l].p, HID};
+    a.vec[l] = {net->b[l].p, net->bm[l].p, net->bv[l].p, net->dZ[l].p, apply ? nullptr : net->gradv[l].p};
   }
-  a.vec[3] = {net->w4.p, net->m4.p, net->v4.p, net->part.p + 3 * vec, apply ? nullptr : net->gradv[3].p, HID};
-  a.vec[4] = {net->b4.p, net->mb4.p, net->vb4.p, nullptr, apply ? nullptr : net->gradv[4].p, 1};
+  a.vec[3] = {net->w4.p, net->m4.p, net->v4.p, net->A[2].p, apply ? nullptr : net->gradv[3].p};
+  a.vec[4] = {net->b4.p, net->mb4.p, net->vb4.p, nullptr, apply ? nullptr : net->gradv[4].p};
   a.dy = net->dy.p;
   a.clear = net->loss.p + (net->slot ^ 1);
   a.B = B;
@@ -1426,9 +1412,9 @@ int emt6_mlp_create(int max_batch, uint64_t seed, int device, emt6_mlp **out) {
   ok = ok && net->w4.alloc(H) && net->m4.alloc(H) && net->v4.alloc(H) && net->b4.alloc(1) &&
        net->mb4.alloc(1) && net->vb4.alloc(1) &&
        net->X16.alloc(static_cast<size_t>(max_batch) * INP) && net->dy.alloc(max_batch) &&
-       net->part.alloc(4 * BH / 32) && net->loss.alloc(2) && net->err.alloc(1);
+       net->loss.alloc(2) && net->err.alloc(1);
   for (int l = 0; l < 3 && ok; ++l)
-    ok = (l == 2 || net->A[l].alloc(BH)) && net->dZ[l].alloc(BH) && net->Z[l].alloc(BH / 8);
+    ok = net->A[l].alloc(BH) && net->dZ[l].alloc(BH) && net->Z[l].alloc(BH / 8);
   for (int i = 0; i < 5 && ok; ++i) ok = net->gradv[i].alloc(i < 4 ? H : 1);
   if (!ok) {
     if (net->stream) cudaStreamDestroy(net->stream);
