@@ -160,21 +160,24 @@ class Surrogate:
                                             ctypes.byref(loss)))
         return loss.value
 
+    _PIECE = 1 << 18
+
     def _predict_rows(self, x: np.ndarray, mean=None, std=None) -> np.ndarray:
         """Network output for rows of 100 FP32 features: one upload, one launch
-        for all rows, one read-back; with `mean` and `std` the rows are raw and
-        standardised on the device."""
+        and one read-back per `_PIECE` rows (105 MB on the device, however many
+        rows there are); with `mean` and `std` the rows are raw and standardised
+        on the device."""
         torch = self._torch
-        n = len(x)
-        out = np.zeros(n, np.float32)
-        if n == 0:
-            return out
-        xd = self._to_dev(x)
-        with torch.cuda.stream(self._stream()):
-            yd = torch.empty(n, dtype=torch.float32, device=f"cuda:{self.device}")
-            N.check(N.lib().emt6_mlp_predict_rows(self._h, xd.data_ptr(), n, N.ptr(mean),
-                                                  N.ptr(std), yd.data_ptr()))
-            torch.from_numpy(out).copy_(yd)
+        out = np.zeros(len(x), np.float32)
+        for i in range(0, len(x), self._PIECE):
+            part = x[i:i + self._PIECE]
+            n = len(part)
+            xd = self._to_dev(part)
+            with torch.cuda.stream(self._stream()):
+                yd = torch.empty(n, dtype=torch.float32, device=f"cuda:{self.device}")
+                N.check(N.lib().emt6_mlp_predict_rows(self._h, xd.data_ptr(), n, N.ptr(mean),
+                                                      N.ptr(std), yd.data_ptr()))
+                torch.from_numpy(out[i:i + n]).copy_(yd)
         return out
 
     def predict_std(self, x_std) -> np.ndarray:

@@ -65,6 +65,14 @@ def test_more_rows_than_run_at_once(n):
     assert np.array_equal(y, np.concatenate([net.predict(x[i:i + 999]) for i in range(0, n, 999)]))
 
 
+def test_rows_in_pieces_on_the_device():
+    net = _net(128)
+    x = np.random.default_rng(4).normal(size=(1000, 100)).astype(np.float32)
+    y = net.predict_std(x)
+    net._PIECE = 333
+    assert np.array_equal(net.predict_std(x), y) and np.array_equal(net.predict_std(x[:0]), y[:0])
+
+
 # 128 and 384 rows: one part; 640: two; 1024: four; 2048: eight
 @pytest.mark.parametrize("batch", [128, 384, 640, 1024, 2048])
 def test_gradients_and_step_at_every_split(batch):
