@@ -300,7 +300,7 @@ struct emt6_batch {
   unsigned long long launches = 0;  // kernels issued by this handle
   bool use_graph = false;
   bool occ_known = false;
-  bool resident = false;
+  bool resident = false, lone = false;
   int sms = 0, per_sm[emt6::kTiers] = {1, 1};
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_key[5] = {0, 0, 0, 0, 0};
@@ -416,8 +416,10 @@ struct emt6_batch {
     for (int tier = 0; tier < emt6::kTiers; ++tier)
       per_sm[tier] = std::max(emt6::max_ctas_per_sm(kp, tier), 1);
     // A batch that is resident at once needs neither an order nor a queue: its
-    // CTAs all start together.
+    // CTAs all start together.  One that has an SM per simulation takes the lone
+    // tier, in one launch.
     resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierWide]) * sms;
+    lone = n <= (int64_t)emt6::max_ctas_per_sm(kp, emt6::kTierLone) * sms;
     if (!side) EMT6_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     if (!join) EMT6_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
     if (!fork) EMT6_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
@@ -444,9 +446,9 @@ struct emt6_batch {
     while (t < target) {
       const uint32_t end = (uint32_t)std::min<uint64_t>(target, (uint64_t)t + chunk);
       if (has_horizon && t >= max_horizon) break;
-      if (resident && end - t < kSplitSteps) {
+      if (lone || (resident && end - t < kSplitSteps)) {
         a.order = nullptr;
-        const int rc = launch(a, end, emt6::kTierWide, stream, count);
+        const int rc = launch(a, end, lone ? emt6::kTierLone : emt6::kTierWide, stream, count);
         if (rc) return rc;
       } else {
         // The tiers side by side, the larger simulations' first, each on the

@@ -4,10 +4,11 @@
 // a whole launch of N steps: the fields, the site-state bytes and the occupied
 // list live in shared memory for the launch; per-site cell records (48 B)
 // stay in global memory, where the few hundred live cells of each resident
-// simulation stay L2-resident.  Two kernels: run_kernel<false> (5 CTAs/SM, a
+// simulation stay L2-resident.  Three kernels: run_kernel<kTierNarrow> (5 CTAs/SM, a
 // window of at most 40 lattice rows on chip) for regions that fit a tile of 32
-// slots per lane, and run_kernel<true> (4 CTAs/SM, the whole lattice) for
-// larger ones.  Per step (reference cadence,
+// slots per lane, run_kernel<kTierWide> (4 CTAs/SM, the whole lattice) for
+// larger ones, and run_kernel<kTierLone> (384 threads) for batches of at most one
+// simulation per SM.  Per step (reference cadence,
 // src/emt6ro/simulation/simulation.cu:153-166):
 //   t % 128 == 0  rebuild the occupied list        (simulation.cu:41-64)
 //   t % 32  == 0  ROI + circular fixed-value mask   (diffusion.cu:65-100)
@@ -35,6 +36,10 @@ __device__ double g_instr_sum_death_prob;
 __device__ unsigned long long g_instr_hist[600];  // irradiation bins, then time-in-repair
 
 constexpr int kThreads = 96;  // one warp per field
+// kTierLone: the wide kernel's registers for as many warps as an SM holds.  All
+// take part in the cell update, the list and the diffusion of large regions.
+constexpr int kThreadsLone = 384;
+__host__ __device__ constexpr int threads_of(int tier) { return tier == kTierLone ? kThreadsLone : kThreads; }
 
 struct Misc {
   float4 met[4];  // consumption by metabolic mode
@@ -42,8 +47,6 @@ struct Misc {
   uint32_t n, n0;
   int has_multi;
   int winner, target;
-  int red[kThreads / 32][4];
-  uint32_t stripe[kThreads / 32][32];  // list rebuild: entries per warp's rows and stripe
   unsigned int ins[4];
   double ins_dp;
   unsigned long long diffused;
@@ -51,7 +54,13 @@ struct Misc {
   TileMap tm;    // the region's tile
   int park;      // the narrow kernel cannot take the next step of this simulation
   int w0, wneed;  // first row of the field window on chip (-1: none), the one the region needs
+  // behind it, for each warp: reductions, and its rows' list entries per stripe
+  __device__ int (*red())[4] { return reinterpret_cast<int (*)[4]>(this + 1); }
+  __device__ uint32_t (*stripe())[32] {
+    return reinterpret_cast<uint32_t (*)[32]>(red() + (blockDim.x >> 5));
+  }
 };
+constexpr uint32_t kMiscPerWarp = 4 * 4 + 32 * 4;
 
 __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
@@ -67,7 +76,7 @@ constexpr int kWindowRows = 40;
 constexpr uint32_t kEntryBytes = 4 + 4 + 2 + 1, kMinEntries = 1024;
 
 struct SmemLayout {
-  uint32_t fld, st, colmask, masks, edge, misc, h0, h1, list, fl, total;
+  uint32_t fld, st, colmask, masks, edge, parts, misc, h0, h1, list, fl, total;
   int rows, plane;    // window rows, floats of a field's window
   int entries, held;  // list capacity, entries with their clocks on chip
 };
@@ -87,9 +96,12 @@ __host__ __device__ inline SmemLayout smem_layout(int H, int W, int lcap, int ti
   L.colmask = o; o += 64 * 8;
   L.masks = o; o += 3u * (wide ? kWordsWide : kWordsNarrow) * 32u * 4u;
   L.edge = o; o += 3u * (wide ? kEdgeWide : kEdgeNarrow) * 4u;
-  L.misc = o; o += align_up(sizeof(Misc), 16);
+  o = align_up(o, 16);
+  L.parts = o; o += tier == kTierLone ? 3u * kPartSlots * 8u : 0u;
+  L.misc = o; o += align_up(sizeof(Misc) + threads_of(tier) / 32 * kMiscPerWarp, 16);
   // a rebuilt list holds at most the interior, and 128 divisions can follow
-  const uint32_t all = align_up((uint32_t)lcap - 128u, 16), room = (wide ? 111u : 88u) * 512u;
+  const uint32_t all = align_up((uint32_t)lcap - 128u, 16),
+                 room = (tier == kTierLone ? 444u : wide ? 111u : 88u) * 512u;
   const uint32_t left = o < room ? room - o : 0u;
   uint32_t entries = all, held;
   if (wide) {
@@ -124,10 +136,10 @@ template <int NT>
 __device__ __forceinline__ int block_min(int v, Misc *m) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   v = __reduce_min_sync(kFull, v);
-  if (lane == 0) m->red[wid][0] = v;
+  if (lane == 0) m->red()[wid][0] = v;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < NT / 32; ++w) v = min(v, m->red[w][0]);
+  for (int w = 0; w < NT / 32; ++w) v = min(v, m->red()[w][0]);
   __syncthreads();
   return v;
 }
@@ -155,12 +167,12 @@ __device__ void rebuild_list(uint8_t *st, uint16_t *list, Misc *m, int H, int W,
     const uint8_t *q = st + r * W + k;
     cnt += (c0 && q[0] == kOccupied) + (c1 && q[32] == kOccupied);
   }
-  m->stripe[wid][k] = cnt;
+  m->stripe()[wid][k] = cnt;
   __syncthreads();
   uint32_t before = 0, all = 0;  // of this stripe: earlier rows; all rows
 #pragma unroll
   for (int w = 0; w < NWARP; ++w) {
-    const uint32_t v = m->stripe[w][k];
+    const uint32_t v = m->stripe()[w][k];
     if (w < wid) before += v;
     all += v;
   }
@@ -247,14 +259,14 @@ __device__ void compute_roi(const uint8_t *st, const uint16_t *list, uint64_t *c
   v[2] = __reduce_max_sync(kFull, v[2]);
   v[3] = __reduce_max_sync(kFull, v[3]);
   if (lane == 0)
-    for (int k = 0; k < 4; ++k) m->red[wid][k] = v[k];
+    for (int k = 0; k < 4; ++k) m->red()[wid][k] = v[k];
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < NWARP; ++w) {
-    v[0] = min(v[0], m->red[w][0]);
-    v[1] = min(v[1], m->red[w][1]);
-    v[2] = max(v[2], m->red[w][2]);
-    v[3] = max(v[3], m->red[w][3]);
+    v[0] = min(v[0], m->red()[w][0]);
+    v[1] = min(v[1], m->red()[w][1]);
+    v[2] = max(v[2], m->red()[w][2]);
+    v[3] = max(v[3], m->red()[w][3]);
   }
   __syncthreads();
   if (v[2] == 0 && v[3] == 0) {
@@ -274,10 +286,10 @@ __device__ void compute_roi(const uint8_t *st, const uint16_t *list, uint64_t *c
     }
   }
   far = __reduce_max_sync(kFull, far);
-  if (lane == 0) m->red[wid][0] = far;
+  if (lane == 0) m->red()[wid][0] = far;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < NWARP; ++w) far = max(far, m->red[w][0]);
+  for (int w = 0; w < NWARP; ++w) far = max(far, m->red()[w][0]);
   const int dist = (int)ceilf(sqrtf((float)far));
   const int sub_r = (midr <= dist) ? 1 : midr - dist;
   const int sub_c = (midc <= dist) ? 1 : midc - dist;
@@ -415,6 +427,22 @@ __device__ __forceinline__ void diffuse_step(float *fld, int plane, const uint32
 #undef EMT6_TILE
 #undef EMT6_LARGE
   static_assert(kNumTiles == 21 && kNarrowTiles == 12, "every tile has a case above");
+}
+
+// The same of a large region by all 12 warps of the lone tier.
+constexpr int kPartTiles = 16;  // from 72 slots per lane on (diffuse_parts)
+__device__ __forceinline__ void diffuse_by_parts(float *fld, int plane, const uint64_t *colmask,
+                                                 float2 *slots, const Misc *m, const KParams &p) {
+  static_assert(kThreadsLone == 384, "four warps per field");
+  const int wid = __shfl_sync(kFull, threadIdx.x >> 5, 0), field = wid >> 2, part = wid & 3;
+  const int h = m->roi[2], w = m->roi[3], r0 = m->roi[0] - m->w0, c0 = m->roi[1];
+  const float ext = p.ext[field], ca = p.da[field], cb = p.db[field], cd = p.dd[field];
+  float *f = fld + field * plane;
+  slots += field * kPartSlots;
+  if (h + 2 <= 4 * 13)
+    diffuse_parts<13>(f, colmask, slots, part, 1 + field, r0, c0, h, w, p.W, ext, ca, cb, cd, p.nfree);
+  else
+    diffuse_parts<14>(f, colmask, slots, part, 1 + field, r0, c0, h, w, p.W, ext, ca, cb, cd, p.nfree);
 }
 
 // Field window (rows w0 .. w0 + rows - 1 of the three planes) from and to
@@ -730,17 +758,22 @@ __device__ __forceinline__ void count_diffused(Misc *m, const KParams &p, uint32
 // ---------------------------------------------------------------------------
 // the fused step kernel
 // ---------------------------------------------------------------------------
-// WIDE = false: regions that fit a tile of at most 32 slots per lane (discs up
+// kTierNarrow: regions that fit a tile of at most 32 slots per lane (discs up
 // to distance 16, clipped regions up to 32 x 32), 5 CTAs/SM.  A simulation it
 // cannot hold (region, window or list) is parked at the start of that step for
-// the WIDE = true kernel: any simulation, 4 CTAs/SM.
-template <bool WIDE>
-__global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __grid_constant__ RunArgs a, uint32_t t_end) {
-  constexpr int NT = kThreads;
+// kTierWide: any simulation, 4 CTAs/SM.  kTierLone: any simulation,
+// one CTA of 384 threads per SM, for batches that leave SMs idle otherwise: a
+// step's latency instead of the SM's throughput (300 steps: one disc of radius 10
+// 1.56 vs 1.67 ms, 100 of them 3.09 vs 3.23; 152 of radius 24, 200 steps, 3.2 vs
+// 6.0).
+template <int TIER>
+__global__ void __launch_bounds__(threads_of(TIER), TIER == kTierLone ? 1 : TIER == kTierWide ? 4 : 5)
+    run_kernel(const __grid_constant__ RunArgs a, uint32_t t_end) {
+  constexpr int NT = threads_of(TIER);
+  constexpr bool WIDE = TIER != kTierNarrow;
   extern __shared__ __align__(16) uint8_t sm[];
   const KParams &p = a.p;
   const int H = p.H, W = p.W, HW = p.HW;
-  constexpr int TIER = WIDE ? kTierWide : kTierNarrow;
   const SmemLayout L = smem_layout(H, W, p.lcap, TIER);
   float *fld = reinterpret_cast<float *>(sm + L.fld);
   uint8_t *st = sm + L.st;
@@ -874,7 +907,10 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
           list[e] = (uint16_t)(s | (vac << kSiteBits));
         }
       dirty = false;
-      diffuse_step<WIDE>(fld, plane, masks, edge, m, p);
+      if (TIER == kTierLone && m->tm.tile >= kPartTiles)
+        diffuse_by_parts(fld, plane, colmask, reinterpret_cast<float2 *>(sm + L.parts), m, p);
+      else if (NT == kThreads || wid < 3)
+        diffuse_step<WIDE>(fld, plane, masks, edge, m, p);
       __syncthreads();
 
       // ---- cell update (simulation.cu:84-96) ----
@@ -1080,11 +1116,11 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5) run_kernel(const __gri
 #pragma unroll
     for (int o = 16; o; o >>= 1) live += __shfl_xor_sync(kFull, live, o);
     __syncthreads();
-    if (lane == 0) m->red[wid][1] = live;
+    if (lane == 0) m->red()[wid][1] = live;
     __syncthreads();
     if (tid == 0) {
       int tot = 0;
-      for (int w2 = 0; w2 < NT / 32; ++w2) tot += m->red[w2][1];
+      for (int w2 = 0; w2 < NT / 32; ++w2) tot += m->red()[w2][1];
       a.counts[sim] = (uint32_t)tot;
       a.meta[sim] = make_int4((int)m->n, (int)m->n0, m->has_multi, 0);
       for (int k2 = 0; k2 < 5; ++k2) a.roi[sim * 8 + k2] = m->roi[k2];
@@ -1354,34 +1390,33 @@ __global__ void __launch_bounds__(kThreads, WIDE ? 4 : 5)
 // ---------------------------------------------------------------------------
 // the dynamic shared-memory limit is raised once per device and size (the
 // attribute call is kept out of CUDA-graph captures)
-static size_t g_smem_set[2][64];
+static size_t g_smem_set[3][64];
 
-static cudaError_t ensure_smem(bool wide, size_t smem) {
+using RunKernel = void (*)(RunArgs, uint32_t);
+static RunKernel kernel_of(int tier) {
+  return tier == kTierNarrow ? run_kernel<kTierNarrow>
+         : tier == kTierWide ? run_kernel<kTierWide> : run_kernel<kTierLone>;
+}
+
+static cudaError_t ensure_smem(int tier, size_t smem) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) dev = 63;
-  if (g_smem_set[wide][dev] >= smem) return cudaSuccess;
-  e = wide ? cudaFuncSetAttribute(run_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)
-           : cudaFuncSetAttribute(run_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem);
-  // both kernels ask for the same split of the L1, so their CTAs share SMs
-  if (e == cudaSuccess)
-    e = wide ? cudaFuncSetAttribute(run_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100)
-             : cudaFuncSetAttribute(run_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (e == cudaSuccess) g_smem_set[wide][dev] = smem;
+  if (g_smem_set[tier][dev] >= smem) return cudaSuccess;
+  const RunKernel k = kernel_of(tier);
+  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // all ask for the same split of the L1, so that their CTAs share SMs
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  if (e == cudaSuccess) g_smem_set[tier][dev] = smem;
   return e;
 }
 
 cudaError_t launch_run(const RunArgs &a, uint32_t t_end, int tier, int grid, cudaStream_t stream) {
   const size_t smem = run_kernel_smem(a.p.H, a.p.W, a.p.lcap, tier);
-  cudaError_t e = ensure_smem(tier != kTierNarrow, smem);
+  cudaError_t e = ensure_smem(tier, smem);
   if (e != cudaSuccess) return e;
-  if (tier != kTierNarrow)
-    run_kernel<true><<<grid, kThreads, smem, stream>>>(a, t_end);
-  else
-    run_kernel<false><<<grid, kThreads, smem, stream>>>(a, t_end);
+  kernel_of(tier)<<<grid, threads_of(tier), smem, stream>>>(a, t_end);
   return cudaGetLastError();
 }
 
@@ -1411,19 +1446,12 @@ cudaError_t launch_reset(const ResetArgs &a, cudaStream_t stream) {
 }
 
 int max_ctas_per_sm(const KParams &p, int tier) {
-  const bool wide = tier != kTierNarrow;
   const size_t smem = run_kernel_smem(p.H, p.W, p.lcap, tier);
   int n = 0;
-  if (ensure_smem(wide, smem) != cudaSuccess) return 0;
-  if (wide) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, run_kernel<true>, kThreads, smem) !=
-        cudaSuccess)
-      return 0;
-  } else {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, run_kernel<false>, kThreads, smem) !=
-        cudaSuccess)
-      return 0;
-  }
+  if (ensure_smem(tier, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel_of(tier), threads_of(tier), smem) !=
+          cudaSuccess)
+    return 0;
   return n;
 }
 

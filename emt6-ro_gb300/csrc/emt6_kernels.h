@@ -57,7 +57,7 @@ struct ResetArgs {
 // takes the simulations that the narrow one left short of the target step
 // (regions too wide or lists too long for the shared memory that lets 5 CTAs
 // share an SM); it holds any.
-enum { kTierNarrow = 0, kTierWide = 1, kTiers = 2 };
+enum { kTierNarrow = 0, kTierWide = 1, kTiers = 2, kTierLone = 2 };
 size_t run_kernel_smem(int H, int W, int lcap, int tier);
 int max_ctas_per_sm(const KParams &p, int tier);
 // Advance the simulations that `tier` holds to step min(t_end, horizon).

@@ -95,3 +95,29 @@ def test_tiers_side_by_side(schedule, layouts, params, oracle):
         assert (small.counts() == counts[m]).all()
         for j in range(0, 100, 9):
             assert small.state(j).sites.tobytes() == b.state(base + j).sites.tobytes(), j
+
+
+@pytest.mark.parametrize("dims", [(51, 51), (54, 60), (49, 50)])
+def test_large_regions_on_every_tier(dims, oracle):
+    """Regions of 45 to 56 rows, centred and clipped, with an SM each, as part of
+    a batch that is one wave, and of a larger one: the oracle's lattices."""
+    from emt6ro import workloads as wl
+    from emt6ro.batch import Batch
+    params = wl.default_parameters()
+    params.native.lattice_height, params.native.lattice_width = dims
+    h, w = dims[0] + 2, dims[1] + 2
+    tumors = [wl.disc_tumor(params, r, seed=40 + k, center=(h // 2 + dr, w // 2 + dc))
+              for k, (r, dr, dc) in enumerate([(21, 0, 0), (22, 0, 1), (23, 0, 0), (24, 0, 0),
+                                               (24, 3, -2), (26, -4, 5), (20, 9, 0), (27, 0, 0)])]
+    steps, k = 70, len(tumors)
+    ob = oracle.Batch(oracle.params_copy(params.native), k, 9)
+    batches = [Batch(params, tumors, [[(0, 0.5)]], np.arange(n) % k, np.zeros(n, np.int32), seed=9)
+               for n in (k, 300, 700)]
+    for j in range(k):
+        ob.set(j, tumors[j].sites, batches[0].doses[0], resolution=300, length=144_000)
+    ob.run(steps, nthreads=8)
+    for b in batches:
+        b.run(steps)
+        assert (b.counts()[:k] == ob.counts()).all()
+        for j in range(k):
+            assert b.state(j).sites.tobytes() == ob.get(j).tobytes(), (b.n, j)
