@@ -900,8 +900,7 @@ static_assert(RED_BYTES >= STAGES * 2 * TILE_BYTES, "the partial tiles replace t
 // memory, and each sums a share of the rows over all parts in order, applies
 // Adam and writes W and W^T.  Warps that do not feed the tensor cores compute
 // the vectors' gradients meanwhile.  Bound by L2 reads at 4,096 rows (75 MB of
-// operands in 9.5 us); 15 us in all, where the seven launches it replaces took
-// 40.
+// operands in 9.5 us); the seven launches it replaces took 40.
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     mlp_grads_kernel(const __grid_constant__ CUtensorMap tmZ0, const __grid_constant__ CUtensorMap tmZ1,
                      const __grid_constant__ CUtensorMap tmZ2, const __grid_constant__ CUtensorMap tmX,
