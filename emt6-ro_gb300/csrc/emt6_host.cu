@@ -420,9 +420,9 @@ struct emt6_batch {
     // tier, in one launch.
     resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierWide]) * sms;
     lone = n <= (int64_t)emt6::max_ctas_per_sm(kp, emt6::kTierLone) * sms;
-    if (!side) EMT6_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-    if (!join) EMT6_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-    if (!fork) EMT6_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    if (!lone && !side) EMT6_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    if (!lone && !join) EMT6_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    if (!lone && !fork) EMT6_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     occ_known = true;
     return EMT6_OK;
   }
