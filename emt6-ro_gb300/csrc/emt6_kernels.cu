@@ -238,14 +238,29 @@ __device__ __forceinline__ void build_colmask(uint64_t *colmask, int h, int w, i
 // product's error s (inv W - 2^20) / (2^20 W) stays below 1 / W)
 __device__ __forceinline__ int row_of(int s, uint32_t inv) { return (int)((uint32_t)s * inv >> 20); }
 
-// The occupied sites are all in the list (rebuilt, then appended to).
+// The occupied sites are all in the list (rebuilt, then appended to), but for cells
+// that divided onto a vacant border site of the last row or column before the last
+// rebuild: the list leaves those out (simulation.cu:50-53), the region does not.
 template <int NT>
 __device__ void compute_roi(const uint8_t *st, const uint16_t *list, uint64_t *colmask, Misc *m,
                             int H, int W) {
   constexpr int NWARP = NT / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t n = m->n, inv = ((1u << 20) + W - 1) / W;
+  // site q of the last row, then of the last column
+  const auto edge = [=](int q, int &r, int &c) {
+    r = q < W ? H - 1 : q - W;
+    c = q < W ? q : W - 1;
+  };
   int v[4] = {H, W, 0, 0};
+  for (int q = threadIdx.x; q < W + H - 1; q += NT) {
+    int r, c;
+    edge(q, r, c);
+    if ((st[r * W + c] & kStMask) == kOccupied) {
+      v[0] = min(v[0], r); v[1] = min(v[1], c);
+      v[2] = max(v[2], r); v[3] = max(v[3], c);
+    }
+  }
   for (uint32_t e = threadIdx.x; e < n; e += NT) {
     const int s = list[e] & kSiteMask;
     if ((st[s] & kStMask) == kOccupied) {
@@ -285,6 +300,13 @@ __device__ void compute_roi(const uint8_t *st, const uint16_t *list, uint64_t *c
       far = max(far, (midr - r) * (midr - r) + (midc - c) * (midc - c));
     }
   }
+  if (v[2] == H - 1 || v[3] == W - 1)
+    for (int q = threadIdx.x; q < W + H - 1; q += NT) {
+      int r, c;
+      edge(q, r, c);
+      if ((st[r * W + c] & kStMask) == kOccupied)
+        far = max(far, (midr - r) * (midr - r) + (midc - c) * (midc - c));
+    }
   far = __reduce_max_sync(kFull, far);
   if (lane == 0) m->red()[wid][0] = far;
   __syncthreads();

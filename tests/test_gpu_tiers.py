@@ -121,3 +121,37 @@ def test_large_regions_on_every_tier(dims, oracle):
         assert (b.counts()[:k] == ob.counts()).all()
         for j in range(k):
             assert b.state(j).sites.tobytes() == ob.get(j).tobytes(), (b.n, j)
+
+
+@pytest.mark.parametrize("n", [8, 160, 700])
+def test_cells_on_a_vacant_far_border_count_for_the_region(n, params, oracle):
+    """A lattice whose last row and column are vacant, not mocked: cells divide
+    onto them and leave the list at its next rebuild, but stay in the region."""
+    from emt6ro import workloads as wl
+    from emt6ro.batch import Batch
+    tumors = []
+    for k, center in enumerate([(50, 50), (51, 26), (26, 51), (51, 12)]):
+        t = wl.disc_tumor(params, 6, seed=300 + k, center=center)
+        s = t.sites
+        s["state"][-1, 1:] = 0
+        s["state"][1:, -1] = 0
+        live = s["state"] == 1  # divide in the steps before the rebuild at step 128
+        rng = np.random.default_rng(k)
+        s["phase"][live] = 3
+        s["proliferation_time"][live] = (s["cycle_times"][live][:, 3] - 0.17
+                                         - 0.04 * rng.random(live.sum()))
+        tumors.append(t)
+    steps, k = 300, 8
+    st = np.arange(n) % 4
+    b = Batch(params, tumors, [[]], st, np.zeros(n, np.int32), seed=6)
+    b.run(steps)
+    ob = oracle.Batch(oracle.params_copy(params.native), k, 6)
+    for j in range(k):
+        ob.set(j, tumors[st[j]].sites, b.doses[0], resolution=300, length=144_000)
+    ob.run(steps, nthreads=8)
+    left_out = [np.setdiff1d(np.flatnonzero(ob.get(j)["state"] == 1), ob.occupied_list(j))
+                for j in range(k)]
+    assert sum(map(len, left_out)) > 10
+    assert (b.counts()[:k] == ob.counts()).all()
+    for j in range(k):
+        assert b.state(j).sites.tobytes() == ob.get(j).tobytes(), j
