@@ -419,6 +419,10 @@ struct RowsArgs {
   uint4 *z[3];         // pre-activations, 8 columns of a row each (z_at)
   __nv_bfloat16 *x16;  // [n][128]
   int *err;
+  // test hook (emt6_test_mlp_stall): the phase whose products the first CTA's
+  // issuer gives up on after waiting stall_ns (0: none) for them to complete
+  int stall_phase;
+  uint32_t stall_ns;
 };
 
 // where training's operands of the weight gradients go, [n][512]
@@ -626,7 +630,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       if (tid == 0) {
         load_tiles(phase, phase == 0 ? 2 : RING, nk);
       } else if (tid == 32) {
-        if (*abort || !arrived()) *abort = 1;
+        // waited for after an abort too: the peers' copies still come, each
+        // exchange's are counted on `in` before the next one's, and none may
+        // reach a CTA that has left
+        if (!arrived() || *abort) *abort = 1;
+        if (a.stall_ns && blockIdx.x == 0 && phase == a.stall_phase && !*abort &&
+            !mbar_wait(done, products & 1, nullptr, a.stall_ns))
+          *abort = 1;
         tc_fence_after();
         for (int kb = 0; kb < nk && !*abort; ++kb) {
           const int s = (used + kb) % RING;
@@ -815,6 +825,7 @@ struct GradsArgs {
   int B, splits;
   float lr, beta1, beta2, eps, bc1, bc2;
   int *err;
+  uint32_t stall_ns;  // test hook, as in RowsArgs: of the first CTA's products
 };
 
 __device__ __forceinline__ void vec_update(const GradsArgs &a, const VecAdam &p, int idx, float g) {
@@ -962,7 +973,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       ++issued;
     }
   } else if (tid == 32) {
-    for (int kb = 0; kb < nk; ++kb) {
+    if (a.stall_ns && blockIdx.x == 0 && !mbar_wait(done, 0, abort, a.stall_ns)) *abort = 1;
+    for (int kb = 0; kb < nk && !*abort; ++kb) {
       const int s = kb % STAGES;
       if (!mbar_wait(full0 + 8 * s, (kb / STAGES) & 1, abort)) {
         *abort = 1;
@@ -1196,12 +1208,22 @@ struct emt6_mlp {
   DevArr<uint4> Z[3];                      // pre-activations, 8 to an element
   DevArr<float> dy, loss, gradw[3], gradv[5];
   int split_override = 0;  // 0: choose per batch size
+  int stall_phase = 0;     // emt6_test_mlp_stall: PHASES - 1 and below, or kStallGrads
+  uint32_t stall_ns = 0;   // of the next launch concerned, 0: none
   DevArr<int> err;
   CUtensorMap mX, mW[3], mWT[3];
   RowsMaps mRows;
 };
 
 namespace {
+
+constexpr int kStallGrads = 5;
+
+// the stall asked of the launch about to be made, once
+uint32_t take_stall(emt6_mlp *net, bool grads) {
+  if (!net->stall_ns || grads != (net->stall_phase == kStallGrads)) return 0;
+  return std::exchange(net->stall_ns, 0u);
+}
 
 int rows_of(int) { return EMT6_MLP_HIDDEN; }
 int cols_of(int l) { return l == 0 ? EMT6_MLP_IN_PAD : EMT6_MLP_HIDDEN; }
@@ -1275,6 +1297,8 @@ int run_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean, cons
     a.w4 = net->w4.p;
     a.b4 = net->b4.p;
     a.err = net->err.p;
+    a.stall_phase = net->stall_phase;
+    a.stall_ns = take_stall(net, false);
     int grid = (a.n + BM - 1) / BM * CLUSTER;
     if (d_target) {
       a.target = d_target;
@@ -1328,6 +1352,7 @@ int run_grads(emt6_mlp *net, int B, bool apply, float lr) {
   a.bc1 = 1.0f - std::pow(net->beta1, step);
   a.bc2 = 1.0f - std::pow(net->beta2, step);
   a.err = net->err.p;
+  a.stall_ns = take_stall(net, true);
   // at most two parts per CTA (two accumulators, two tiles of shared memory),
   // and clusters of 4, 36 of which are resident at once
   const int cluster = a.splits < 4 ? a.splits : 4;
@@ -1568,6 +1593,15 @@ int emt6_mlp_sync(emt6_mlp *net) {
   if (!net) return fail("emt6_mlp_sync: null", EMT6_ERR_INVALID);
   cudaSetDevice(net->device);
   return read_err(net);
+}
+
+int emt6_test_mlp_stall(emt6_mlp *net, int phase, uint32_t stall_us) {
+  if (!net || phase < 0 || phase > kStallGrads || stall_us == 0 || stall_us > 100000)
+    return fail("emt6_test_mlp_stall: null handle, phase outside 0..5 or stall outside 1..100000 us",
+                EMT6_ERR_INVALID);
+  net->stall_phase = phase;
+  net->stall_ns = stall_us * 1000u;
+  return EMT6_OK;
 }
 
 int emt6_test_mlp_gemm(const void *d_a, const void *d_b, float *d_c, int M, int N, int K,

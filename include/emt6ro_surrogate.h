@@ -78,6 +78,13 @@ int emt6_mlp_set_splitk(emt6_mlp *net, int splits);
  * timed out since the last check. */
 int emt6_mlp_sync(emt6_mlp *net);
 
+/* Failure-path hook (no reference counterpart): in the handle's next launch of the
+ * row kernel (phase 0..2: the hidden layers, 3..4: the error back through layers 3
+ * and 2, training only) or of the gradient kernel (phase 5), the first CTA's issuer
+ * waits stall_us (1..100000) microseconds for products that it has not issued and
+ * gives up, as after a pipeline wait that ran out.  Every CTA returns, and the call
+ * that reads the handle's error flag reports EMT6_ERR_DEVICE. */
+int emt6_test_mlp_stall(emt6_mlp *net, int phase, uint32_t stall_us);
 /* Test hook: d_c[M][N] (FP32) = d_a[M][K] d_b[N][K]^T with BF16 d_a, d_b
  * (row-major); M, N multiples of 128, K of 64.  Waits. */
 int emt6_test_mlp_gemm(const void *d_a, const void *d_b, float *d_c, int M, int N, int K,

@@ -113,3 +113,28 @@ def test_losses_of_consecutive_steps_do_not_mix():
                                             ctypes.byref(loss) if read else None))
         if read:
             assert loss.value == pytest.approx(want, rel=1e-5)
+
+
+def _stall(net, phase, us=200):
+    from emt6ro import _native as N
+    N.check(N.lib().emt6_test_mlp_stall(net._h, phase, us))
+
+
+@pytest.mark.parametrize("phase", range(6))
+@pytest.mark.parametrize("batch", [128, 1024])
+def test_a_wait_that_runs_out_in_training_is_reported(batch, phase):
+    """The first CTA's issuer gives up in each phase of the row kernel and in the
+    gradient kernel: the cluster still goes through every exchange and returns, the
+    step reports the error, and the same work on another handle is right."""
+    from emt6ro import _native as N
+    rng = np.random.default_rng(batch)
+    x = rng.normal(size=(batch, 100)).astype(np.float32)
+    t = rng.normal(size=batch).astype(np.float32)
+    net = _net(1024)
+    want, _ = net.gradients(x, t)
+    _stall(net, phase)
+    with pytest.raises(N.NativeError, match="timed out"):
+        net.train_step(x, t, 1e-3)
+    got, _ = _net(1024).gradients(x, t)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
