@@ -280,6 +280,14 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t saddr) {
 }
 constexpr uint32_t kIdescMN = kIdesc | (1u << 15) | (1u << 16);
 
+// The handle's error flag: on the device, and (host_err) where the host reads it
+// without a copy.
+__device__ __forceinline__ void raise_error(int *err, int *host_err) {
+  atomicOr(err, 1);
+  *reinterpret_cast<volatile int *>(host_err) = 1;
+  __threadfence_system();
+}
+
 // GELU and its derivative, by erff and expf: they round as the library's do, which
 // a cheaper normal tail did not, and an activation that rounds to the other of two
 // BF16 values travels through every layer above.
@@ -418,7 +426,7 @@ struct RowsArgs {
   float *dy, *loss;
   uint4 *z[3];         // pre-activations, 8 columns of a row each (z_at)
   __nv_bfloat16 *x16;  // [n][128]
-  int *err;
+  int *err, *host_err;
   // test hook (emt6_test_mlp_stall): the phase whose products the first CTA's
   // issuer gives up on after waiting stall_ns (0: none) for them to complete
   int stall_phase;
@@ -793,7 +801,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   cluster_meet();
   pdl_trigger();
   if (*abort || failed) {
-    if (lane == 0) atomicOr(a.err, 1);
+    if (lane == 0) raise_error(a.err, a.host_err);
     // loads still in flight (at most the last RING issued) land before the
     // CTA frees its shared memory
     if (tid == 0)
@@ -824,7 +832,7 @@ struct GradsArgs {
   float *clear;  // the next step's loss sum
   int B, splits;
   float lr, beta1, beta2, eps, bc1, bc2;
-  int *err;
+  int *err, *host_err;
   uint32_t stall_ns;  // test hook, as in RowsArgs: of the first CTA's products
 };
 
@@ -1020,7 +1028,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     for (int i = 0; i < 8; ++i)
       dst[(group * 8 + i) ^ (row & 31)] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
   }
-  if (failed && lane == 0) atomicOr(a.err, 1);
+  if (failed && lane == 0) raise_error(a.err, a.host_err);
   tc_fence_before();
   cluster_sync();
   const int share = BM / cluster, r0 = rank * share;  // rows this CTA finishes
@@ -1211,6 +1219,10 @@ struct emt6_mlp {
   int stall_phase = 0;     // emt6_test_mlp_stall: PHASES - 1 and below, or kStallGrads
   uint32_t stall_ns = 0;   // of the next launch concerned, 0: none
   DevArr<int> err;
+  int *host_err = nullptr, *host_err_dev = nullptr;  // pinned, written by the kernels
+  ~emt6_mlp() {
+    if (host_err) cudaFreeHost(host_err);
+  }
   CUtensorMap mX, mW[3], mWT[3];
   RowsMaps mRows;
 };
@@ -1242,11 +1254,9 @@ int check_batch(emt6_mlp *net, int B) {
 }
 
 int read_err(emt6_mlp *net) {
-  int h = 0;
-  cudaError_t e = cudaMemcpyAsync(&h, net->err.p, sizeof(int), cudaMemcpyDeviceToHost, net->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(net->stream);
+  const cudaError_t e = cudaStreamSynchronize(net->stream);
   if (e != cudaSuccess) return cuda_fail(e, "surrogate");
-  if (h) return fail("surrogate GEMM: a tensor-core pipeline wait timed out");
+  if (*static_cast<volatile int *>(net->host_err)) return fail("surrogate GEMM: a tensor-core pipeline wait timed out");
   return EMT6_OK;
 }
 
@@ -1297,6 +1307,7 @@ int run_rows(emt6_mlp *net, const float *d_x, int64_t n, const float *mean, cons
     a.w4 = net->w4.p;
     a.b4 = net->b4.p;
     a.err = net->err.p;
+    a.host_err = net->host_err_dev;
     a.stall_phase = net->stall_phase;
     a.stall_ns = take_stall(net, false);
     int grid = (a.n + BM - 1) / BM * CLUSTER;
@@ -1352,6 +1363,7 @@ int run_grads(emt6_mlp *net, int B, bool apply, float lr) {
   a.bc1 = 1.0f - std::pow(net->beta1, step);
   a.bc2 = 1.0f - std::pow(net->beta2, step);
   a.err = net->err.p;
+  a.host_err = net->host_err_dev;
   a.stall_ns = take_stall(net, true);
   // at most two parts per CTA (two accumulators, two tiles of shared memory),
   // and clusters of 4, 36 of which are resident at once
@@ -1436,7 +1448,10 @@ int emt6_mlp_create(int max_batch, uint64_t seed, int device, emt6_mlp **out) {
   ok = ok && net->w4.alloc(H) && net->m4.alloc(H) && net->v4.alloc(H) && net->b4.alloc(1) &&
        net->mb4.alloc(1) && net->vb4.alloc(1) &&
        net->X16.alloc(static_cast<size_t>(max_batch) * INP) && net->dy.alloc(max_batch) &&
-       net->loss.alloc(2) && net->err.alloc(1);
+       net->loss.alloc(2) && net->err.alloc(1) &&
+       cudaHostAlloc(&net->host_err, sizeof(int), cudaHostAllocMapped) == cudaSuccess &&
+       cudaHostGetDevicePointer(&net->host_err_dev, net->host_err, 0) == cudaSuccess;
+  if (ok) *net->host_err = 0;
   for (int l = 0; l < 3 && ok; ++l)
     ok = net->A[l].alloc(BH) && net->dZ[l].alloc(BH) && net->Z[l].alloc(BH / 8);
   for (int i = 0; i < 5 && ok; ++i) ok = net->gradv[i].alloc(i < 4 ? H : 1);

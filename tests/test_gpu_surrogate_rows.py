@@ -138,3 +138,19 @@ def test_a_wait_that_runs_out_in_training_is_reported(batch, phase):
     got, _ = _net(1024).gradients(x, t)
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,phase", [(1, 0), (200, 1), (30_000, 2)])
+def test_a_wait_that_runs_out_in_scoring_is_reported(n, phase):
+    """Predictions of a launch that gave up are not returned."""
+    from emt6ro import _native as N
+    net = _net(128)
+    x = np.random.default_rng(n).normal(size=(n, 100)).astype(np.float32)
+    want = net.predict(x)
+    _stall(net, phase)
+    with pytest.raises(N.NativeError, match="timed out"):
+        net.predict(x)
+    _stall(net, phase)
+    with pytest.raises(N.NativeError, match="timed out"):
+        net.predict_std(x)
+    assert np.array_equal(_net(128).predict(x), want)
