@@ -178,6 +178,12 @@ __device__ __forceinline__ void peer_store4(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
+__device__ __forceinline__ int peer_load4(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ float4 peer_load16(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -836,11 +842,13 @@ struct GradsArgs {
   uint32_t stall_ns;  // test hook, as in RowsArgs: of the first CTA's products
 };
 
-__device__ __forceinline__ void vec_update(const GradsArgs &a, const VecAdam &p, int idx, float g) {
+__device__ __forceinline__ void vec_update(const GradsArgs &a, const VecAdam &p, int idx, float g,
+                                           bool stale) {
   if (p.grad_out) {
     p.grad_out[idx] = g;
     return;
   }
+  if (stale) return;
   const float m = a.beta1 * p.m[idx] + (1.0f - a.beta1) * g;
   const float s = a.beta2 * p.v[idx] + (1.0f - a.beta2) * g * g;
   p.m[idx] = m;
@@ -854,7 +862,8 @@ __device__ __forceinline__ void vec_update(const GradsArgs &a, const VecAdam &p,
 // columns of it; then slots 16, 8, 4, 2 and 1 apart.  Latency bound, beside the
 // products: 32 bytes of 8 rows per load round.
 constexpr int VEC_COLS = 16, VEC_TASKS = 4 * HID / VEC_COLS, VEC_WARPS = 8;
-__device__ __forceinline__ void vec_adam(const GradsArgs &a, int task, float *part, int w, int lane) {
+__device__ __forceinline__ void vec_adam(const GradsArgs &a, int task, float *part, int w, int lane,
+                                         bool stale) {
   const int k = task / (HID / VEC_COLS), c0 = task % (HID / VEC_COLS) * VEC_COLS;
   const uint32_t *src =
       reinterpret_cast<const uint32_t *>(a.vec[k].rows + c0) + (lane & 7);
@@ -900,7 +909,7 @@ __device__ __forceinline__ void vec_adam(const GradsArgs &a, int task, float *pa
     for (int o = 4; o; o >>= 1)
 #pragma unroll
       for (int q = 0; q < o; ++q) t[q] += t[q + o];
-    vec_update(a, a.vec[k], c0 + lane, t[0]);
+    vec_update(a, a.vec[k], c0 + lane, t[0], stale);
   }
   __syncwarp();
   asm volatile("bar.sync 1, %0;" ::"n"(32 * VEC_WARPS) : "memory");  // part is free again
@@ -998,17 +1007,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     }
     umma_commit(done);  // arrives once every product above has completed
   } else if (warp >= 2) {
+    // the step's rows failed (or another CTA's products have): nothing is updated
+    const bool stale = *static_cast<const volatile int *>(a.err) != 0;
     if (blockIdx.x == 0 && tid == 64) *a.clear = 0.0f;
     if (warp < 2 + VEC_WARPS) {
       for (int task = blockIdx.x; task < VEC_TASKS; task += gridDim.x)
-        vec_adam(a, task, vec_part, warp - 2, lane);
+        vec_adam(a, task, vec_part, warp - 2, lane, stale);
     } else if (blockIdx.x == gridDim.x - 1 && warp == 2 + VEC_WARPS) {  // b4: sum dy
       float g = 0.0f;
       for (int j = lane; j < a.B; j += 32) g += a.dy[j];
 #pragma unroll
       for (int o = 16; o; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-      if (lane == 0) vec_update(a, a.vec[4], 0, g);
+      if (lane == 0) vec_update(a, a.vec[4], 0, g, stale);
     }
+    if (stale) *abort = 1;
   }
   __syncwarp();
   bool failed = !mbar_wait(done, 0, nullptr);
@@ -1016,6 +1028,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     for (int q = issued - STAGES < 0 ? 0 : issued - STAGES; q < issued; ++q)
       mbar_wait(full0 + 8 * (q % STAGES), (q / STAGES) & 1, nullptr);
   failed = failed || *abort;
+  if (failed) *abort = 1;
   tc_fence_after();
   __syncthreads();  // (after an abort: nothing lands in the ring any more)
   const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane;
@@ -1031,6 +1044,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   if (failed && lane == 0) raise_error(a.err, a.host_err);
   tc_fence_before();
   cluster_sync();
+  // a part that failed would spoil the tile: no CTA of its cluster updates it
+  int part_failed = 0;
+  if (lane < cluster) part_failed = peer_load4(peer_addr(smem_u32(const_cast<int *>(abort)), lane));
+  bool skip = false;
   const int share = BM / cluster, r0 = rank * share;  // rows this CTA finishes
   const uint32_t base = smem_u32(red);
   for (int i = tid; i < share * 32; i += GEMM_THREADS) {
@@ -1058,6 +1075,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       *reinterpret_cast<float4 *>(a.grad[l] + at_w) = g;
       continue;
     }
+    skip = __any_sync(0xffffffffu, part_failed);  // (every thread runs as many rounds)
+    if (skip) continue;
     const float gg[4] = {g.x, g.y, g.z, g.w}, mo[4] = {m4.x, m4.y, m4.z, m4.w},
                 vo[4] = {v4.x, v4.y, v4.z, v4.w}, wo[4] = {w4.x, w4.y, w4.z, w4.w};
     float mn[4], vn[4], wn[4];
@@ -1076,7 +1095,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     *reinterpret_cast<uint2 *>(a.wb[l] + at_w) = *reinterpret_cast<const uint2 *>(wb);
   }
   __syncthreads();
-  if (!a.grad[l] && a.wbt[l])
+  if (!a.grad[l] && a.wbt[l] && !skip)
     for (int i = tid; i < BN * share / 8; i += GEMM_THREADS) {
       const int c = i / (share / 8), q = i % (share / 8);
       *reinterpret_cast<uint4 *>(a.wbt[l] + static_cast<size_t>(n0 + c) * HID + m0 + r0 + 8 * q) =
@@ -1539,7 +1558,7 @@ int emt6_mlp_get_params(emt6_mlp *net, float *const *host) {
   cudaError_t e = cudaStreamSynchronize(net->stream);
   for (int i = 0; i < 8 && e == cudaSuccess; ++i)
     e = cudaMemcpy(host[i], dev[i], cnt[i] * sizeof(float), cudaMemcpyDeviceToHost);
-  return e == cudaSuccess ? EMT6_OK : cuda_fail(e, "emt6_mlp_get_params");
+  return e == cudaSuccess ? read_err(net) : cuda_fail(e, "emt6_mlp_get_params");
 }
 
 int emt6_mlp_predict(emt6_mlp *net, const float *d_x, int B, float *d_y) {

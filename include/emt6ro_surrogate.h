@@ -45,7 +45,10 @@ void emt6_mlp_destroy(emt6_mlp *net);
 /* cudaStream_t of the handle */
 void *emt6_mlp_stream(emt6_mlp *net);
 
-/* Host copies of the 8 parameter arrays (order above). */
+/* Host copies of the 8 parameter arrays (order above).  Reading them reports
+ * EMT6_ERR_DEVICE if a pipeline wait of a training step timed out: a step whose
+ * rows failed updated nothing, one whose gradients failed not the tiles of weights
+ * that the failed CTAs belonged to. */
 int emt6_mlp_set_params(emt6_mlp *net, const float *const *host);
 int emt6_mlp_get_params(emt6_mlp *net, float *const *host);
 

@@ -154,3 +154,29 @@ def test_a_wait_that_runs_out_in_scoring_is_reported(n, phase):
     with pytest.raises(N.NativeError, match="timed out"):
         net.predict_std(x)
     assert np.array_equal(_net(128).predict(x), want)
+
+
+@pytest.mark.parametrize("batch", [128, 640, 1024, 2048])
+@pytest.mark.parametrize("phase", [0, 4, 5])
+def test_a_failed_step_leaves_weights_alone(batch, phase):
+    """A step whose rows failed updates nothing; one whose first gradient CTA
+    failed (a part of W3's first tile) leaves that tile as it was.  Reading the
+    parameters of such a handle reports the error."""
+    from emt6ro import _native as N
+    rng = np.random.default_rng(batch)
+    x = rng.normal(size=(batch, 100)).astype(np.float32)
+    t = rng.normal(size=batch).astype(np.float32)
+    net = _net(2048)
+    before = net.get_params()
+    _stall(net, phase)
+    xd, td = net._to_dev(x), net._to_dev(t)
+    N.check(N.lib().emt6_mlp_train_step(net._h, xd.data_ptr(), td.data_ptr(), batch, 1e-3, None))
+    after = [np.zeros_like(p) for p in before]
+    rc = N.lib().emt6_mlp_get_params(net._h, (ctypes.c_void_p * 8)(*[a.ctypes.data for a in after]))
+    assert rc == N.EMT6_ERR_DEVICE
+    if phase == 5:
+        assert np.array_equal(after[4][:128, :128], before[4][:128, :128])
+        assert not np.array_equal(after[4], before[4])
+    else:
+        for a, b in zip(after, before):
+            assert np.array_equal(a, b)
