@@ -81,3 +81,28 @@ def test_noalloc_rejects_requests_beyond_capacity():
                torch.cuda.current_stream(dev).cuda_stream)
     assert rc == N.EMT6_ERR_LIMIT if hasattr(N, "EMT6_ERR_LIMIT") else rc == 5
     assert "at most 47 simulations" in N.lib().emt6_last_error().decode()
+
+
+@pytest.mark.parametrize("dims,radii,n", [((51, 51), (17, 22, 24), 40), ((12, 14), (2, 5, 9), 400)])
+def test_noalloc_matches_batch_with_and_without_an_sm_per_simulation(dims, radii, n):
+    import torch
+    from emt6ro import _native as N
+    from emt6ro import workloads as wl
+    from emt6ro.batch import Batch
+
+    params = wl.default_parameters()
+    params.native.lattice_height, params.native.lattice_width = dims
+    tumors = [wl.disc_tumor(params, r, seed=r) for r in radii]
+    st, sp, steps, seed = (np.arange(n) % 3).astype(np.int32), np.zeros(n, np.int32), 1300, 11
+    ref = Batch(params, tumors, [[(0, 1.0)]], st, sp, seed=seed)
+    ref.run(steps)
+    dev = torch.device("cuda:0")
+    stack = np.ascontiguousarray(np.stack([t.sites for t in tumors]))
+    tumors_dev = torch.from_numpy(stack.view(np.uint8).reshape(-1)).to(dev)
+    doses_dev = torch.from_numpy(np.ascontiguousarray(ref.doses)).to(dev)
+    counts_dev = torch.zeros(n, dtype=torch.int32, device=dev)
+    rc = _call(N, params, tumors_dev, dims[0] + 2, dims[1] + 2, torch.from_numpy(st).to(dev),
+               torch.from_numpy(sp).to(dev), n, doses_dev, ref.bins, steps, seed, counts_dev,
+               torch.cuda.current_stream(dev).cuda_stream)
+    assert rc == 0, N.lib().emt6_last_error()
+    assert (counts_dev.cpu().numpy().astype(np.uint32) == ref.counts()).all()
