@@ -11,7 +11,7 @@ namespace emt6 {
 
 // Device-resident batch, simulation-major.  Per simulation: fields
 // [3][H*W] FP32 (stride fstride floats), state bytes (sstride), cell records
-// [H*W][3] float4, occupied list (lstride u16), meta = (n, n0, multi, -),
+// [H*W][3] float4, occupied list (lstride u16), meta = (n, n0, multi, edge),
 // roi[8] = (r0, c0, h, w, dist, cells at the last reset, -, -), step counter.
 struct RunArgs {
   KParams p;
