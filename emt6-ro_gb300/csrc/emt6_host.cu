@@ -314,8 +314,15 @@ struct emt6_batch {
   DevBuf<int4> meta;
   DevBuf<int32_t> roi, sim_tumor, sim_protocol, tpl_roi;
   DevBuf<uint8_t> tier;  // per chunk: the launch tier of each simulation
-  cudaStream_t side = nullptr;  // the wide tier's, beside `stream`
-  cudaEvent_t fork = nullptr, join = nullptr;
+  // launches beside `stream`: the wide tier's, and the lone one's where it has a part
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
+  // The lone tier's part of a split launch: regions from this class on (0: none), if
+  // any were seen since the reset.  The step kernels note the classes they meet in
+  // pinned memory; what it holds by the time of a run only chooses the launches.
+  int lone_part = 0;
+  volatile uint8_t *seen = nullptr, *seen_dev = nullptr;
+  uint8_t tpl_seen[emt6::kRegionClasses] = {0, 0, 0};  // of the tumours
   DevBuf<uint32_t> step, horizon, counts, err, ticket, order_hist;
   DevBuf<int64_t> order;  // per chunk: simulations by region, largest first
   DevBuf<unsigned long long> diffused;
@@ -326,11 +333,14 @@ struct emt6_batch {
       DeviceGuard g(device);
       cudaStreamSynchronize(stream);
       if (graph_exec) cudaGraphExecDestroy(graph_exec);
-      if (side) cudaStreamSynchronize(side);
-      if (join) cudaEventDestroy(join);
-      if (side) cudaStreamDestroy(side);
+      for (int k = 0; k < 2; ++k) {
+        if (side[k]) cudaStreamSynchronize(side[k]);
+        if (join[k]) cudaEventDestroy(join[k]);
+        if (side[k]) cudaStreamDestroy(side[k]);
+      }
       if (fork) cudaEventDestroy(fork);
       cudaStreamDestroy(stream);
+      if (seen) cudaFreeHost(const_cast<uint8_t *>(seen));
     }
   }
 
@@ -359,6 +369,7 @@ struct emt6_batch {
     a.ticket = ticket.p;
     a.order = order.p;
     a.tier_of = nullptr;
+    a.seen = seen_dev;
     return a;
   }
 
@@ -405,7 +416,12 @@ struct emt6_batch {
     if (rc) return rc;
     t_host = 0;
     epoch += 1;
+    forget_seen();
     return EMT6_OK;
+  }
+
+  void forget_seen() {
+    for (int k = 0; seen && k < emt6::kRegionClasses; ++k) seen[k] = tpl_seen[k];
   }
 
   // Occupancy, kernel attributes, side streams and events of issue(): once, and
@@ -420,8 +436,29 @@ struct emt6_batch {
     // tier, in one launch.
     resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierWide]) * sms;
     lone = n <= (int64_t)emt6::max_ctas_per_sm(kp, emt6::kTierLone) * sms;
-    if (!lone && !side) EMT6_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-    if (!lone && !join) EMT6_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    // Side by side, the lone tier takes a part where the wide one is slower than it
+    // in turns of one simulation per SM.  Regions above 6 x 12 slots with two
+    // simulations per SM, or with four where the wide tier holds three: 150 steps of
+    // 304 discs of radius 26 5.6 vs 6.5 ms, 608 of radius 24 on 54 x 60 9.1 vs 11.5
+    // (three or four per SM at once: 420 of radius 24 6.6, 9.1 in turns).  Regions of
+    // the largest tile, which the wide tier spills, in any number: 608 of radius 27 on
+    // 54 x 60 11.2 vs 17.8 ms, 3,000 55.7 vs 68.4.
+    const int64_t load = (n + sms - 1) / sms;
+    lone_part = load <= 2 || (load == 4 && per_sm[emt6::kTierWide] == 3) ? emt6::kRegionLarge
+                : W > emt6::kLargestWidth ? emt6::kRegionLargest : 0;
+    if (lone) lone_part = 0;
+    if (lone_part && !seen) {
+      void *host = nullptr, *dev = nullptr;
+      EMT6_CUDA(cudaHostAlloc(&host, emt6::kRegionClasses, cudaHostAllocMapped));
+      seen = static_cast<uint8_t *>(host);
+      EMT6_CUDA(cudaHostGetDevicePointer(&dev, host, 0));
+      seen_dev = static_cast<uint8_t *>(dev);
+      forget_seen();
+    }
+    for (int k = 0; k < (lone ? 0 : lone_part ? 2 : 1); ++k) {
+      if (!side[k]) EMT6_CUDA(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
+      if (!join[k]) EMT6_CUDA(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming));
+    }
     if (!lone && !fork) EMT6_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     occ_known = true;
     return EMT6_OK;
@@ -433,6 +470,9 @@ struct emt6_batch {
       grid = (int)std::min<int64_t>(n, (int64_t)per_sm[tier] * sms);
       a.queue = 1;
       a.ticket = ticket.p + (a.tier_of ? tier : emt6::kTiers);
+    } else if (tier == emt6::kTierLone && a.order) {
+      // its simulations are the first of the order; the others cost no CTA each
+      grid = (int)std::min<int64_t>(n, (int64_t)per_sm[tier] * sms);
     }
     EMT6_CUDA(emt6::launch_run(a, end, tier, grid, st));
     *count += 1;
@@ -446,7 +486,9 @@ struct emt6_batch {
     while (t < target) {
       const uint32_t end = (uint32_t)std::min<uint64_t>(target, (uint64_t)t + chunk);
       if (has_horizon && t >= max_horizon) break;
-      if (lone || (resident && end - t < kSplitSteps)) {
+      const bool brief = resident && end - t < kSplitSteps;
+      const int part = lone_part && (seen[emt6::kRegionLargest] || seen[lone_part]) ? lone_part : 0;
+      if (lone || (brief && !part)) {
         a.order = nullptr;
         const int rc = launch(a, end, lone ? emt6::kTierLone : emt6::kTierWide, stream, count);
         if (rc) return rc;
@@ -457,10 +499,10 @@ struct emt6_batch {
         // is finished by the last launch.
         if (resident) {
           a.order = nullptr;
-          EMT6_CUDA(emt6::launch_tiers(a, tier.p, stream));
+          EMT6_CUDA(emt6::launch_tiers(a, tier.p, part, !brief, stream));
           *count += 1;
         } else {
-          EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, tier.p, stream));
+          EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, tier.p, part, stream));
           *count += 3;
           if (sched == 1)
             EMT6_CUDA(cudaMemsetAsync(ticket.p, 0, (emt6::kTiers + 1) * sizeof(uint32_t), stream));
@@ -468,14 +510,19 @@ struct emt6_batch {
         EMT6_CUDA(cudaEventRecord(fork, stream));
         emt6::RunArgs b = a;
         b.tier_of = tier.p;
-        EMT6_CUDA(cudaStreamWaitEvent(side, fork, 0));
-        int rc = launch(b, end, emt6::kTierWide, side, count);
+        int rc = EMT6_OK, beside = 0;  // launches on the side streams
+        for (int tr : {emt6::kTierLone, emt6::kTierWide}) {
+          if (tr == emt6::kTierLone ? !part : brief) continue;
+          EMT6_CUDA(cudaStreamWaitEvent(side[beside], fork, 0));
+          rc = launch(b, end, tr, side[beside], count);
+          if (rc) return rc;
+          EMT6_CUDA(cudaEventRecord(join[beside], side[beside]));
+          ++beside;
+        }
+        rc = launch(b, end, brief ? emt6::kTierWide : emt6::kTierNarrow, stream, count);
         if (rc) return rc;
-        EMT6_CUDA(cudaEventRecord(join, side));
-        rc = launch(b, end, emt6::kTierNarrow, stream, count);
-        if (rc) return rc;
-        EMT6_CUDA(cudaStreamWaitEvent(stream, join, 0));
-        rc = launch(a, end, emt6::kTierWide, stream, count);
+        while (beside) EMT6_CUDA(cudaStreamWaitEvent(stream, join[--beside], 0));
+        if (!brief) rc = launch(a, end, emt6::kTierWide, stream, count);
         if (rc) return rc;
       }
       t = end;
@@ -902,7 +949,11 @@ int emt6_batch_create(const emt6_params *p, const emt6_site *tumors, int32_t n_t
       }
     std::vector<int32_t> hr((size_t)n_tumors * 8, 0);
     for (int32_t t = 0; t < n_tumors; ++t)
-      template_roi(&hs[(size_t)t * b->sstride], height, width, &hr[(size_t)t * 8]);
+    {
+      int32_t *roi = &hr[(size_t)t * 8];
+      template_roi(&hs[(size_t)t * b->sstride], height, width, roi);
+      b->tpl_seen[emt6::region_class(roi, height, width)] = 1;
+    }
     EMT6_CUDA(b->tpl_roi.alloc(hr.size()));
     EMT6_CUDA(cudaMemcpy(b->tpl_roi.p, hr.data(), hr.size() * 4, cudaMemcpyHostToDevice));
     EMT6_CUDA(cudaMemcpy(b->tpl_fld.p, hf.data(), hf.size() * 4, cudaMemcpyHostToDevice));
@@ -1445,7 +1496,7 @@ int emt6_test_order(const int32_t *roi, const uint32_t *step, const uint32_t *ho
   a.step = st.p;
   a.horizon = horizon ? hz.p : nullptr;
   a.nsims = nsims;
-  EMT6_CUDA(emt6::launch_order(a, t_end, hist.p, out.p, nullptr, 0));
+  EMT6_CUDA(emt6::launch_order(a, t_end, hist.p, out.p, nullptr, 0, 0));
   EMT6_CUDA(cudaMemcpy(order, out.p, nsims * sizeof(int64_t), cudaMemcpyDeviceToHost));
   return EMT6_OK;
 }

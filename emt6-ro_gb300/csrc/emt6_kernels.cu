@@ -475,6 +475,25 @@ __device__ __forceinline__ void diffuse_by_parts(float *fld, int plane, const ui
     diffuse_parts<14>(f, colmask, slots, part, 1 + field, r0, c0, h, w, p.W, ext, ca, cb, cd, p.nfree);
 }
 
+// The class (kRegion*) of a region: what tile_mapping's tiles hold of it.  "Large"
+// starts where the lone tier is faster for short runs, too (10 steps of 304 discs of
+// distance 23, which 6 x 12 slots hold: 0.42 ms there, 0.39 on the wide tier; of
+// distance 24 0.38 and 0.41).
+__host__ __device__ inline int class_of(int h, int w, int d, int H, int W) {
+  constexpr TileShape below = tile_shape(kPartTiles), largest = tile_shape(kNumTiles - 2);
+  static_assert(!below.RE && !below.CE && largest.RE && !largest.CE && 4 * largest.R >= 56 &&
+                    8 * largest.C - 1 == kLargestWidth,
+                "what the tiles hold");
+  const bool block = h == 2 * d + 1 && w == h;
+  const bool next = block && h + 2 <= H - 2 && w + 2 <= W - 2;  // a block one site larger, too
+  const int nr = block ? 2 * d : h + 2, nc = block ? 2 * d : w + 2;
+  const int grown = next ? w + 1 : (w + 2 < W - 2 ? w + 2 : W - 2) + 2;
+  if (h > 0 && (nc > kLargestWidth || grown > kLargestWidth)) return kRegionLargest;
+  return nr > 4 * below.R - 1 || nc > 8 * below.C - 1 ? kRegionLarge : kRegionSmall;
+}
+
+int region_class(const int32_t roi[5], int H, int W) { return class_of(roi[2], roi[3], roi[4], H, W); }
+
 // Field window (rows w0 .. w0 + rows - 1 of the three planes) from and to
 // global memory.  The whole lattice is one contiguous copy of 16-byte words
 // (strides are padded); a window's rows start at any 4-byte word.
@@ -1157,6 +1176,10 @@ __global__ void __launch_bounds__(threads_of(TIER), TIER == kTierLone ? 1 : TIER
       a.meta[sim] = make_int4((int)m->n, (int)m->n0, m->has_multi, m->edge);
       for (int k2 = 0; k2 < 5; ++k2) a.roi[sim * 8 + k2] = m->roi[k2];
       a.step[sim] = t;
+      if (WIDE && a.seen) {
+        const int c = class_of(m->roi[2], m->roi[3], m->roi[4], H, W);
+        if (c != kRegionSmall) a.seen[c] = 1;
+      }
       if (m->ins[0]) atomicAdd(&g_instr_counts[0], (unsigned long long)m->ins[0]);
       if (m->ins[1]) atomicAdd(&g_instr_counts[1], (unsigned long long)m->ins[1]);
       if (m->ins[2]) atomicAdd(&g_instr_counts[2], (unsigned long long)m->ins[2]);
@@ -1221,27 +1244,31 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t *hist) {
 // (or, after a reset, its tumour's): a wrong guess only costs time, the launch
 // after the concurrent ones takes what they leave.  A region at the narrow
 // tiles' limit is given to the wide tier, which runs it nearly as fast: it may
-// grow in the next steps, and what is left for the last launch runs alone.
-__device__ __forceinline__ uint8_t expected_tier(const RunArgs &a, int64_t sim) {
+// grow in the next steps, and what is left for the last launch runs alone.  Regions
+// from class `lone` on (unless 0) go to the lone tier.
+__device__ __forceinline__ uint8_t expected_tier(const RunArgs &a, int64_t sim, int lone,
+                                                  bool narrow) {
   const int *roi = a.roi + sim * 8;
   const int h = roi[2], w = roi[3], d = roi[4], n = max(a.meta[sim].x, roi[5]) + 64;
-  const bool narrow = (h == 2 * d + 1 && w == h) ? d <= 15 : h + 2 <= 30 && w + 2 <= 30;
-  if (narrow && n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierNarrow).entries) return kTierNarrow;
+  const bool small = (h == 2 * d + 1 && w == h) ? d <= 15 : h + 2 <= 30 && w + 2 <= 30;
+  if (lone && class_of(h, w, d, a.p.H, a.p.W) >= lone) return kTierLone;
+  if (narrow && small && n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierNarrow).entries)
+    return kTierNarrow;
   return kTierWide;
 }
 
 __global__ void order_scatter_kernel(const RunArgs a, uint32_t t_end, uint32_t *hist,
-                                     int64_t *out, uint8_t *tier) {
+                                     int64_t *out, uint8_t *tier, int lone) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.nsims;
        i += (int64_t)gridDim.x * blockDim.x) {
     out[atomicAdd(&hist[order_key(a, i, t_end)], 1u)] = i;
-    if (tier) tier[i] = expected_tier(a, i);
+    if (tier) tier[i] = expected_tier(a, i, lone, true);
   }
 }
 
-__global__ void tier_kernel(const RunArgs a, uint8_t *tier) {
+__global__ void tier_kernel(const RunArgs a, uint8_t *tier, int lone, bool narrow) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < a.nsims) tier[i] = expected_tier(a, i);
+  if (i < a.nsims) tier[i] = expected_tier(a, i, lone, narrow);
 }
 
 // ---------------------------------------------------------------------------
@@ -1454,7 +1481,7 @@ cudaError_t launch_run(const RunArgs &a, uint32_t t_end, int tier, int grid, cud
 }
 
 cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64_t *out,
-                         uint8_t *tier, cudaStream_t stream) {
+                         uint8_t *tier, int lone, cudaStream_t stream) {
   if (a.nsims < 1) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(hist, 0, kOrderKeys * sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
@@ -1462,12 +1489,13 @@ cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64
   const int grid = (int)(blocks < 4096 ? blocks : 4096);
   order_count_kernel<<<grid, 256, 0, stream>>>(a, t_end, hist);
   order_scan_kernel<<<1, 1024, 0, stream>>>(hist);
-  order_scatter_kernel<<<grid, 256, 0, stream>>>(a, t_end, hist, out, tier);
+  order_scatter_kernel<<<grid, 256, 0, stream>>>(a, t_end, hist, out, tier, lone);
   return cudaGetLastError();
 }
 
-cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, cudaStream_t stream) {
-  tier_kernel<<<(unsigned)((a.nsims + 127) / 128), 128, 0, stream>>>(a, tier);
+cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, int lone, bool narrow,
+                         cudaStream_t stream) {
+  tier_kernel<<<(unsigned)((a.nsims + 127) / 128), 128, 0, stream>>>(a, tier, lone, narrow);
   return cudaGetLastError();
 }
 

@@ -34,6 +34,7 @@ struct RunArgs {
   uint32_t *ticket;
   const int64_t *order;  // simulation of each CTA or ticket (null: the identity)
   const uint8_t *tier_of;  // tier of each simulation (null: this launch takes any)
+  volatile uint8_t *seen;  // [kRegionClasses] classes met at a launch's end (or null)
 };
 
 struct ResetArgs {
@@ -57,7 +58,13 @@ struct ResetArgs {
 // takes the simulations that the narrow one left short of the target step
 // (regions too wide or lists too long for the shared memory that lets 5 CTAs
 // share an SM); it holds any.
-enum { kTierNarrow = 0, kTierWide = 1, kTiers = 2, kTierLone = 2 };
+enum { kTierNarrow = 0, kTierWide = 1, kTierLone = 2, kTiers = 3 };
+// Classes of regions, by the wide tier's tile: up to 6 x 12 slots per lane, above,
+// and those that only the largest tile holds (or will, one site larger).  A launch of
+// several tiers side by side may give the lone one the regions from a class on.
+enum { kRegionSmall = 0, kRegionLarge = 1, kRegionLargest = 2, kRegionClasses = 3 };
+constexpr int kLargestWidth = 55;  // wider whole regions need the largest tile
+int region_class(const int32_t roi[5], int H, int W);
 size_t run_kernel_smem(int H, int W, int lcap, int tier);
 int max_ctas_per_sm(const KParams &p, int tier);
 // Advance the simulations that `tier` holds to step min(t_end, horizon).
@@ -65,12 +72,13 @@ cudaError_t launch_run(const RunArgs &a, uint32_t t_end, int tier, int grid, cud
 cudaError_t launch_reset(const ResetArgs &a, cudaStream_t stream);
 // simulations sorted largest region first into out[0 .. a.nsims) for the
 // launches of a chunk ending at t_end, and (unless null) the tier expected to
-// hold each; hist holds kOrderKeys counters
+// hold each, the lone one for regions from class `lone` on (0: none); hist holds
+// kOrderKeys counters
 constexpr uint32_t kOrderKeys = 4096;
 cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64_t *out,
-                         uint8_t *tier, cudaStream_t stream);
-// the tiers alone, for a batch that needs no order
-cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, cudaStream_t stream);
+                         uint8_t *tier, int lone, cudaStream_t stream);
+// the tiers alone, for a batch that needs no order, without the narrow one if asked
+cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, int lone, bool narrow, cudaStream_t stream);
 cudaError_t instr_read(unsigned long long counts[4], double *sum_dp, unsigned long long *hist);
 cudaError_t instr_reset();
 cudaError_t fp32_peak(int device, double *tflops);

@@ -258,6 +258,7 @@ int emt6_simulate_noalloc(const emt6_params *p, const emt6_site *d_tumors, int32
   a.ticket = ticket;
   a.order = nullptr;
   a.tier_of = nullptr;
+  a.seen = nullptr;
 
   // the header (error flag, ticket, counter) must start at zero
   e = cudaMemsetAsync(base + o_err, 0, 256, s);

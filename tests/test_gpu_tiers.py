@@ -155,3 +155,41 @@ def test_cells_on_a_vacant_far_border_count_for_the_region(n, params, oracle):
     assert (b.counts()[:k] == ob.counts()).all()
     for j in range(k):
         assert b.state(j).sites.tobytes() == ob.get(j).tobytes(), j
+
+
+@pytest.mark.parametrize("dims,radii,n,schedule,launches", [
+    ((51, 51), (5, 24, 26, 36), 200, 0, (5, 3)),   # two simulations per SM
+    ((51, 51), (5, 12, 17, 20), 200, 2, (4, 1)),   # no large region
+    ((51, 51), (5, 24, 26, 36), 400, 0, (4, 1)),   # more per SM
+    ((51, 51), (5, 24, 26, 36), 700, 1, (6, 6)),
+    ((54, 60), (6, 26, 27, 40), 200, 3, (5, 3)),
+    ((54, 60), (6, 26, 27, 40), 400, 0, (5, 3)),   # the largest tile alone
+    ((54, 60), (6, 24, 27, 40), 500, 2, (7, 7)),   # four per SM
+    ((54, 60), (6, 26, 27, 40), 700, 0, (7, 7)),
+    ((54, 60), (6, 26, 27, 40), 700, 1, (7, 7)),
+    ((54, 60), (6, 26, 27, 40), 700, 3, (7, 7)),
+    ((54, 60), (6, 20, 23, 25), 700, 0, (6, 6))])  # no region of the largest tile
+def test_large_regions_in_turns_beside_the_other_tiers(dims, radii, n, schedule, launches, oracle):
+    """The lone tier's part of a split launch: launches of a long and a short run,
+    and the oracle's lattices."""
+    from emt6ro import workloads as wl
+    from emt6ro.batch import Batch
+    params = wl.default_parameters()
+    params.native.lattice_height, params.native.lattice_width = dims
+    tumors = [wl.disc_tumor(params, r, seed=80 + r) for r in radii]
+    st, k = np.arange(n) % 4, 8
+    b = Batch(params, tumors, [[(0, 0.5)]], st, np.zeros(n, np.int32), seed=13)
+    b.set_schedule(schedule, 0)
+    before, count = b.launches(), []
+    for steps in (70, 20):
+        b.run(steps)
+        count.append(b.launches() - before)
+        before = b.launches()
+    ob = oracle.Batch(oracle.params_copy(params.native), k, 13)
+    for j in range(k):
+        ob.set(j, tumors[st[j]].sites, b.doses[0], resolution=300, length=144_000)
+    ob.run(90, nthreads=8)
+    assert (b.counts()[:k] == ob.counts()).all()
+    for j in range(k):
+        assert b.state(j).sites.tobytes() == ob.get(j).tobytes(), j
+    assert tuple(count) == launches
