@@ -301,6 +301,7 @@ struct emt6_batch {
   bool use_graph = false;
   bool occ_known = false;
   bool resident = false, lone = false;
+  int route = 0;  // emt6_test_batch_route
   int sms = 0, per_sm[emt6::kTiers] = {1, 1};
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_key[5] = {0, 0, 0, 0, 0};
@@ -446,6 +447,11 @@ struct emt6_batch {
     const int64_t load = (n + sms - 1) / sms;
     lone_part = load <= 2 || (load == 4 && per_sm[emt6::kTierWide] == 3) ? emt6::kRegionLarge
                 : W > emt6::kLargestWidth ? emt6::kRegionLargest : 0;
+    if (route) {
+      lone = route == 1;
+      resident = route < 4;
+      lone_part = route == 5 ? emt6::kRegionLarge : 0;
+    }
     if (lone) lone_part = 0;
     if (lone_part && !seen) {
       void *host = nullptr, *dev = nullptr;
@@ -486,7 +492,7 @@ struct emt6_batch {
     while (t < target) {
       const uint32_t end = (uint32_t)std::min<uint64_t>(target, (uint64_t)t + chunk);
       if (has_horizon && t >= max_horizon) break;
-      const bool brief = resident && end - t < kSplitSteps;
+      const bool brief = resident && (route ? route == 2 : end - t < kSplitSteps);
       const int part = lone_part && (seen[emt6::kRegionLargest] || seen[lone_part]) ? lone_part : 0;
       if (lone || (brief && !part)) {
         a.order = nullptr;
@@ -1130,6 +1136,14 @@ int emt6_batch_set_schedule(emt6_batch *b, int32_t mode, uint32_t steps_per_laun
   b->sched = mode & 1;
   b->use_graph = (mode & 2) != 0;
   if (steps_per_launch) b->chunk = steps_per_launch;
+  return EMT6_OK;
+}
+
+int emt6_test_batch_route(emt6_batch *b, int32_t route) {
+  if (!b || route < 0 || route > 5) return fail(EMT6_ERR_INVALID, "null handle or unknown route");
+  std::lock_guard<std::mutex> lk(b->mu);
+  if (b->occ_known) return fail(EMT6_ERR_INVALID, "the route is chosen before the first run");
+  b->route = route;
   return EMT6_OK;
 }
 

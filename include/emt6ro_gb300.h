@@ -208,6 +208,11 @@ int emt6_test_list(const uint8_t *state, int32_t height, int32_t width, uint16_t
 /* variant 0: the narrow kernel's path (regions up to 32 x 31), 1: the wide one */
 int emt6_test_diffuse(const emt6_params *p, float *fields, int32_t height, int32_t width,
                       const int32_t *roi, int32_t variant, int32_t device);
+/* Route of the batch's runs, whatever its size (before the first run; results do not
+ * depend on it): 0 as its size and regions say, 1 the lone tier alone, 2 the wide tier
+ * alone, 3 the narrow and wide tiers side by side, 4 the same over the launch order
+ * (and the work queue, if scheduled), 5 with large regions on the lone tier, too. */
+int emt6_test_batch_route(emt6_batch *b, int32_t route);
 /* The launch order of a chunk ending at t_end for nsims simulations with
  * stored ROIs roi[8 i .. 8 i + 4] (r0, c0, h, w, dist), current steps and
  * optional horizons: order[] receives the simulation indices, largest region
