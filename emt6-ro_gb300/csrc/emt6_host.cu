@@ -1147,6 +1147,16 @@ int emt6_test_batch_route(emt6_batch *b, int32_t route) {
   return EMT6_OK;
 }
 
+int emt6_test_batch_tiers(emt6_batch *b, uint8_t *out) {
+  if (!b || !out) return fail(EMT6_ERR_INVALID, "null argument");
+  std::lock_guard<std::mutex> lk(b->mu);
+  DeviceGuard g(b->device);
+  EMT6_CUDA(emt6::launch_tiers(b->run_args(), b->tier.p, 0, true, b->stream));
+  EMT6_CUDA(cudaMemcpyAsync(out, b->tier.p, (size_t)b->n, cudaMemcpyDeviceToHost, b->stream));
+  EMT6_CUDA(cudaStreamSynchronize(b->stream));
+  return EMT6_OK;
+}
+
 int emt6_batch_set_layouts(emt6_batch *b, uint32_t layouts) {
   if (!b) return fail(EMT6_ERR_INVALID, "null handle");
   if (layouts & ~kLayoutAll) return fail(EMT6_ERR_INVALID, "unknown layout bits");

@@ -1241,7 +1241,7 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t *hist) {
 }
 
 // The tier expected to hold a simulation, from its stored region and list
-// (or, after a reset, its tumour's): a wrong guess only costs time, the launch
+// (or, until its first step, its tumour's cells): a wrong guess only costs time, the launch
 // after the concurrent ones takes what they leave.  A region at the narrow
 // tiles' limit is given to the wide tier, which runs it nearly as fast: it may
 // grow in the next steps, and what is left for the last launch runs alone.  Regions
@@ -1249,7 +1249,8 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t *hist) {
 __device__ __forceinline__ uint8_t expected_tier(const RunArgs &a, int64_t sim, int lone,
                                                   bool narrow) {
   const int *roi = a.roi + sim * 8;
-  const int h = roi[2], w = roi[3], d = roi[4], n = max(a.meta[sim].x, roi[5]) + 64;
+  const int h = roi[2], w = roi[3], d = roi[4];
+  const int n = (a.step[sim] == 0 ? roi[5] : a.meta[sim].x) + 64;
   const bool small = (h == 2 * d + 1 && w == h) ? d <= 15 : h + 2 <= 30 && w + 2 <= 30;
   if (lone && class_of(h, w, d, a.p.H, a.p.W) >= lone) return kTierLone;
   if (narrow && small && n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierNarrow).entries)

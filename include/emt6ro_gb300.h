@@ -213,6 +213,8 @@ int emt6_test_diffuse(const emt6_params *p, float *fields, int32_t height, int32
  * alone, 3 the narrow and wide tiers side by side, 4 the same over the launch order
  * (and the work queue, if scheduled), 5 with large regions on the lone tier, too. */
 int emt6_test_batch_route(emt6_batch *b, int32_t route);
+/* The tier that a run would expect to hold each simulation now: 0 narrow, 1 wide. */
+int emt6_test_batch_tiers(emt6_batch *b, uint8_t *out);
 /* The launch order of a chunk ending at t_end for nsims simulations with
  * stored ROIs roi[8 i .. 8 i + 4] (r0, c0, h, w, dist), current steps and
  * optional horizons: order[] receives the simulation indices, largest region

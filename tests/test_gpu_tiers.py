@@ -193,3 +193,28 @@ def test_large_regions_in_turns_beside_the_other_tiers(dims, radii, n, schedule,
     for j in range(k):
         assert b.state(j).sites.tobytes() == ob.get(j).tobytes(), j
     assert tuple(count) == launches
+
+
+def test_a_tumour_that_shrank_is_expected_on_the_narrow_tier(params):
+    """A disc too large for the narrow tier whose outer cells die of age: from then
+    on, its own list and region decide, not the initial tumour's cells."""
+    from emt6ro import _native as N
+    from emt6ro import workloads as wl
+    from emt6ro.batch import Batch
+    big, small = (wl.disc_tumor(params, r, seed=5) for r in (23, 6))
+    s = big.sites
+    rr, cc = np.mgrid[0:53, 0:53]
+    outer = (s["state"] == 1) & ((rr - 26) ** 2 + (cc - 26) ** 2 > 36)
+    s["proliferation_time"][outer] = s["cycle_times"][outer][:, 4] + 1
+    n = 300
+    b = Batch(params, [big, small], [[]], np.arange(n) % 2, np.zeros(n, np.int32), seed=2)
+
+    def tiers():
+        out = np.zeros(n, np.uint8)
+        N.check(N.lib().emt6_test_batch_tiers(b._h, N.ptr(out)))
+        return out[:2].tolist()
+    assert tiers() == [1, 0]
+    b.run(200)
+    assert tiers() == [0, 0]
+    b.reset()
+    assert tiers() == [1, 0]
