@@ -187,10 +187,15 @@ class Surrogate:
         n = len(x)
         if n == 0:
             return np.zeros(0, np.float32)
-        if x.size == n * N_FEATURES:
+        # more dimensions only where the rows are whole tiles, taken as they lie
+        if x.ndim > 2 and n % 128 == 0 and x.size == n * N_FEATURES:
             x = x.reshape(n, N_FEATURES)
-        else:
-            x = np.ascontiguousarray(np.broadcast_to(x, (n, N_FEATURES)))
+        if x.shape != (n, N_FEATURES):
+            try:
+                x = np.ascontiguousarray(np.broadcast_to(x, (n, N_FEATURES)))
+            except ValueError:
+                raise RuntimeError(f"rows of {N_FEATURES} features expected, got an array of "
+                                   f"shape {x.shape}") from None
         return self._predict_rows(x)
 
     # ---- training / inference in living cells -------------------------------

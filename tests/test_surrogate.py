@@ -70,3 +70,24 @@ def test_features(params):
     assert f[0] == 317 and f[1] == pytest.approx(10.0, abs=0.5) and 0 < f[2] < 1
     x = s.features([[(0, 2.0)], []], [wl.disc_tumor(params, 5, seed=1)], [0, 1], [0, 0])
     assert x.shape == (2, 100) and x[0, 0] == 2.0 and x[1, :96].sum() == 0
+
+
+@pytest.mark.parametrize("shape,taken", [
+    ((5, 100), True), ((5, 1), True), ((100,), True), ((256, 10, 10), True), ((0, 100), True),
+    ((5, 10, 10), False), ((5, 1, 100), False), ((1, 1, 100), False), ((1, 10, 10), False),
+    ((5, 64), False), ((7,), False), ((128, 64), False), ((128, 1, 64), False)])
+def test_shapes_that_scoring_takes(shape, taken):
+    """predict_std takes what broadcasts to rows of 100 features, and refuses the rest."""
+    from emt6ro.surrogate import Surrogate
+    net = Surrogate.__new__(Surrogate)
+    net._predict_rows = lambda rows: rows
+    x = np.arange(np.prod(shape), dtype=np.float32).reshape(shape)
+    if not taken:
+        with pytest.raises(RuntimeError, match="features"):
+            net.predict_std(x)
+    elif x.size:
+        got = net.predict_std(x)
+        want = x.reshape(len(x), 100) if x.size == 100 * len(x) else np.broadcast_to(x, (len(x), 100))
+        assert got.shape == (len(x), 100) and got.flags.c_contiguous and np.array_equal(got, want)
+    else:
+        assert net.predict_std(x).shape == (0,)
