@@ -180,3 +180,25 @@ def test_a_failed_step_leaves_weights_alone(batch, phase):
     else:
         for a, b in zip(after, before):
             assert np.array_equal(a, b)
+
+
+def test_each_step_reports_its_own_batchs_loss():
+    """Batches of different losses in turn, some steps' losses unread: what is read
+    is the loss of that step's batch, not of the one before or of a sum."""
+    from emt6ro import _native as N
+    net = _net(128)
+    rng = np.random.default_rng(5)
+    x = rng.normal(size=(128, 100)).astype(np.float32)
+    batches, want = [], []
+    for k in range(3):
+        t = ((k + 1) ** 2 * rng.normal(size=128)).astype(np.float32)
+        want.append(_net(128).train_step(x, t, 0.0))
+        batches.append((net._to_dev(x), net._to_dev(t)))
+    assert want[0] < 0.5 * want[1] < 0.25 * want[2]
+    loss = ctypes.c_float()
+    for k, read in zip([0, 1, 2, 0, 2, 1, 1, 0, 2, 2, 0], [1, 1, 0, 1, 1, 0, 1, 0, 0, 1, 1]):
+        xd, td = batches[k]
+        N.check(N.lib().emt6_mlp_train_step(net._h, xd.data_ptr(), td.data_ptr(), 128, 0.0,
+                                            ctypes.byref(loss) if read else None))
+        if read:
+            assert loss.value == pytest.approx(want[k], rel=1e-5)
