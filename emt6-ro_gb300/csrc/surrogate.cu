@@ -1272,11 +1272,15 @@ int check_batch(emt6_mlp *net, int B) {
   return EMT6_OK;
 }
 
+int status(const emt6_mlp *net) {
+  if (*static_cast<const volatile int *>(net->host_err))
+    return fail("surrogate GEMM: a tensor-core pipeline wait timed out");
+  return EMT6_OK;
+}
+
 int read_err(emt6_mlp *net) {
   const cudaError_t e = cudaStreamSynchronize(net->stream);
-  if (e != cudaSuccess) return cuda_fail(e, "surrogate");
-  if (*static_cast<volatile int *>(net->host_err)) return fail("surrogate GEMM: a tensor-core pipeline wait timed out");
-  return EMT6_OK;
+  return e == cudaSuccess ? status(net) : cuda_fail(e, "surrogate");
 }
 
 // every map covers a whole allocation: batches use its first rows or columns
@@ -1621,6 +1625,10 @@ int emt6_mlp_set_splitk(emt6_mlp *net, int splits) {
                 EMT6_ERR_INVALID);
   net->split_override = splits;
   return EMT6_OK;
+}
+
+int emt6_mlp_status(const emt6_mlp *net) {
+  return net ? status(net) : fail("emt6_mlp_status: null", EMT6_ERR_INVALID);
 }
 
 int emt6_mlp_sync(emt6_mlp *net) {

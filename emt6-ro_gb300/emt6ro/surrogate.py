@@ -178,7 +178,8 @@ class Surrogate:
                 N.check(N.lib().emt6_mlp_predict_rows(self._h, xd.data_ptr(), n, N.ptr(mean),
                                                       N.ptr(std), yd.data_ptr()))
                 torch.from_numpy(out[i:i + n]).copy_(yd)
-        N.check(N.lib().emt6_mlp_sync(self._h))  # no values of a launch that gave up
+        # the copies have waited: no values of a launch that gave up
+        N.check(N.lib().emt6_mlp_status(self._h))
         return out
 
     def predict_std(self, x_std) -> np.ndarray:

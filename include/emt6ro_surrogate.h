@@ -52,8 +52,8 @@ void *emt6_mlp_stream(emt6_mlp *net);
 int emt6_mlp_set_params(emt6_mlp *net, const float *const *host);
 int emt6_mlp_get_params(emt6_mlp *net, float *const *host);
 
-/* d_y[B] = network(d_x[B][100]); asynchronous: emt6_mlp_sync says whether the
- * values are good. */
+/* d_y[B] = network(d_x[B][100]); asynchronous: emt6_mlp_sync, or after a
+ * wait emt6_mlp_status, says whether the values are good. */
 int emt6_mlp_predict(emt6_mlp *net, const float *d_x, int B, float *d_y);
 
 /* d_y[n] = network(rows of d_x[n][100]) for any number of rows, in one launch;
@@ -81,6 +81,8 @@ int emt6_mlp_set_splitk(emt6_mlp *net, int splits);
 /* Waits for the handle's stream; EMT6_ERR_DEVICE if a pipeline wait of the
  * handle's kernels timed out at any time. */
 int emt6_mlp_sync(emt6_mlp *net);
+/* The same of the launches that have completed, without waiting. */
+int emt6_mlp_status(const emt6_mlp *net);
 
 /* Failure-path hook (no reference counterpart): in the handle's next launch of the
  * row kernel (phase 0..2: the hidden layers, 3..4: the error back through layers 3
