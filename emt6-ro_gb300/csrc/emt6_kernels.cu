@@ -241,42 +241,23 @@ __device__ __forceinline__ void build_colmask(uint64_t *colmask, int h, int w, i
 // product's error s (inv W - 2^20) / (2^20 W) stays below 1 / W)
 __device__ __forceinline__ int row_of(int s, uint32_t inv) { return (int)((uint32_t)s * inv >> 20); }
 
-// Cells that divided onto a vacant border site of the last row or column (m->edge):
-// the list leaves them out at its next rebuild (simulation.cu:50-53), the region does
-// not.  Their extent, and their largest squared distance from (mr, mc).
-__device__ __noinline__ int4 edge_extent(const uint8_t *st, int H, int W) {
-  int4 v = make_int4(H, W, 0, 0);
-  for (int q = threadIdx.x; q < W + H - 1; q += blockDim.x) {
-    const int r = q < W ? H - 1 : q - W, c = q < W ? q : W - 1;
-    if ((st[r * W + c] & kStMask) == kOccupied)
-      v = make_int4(min(v.x, r), min(v.y, c), max(v.z, r), max(v.w, c));
-  }
-  return v;
-}
-__device__ __noinline__ int edge_far(const uint8_t *st, int H, int W, int mr, int mc) {
-  int far = 0;
-  for (int q = threadIdx.x; q < W + H - 1; q += blockDim.x) {
-    const int r = q < W ? H - 1 : q - W, c = q < W ? q : W - 1;
-    if ((st[r * W + c] & kStMask) == kOccupied)
-      far = max(far, (mr - r) * (mr - r) + (mc - c) * (mc - c));
-  }
-  return far;
-}
-
-// The occupied sites are all in the list (rebuilt, then appended to) but those.
+// The occupied sites are all in the list (rebuilt, then appended to), but for cells
+// that divided onto a vacant border site of the last row or column (m->edge): the
+// list leaves them out at its next rebuild (simulation.cu:50-53), the region does not.
 template <int NT>
 __device__ __noinline__ void compute_roi(const uint8_t *st, const uint16_t *list, uint64_t *colmask, Misc *m,
                             int H, int W) {
   constexpr int NWARP = NT / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint32_t n = m->n, inv = ((1u << 20) + W - 1) / W;
+  const uint32_t n = m->n, all = n + (m->edge ? H + W - 1 : 0), inv = ((1u << 20) + W - 1) / W;
+  const auto site = [&](uint32_t e) -> int {  // of the list, the last row, the last column
+    if (e < n) return list[e] & kSiteMask;
+    const int q = (int)(e - n);
+    return q < W ? (H - 1) * W + q : (q - W) * W + W - 1;
+  };
   int v[4] = {H, W, 0, 0};
-  if (m->edge) {
-    const int4 x = edge_extent(st, H, W);
-    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-  }
-  for (uint32_t e = threadIdx.x; e < n; e += NT) {
-    const int s = list[e] & kSiteMask;
+  for (uint32_t e = threadIdx.x; e < all; e += NT) {
+    const int s = site(e);
     if ((st[s] & kStMask) == kOccupied) {
       const int r = row_of(s, inv), c = s - r * W;
       v[0] = min(v[0], r); v[1] = min(v[1], c);
@@ -307,14 +288,13 @@ __device__ __noinline__ void compute_roi(const uint8_t *st, const uint16_t *list
   const int midr = v[0] + (v[2] - v[0] + 1) / 2;
   const int midc = v[1] + (v[3] - v[1] + 1) / 2;
   int far = 0;  // largest squared distance
-  for (uint32_t e = threadIdx.x; e < n; e += NT) {
-    const int s = list[e] & kSiteMask;
+  for (uint32_t e = threadIdx.x; e < all; e += NT) {
+    const int s = site(e);
     if ((st[s] & kStMask) == kOccupied) {
       const int r = row_of(s, inv), c = s - r * W;
       far = max(far, (midr - r) * (midr - r) + (midc - c) * (midc - c));
     }
   }
-  if (m->edge) far = max(far, edge_far(st, H, W, midr, midc));
   far = __reduce_max_sync(kFull, far);
   if (lane == 0) m->red()[wid][0] = far;
   __syncthreads();
