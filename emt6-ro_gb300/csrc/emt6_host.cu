@@ -274,11 +274,13 @@ struct DevBuf {
 }  // namespace
 
 // Launches of fewer steps run a resident batch on the wide tier alone, which takes
-// any simulation: one launch instead of the tier guess and three launches.  The
-// narrow tier is 2 to 4 % faster where it fits.  600 discs of radius 6, both tiers
-// in turn and wide alone: 1 step 28 and 22 us, 20 steps 119 and 121, 40 steps 217
-// and 226; of radius 18: 67 and 58, 472 and 463.  Side by side costs what both in
-// turn do, and less where some simulations outgrow the narrow tier.
+// any simulation: one launch instead of the tier guess and three launches.  Run and
+// wait for 600 discs of radius 6, side by side and wide alone: 1 step 60 and 44 us,
+// 20 steps 146 and 138, 40 steps 258 and 243, 100 steps 536 and 554 (the narrow tier
+// is 2 to 4 % faster where it fits); of radius 18: 96 and 81, 533 and 518, 965 and
+// 952, 2,415 and 2,403.  The line is where the two tiers in turn met the wide one;
+// side by side a batch with both kinds of regions gains from far fewer steps on
+// (100 discs of radius 16, which outgrow the narrow tier, 300 steps: 3.6 vs 5.9 ms).
 constexpr uint32_t kSplitSteps = 24;
 
 struct emt6_batch {
@@ -440,10 +442,11 @@ struct emt6_batch {
     // Side by side, the lone tier takes a part where the wide one is slower than it
     // in turns of one simulation per SM.  Regions above 6 x 12 slots with two
     // simulations per SM, or with four where the wide tier holds three: 150 steps of
-    // 304 discs of radius 26 5.6 vs 6.5 ms, 608 of radius 24 on 54 x 60 9.1 vs 11.5
-    // (three or four per SM at once: 420 of radius 24 6.6, 9.1 in turns).  Regions of
-    // the largest tile, which the wide tier spills, in any number: 608 of radius 27 on
-    // 54 x 60 11.2 vs 17.8 ms, 3,000 55.7 vs 68.4.
+    // 304 discs of radius 24 4.5 vs 5.5 ms, of radius 26 5.5 vs 6.5, 608 of radius 24
+    // on 54 x 60 9.0 vs 11.4 (with three or four on an SM at once the wide tier is
+    // the faster one: 420 of radius 24 6.5 vs 6.7).  Regions of the largest tile,
+    // which the wide tier spills, in any number: 608 of radius 27 on 54 x 60 11.2 vs
+    // 18.0 ms, 3,000 55.4 vs 68.9.
     const int64_t load = (n + sms - 1) / sms;
     lone_part = load <= 2 || (load == 4 && per_sm[emt6::kTierWide] == 3) ? emt6::kRegionLarge
                 : W > emt6::kLargestWidth ? emt6::kRegionLargest : 0;

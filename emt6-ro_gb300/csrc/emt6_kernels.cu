@@ -7,13 +7,14 @@
 // simulation stay L2-resident.  Three kernels: run_kernel<kTierNarrow> (5 CTAs/SM, a
 // window of at most 40 lattice rows on chip) for regions that fit a tile of 32
 // slots per lane, run_kernel<kTierWide> (4 CTAs/SM, the whole lattice) for
-// larger ones, and run_kernel<kTierLone> (384 threads) for batches of at most one
-// simulation per SM.  Per step (reference cadence,
-// src/emt6ro/simulation/simulation.cu:153-166):
+// larger ones (on the default lattice; smem_layout has the others), and
+// run_kernel<kTierLone> (384 threads, 1 CTA/SM) for batches of at most one
+// simulation per SM and for the large regions of some others.  Per step (reference
+// cadence, src/emt6ro/simulation/simulation.cu:153-166):
 //   t % 128 == 0  rebuild the occupied list        (simulation.cu:41-64)
 //   t % 32  == 0  ROI + circular fixed-value mask   (diffusion.cu:65-100)
 //   diffusion: 23 substeps over free sites + 1 over the ROI (diffusion.cu:135-191),
-//     each field in the registers of one warp (emt6_tiles.cuh)
+//     each field in the registers of one warp, or of four (emt6_tiles.cuh)
 //   cell update: 8-neighbour vacancy snapshot, Site::step per list entry,
 //     at most one division per simulation (simulation.cu:66-110).
 // Randomness is Philox keyed by (step, simulation, site, occurrence), so the
@@ -72,7 +73,9 @@ __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x
 // 3 on each quarter of the SM; with 3 CTAs one quarter has 3 warps and the CTAs
 // wait for it: 23% slower diffusion).  Its list may hold every interior site;
 // what does not fit of the entries' clocks lies in the padding of the cell
-// records, entry by entry (`held` of them are on chip).
+// records, entry by entry (`held` of them are on chip).  kMinEntries are held on
+// any lattice, so the counts are those of lattices up to 53 x 53 sites: larger ones
+// have 3 CTAs of the wide tier, and the largest (56 x 62) 4 of the narrow one.
 constexpr int kWindowRows = 40;
 constexpr uint32_t kEntryBytes = 4 + 4 + 2 + 1, kMinEntries = 1024;
 
@@ -790,11 +793,12 @@ __device__ __forceinline__ void count_diffused(Misc *m, const KParams &p, uint32
 // kTierNarrow: regions that fit a tile of at most 32 slots per lane (discs up
 // to distance 16, clipped regions up to 32 x 32), 5 CTAs/SM.  A simulation it
 // cannot hold (region, window or list) is parked at the start of that step for
-// kTierWide: any simulation, 4 CTAs/SM.  kTierLone: any simulation,
-// one CTA of 384 threads per SM, for batches that leave SMs idle otherwise: a
-// step's latency instead of the SM's throughput (300 steps: one disc of radius 10
-// 1.56 vs 1.67 ms, 100 of them 3.09 vs 3.23; 152 of radius 24, 200 steps, 3.2 vs
-// 6.0).
+// kTierWide: any simulation, 4 CTAs/SM.  kTierLone: any simulation, one CTA of 384
+// threads per SM, for batches that leave SMs idle otherwise, and for regions that
+// the wide tier is slower on (emt6_batch::prepare_launch): a step's latency instead
+// of the SM's throughput (one disc of radius 10, 300 steps: 1.39 vs 1.46 ms with the
+// other tiers side by side, 100 of them 1.41 vs 1.47; 152 of radius 24, 200 steps:
+// 3.01 vs 5.92).
 template <int TIER>
 __global__ void __launch_bounds__(threads_of(TIER), TIER == kTierLone ? 1 : TIER == kTierWide ? 4 : 5)
     run_kernel(const __grid_constant__ RunArgs a, uint32_t t_end) {

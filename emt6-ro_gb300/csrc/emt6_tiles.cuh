@@ -1,4 +1,5 @@
-// emt6_tiles.cuh -- register tiles of the diffusion step, one warp per field.
+// emt6_tiles.cuh -- register tiles of the diffusion step, one warp per field (four at
+// the end of this file).
 //
 // A warp holds one field's active block in registers for the whole step (23 +
 // 1 substeps): lane = 8 * bw + bl owns the C columns C*bl .. and the R rows
@@ -140,7 +141,7 @@ __device__ __forceinline__ void diffuse_tile(float *__restrict__ f, const uint32
              (c == C - 1 ? rv[i] : X[i][c < C - 1 ? c + 1 : 0]);
     };
     // the band's first and last rows first: their G crosses to other lanes.
-    // Tiles of up to 32 slots fetch every row's neighbours at once, larger
+    // Tiles of up to 50 slots fetch every row's neighbours at once, larger
     // ones a row ahead (their registers are taken by the tile).
     constexpr bool AHEAD = C * R > 50;
     hshuffle(0);
@@ -245,9 +246,9 @@ __device__ __noinline__ void diffuse_large(float *f, const uint32_t *masks, int 
 // through shared memory, a barrier of the field's warps per substep: slower per
 // SM than one warp per tile, but a lone warp fetches and issues an instruction in
 // two cycles, so that a simulation with an SM to itself is done sooner this way
-// from 72 slots on (152 discs of radius 24, 200 steps: 3.2 vs 5.0 ms with one
-// warp per field; of radius 22, 66 slots, 3.1 with one).  `slots` holds 2 x 4 x 2
-// rows of 32 float2.
+// from 72 slots on (152 discs of radius 24, 200 steps: 3.0 ms, 5.0 with one warp per
+// field in the same CTA; of radius 22, 66 slots, 3.1 with one).  `slots` holds
+// 2 x 4 x 2 rows of 32 float2.
 constexpr int kPartSlots = 2 * 4 * 2 * 32;
 template <int RH>
 __device__ __forceinline__ void diffuse_parts(float *__restrict__ f, const uint64_t *__restrict__ colmask,

@@ -18,8 +18,10 @@
 //     memory, with Adam on the spot; the vectors' gradients beside them.
 //
 // Every wait on an mbarrier is bounded (kWaitLimitNs); a wait that runs out
-// sets an error flag, the CTA stops issuing work, waits (bounded) for its own
-// tensor-core work, frees its TMEM and returns; the host reports the flag.
+// sets an error flag, the CTA stops issuing products and loads, goes through its
+// cluster's exchanges and barriers with the others, waits (bounded) for its own
+// tensor-core work, frees its TMEM and returns; weights that would be spoiled are not
+// updated, and the host reports the flag.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -509,7 +511,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   pdl_wait();  // weights come from the previous kernel
 
   // weight tiles of all phases in one sequence: layer 1 has 2 k-blocks, the
-  // others 8; the producer runs ahead of the products by the ring's 4 stages
+  // others 8; the producer runs ahead of the products by the ring's 6 stages
   int issued = 0;
   bool failed = false;
   auto load_tiles = [&](int phase, int from, int to) {  // thread 0
