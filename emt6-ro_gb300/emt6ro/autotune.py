@@ -9,7 +9,7 @@ stages on a stratified sample of the batch from identical initial states:
    the per-launch load/store of every lattice; shorter ones let simulations
    that finish or outgrow the narrow kernel be rescheduled sooner), the
    schedule (one CTA per simulation vs persistent CTAs over a device work
-   queue ordered by horizon) and CUDA-graph replay of the launch sequence;
+   queue, both in region order) and CUDA-graph replay of the launch sequence;
 2. with the fastest launch, which tile shapes the kernels may use
    (Batch.LAYOUT_* bits: tiles of just the free block of unclipped regions,
    small and large ones, and tiles filled to their last row and column).

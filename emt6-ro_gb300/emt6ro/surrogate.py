@@ -167,19 +167,19 @@ class Surrogate:
         and one read-back per `_PIECE` rows (105 MB on the device, however many
         rows there are); with `mean` and `std` the rows are raw and standardised
         on the device."""
-        torch = self._torch
+        torch, lib, dev = self._torch, N.lib(), f"cuda:{self.device}"
         out = np.zeros(len(x), np.float32)
-        for i in range(0, len(x), self._PIECE):
-            part = x[i:i + self._PIECE]
-            n = len(part)
-            xd = self._to_dev(part)
-            with torch.cuda.stream(self._stream()):
-                yd = torch.empty(n, dtype=torch.float32, device=f"cuda:{self.device}")
-                N.check(N.lib().emt6_mlp_predict_rows(self._h, xd.data_ptr(), n, N.ptr(mean),
-                                                      N.ptr(std), yd.data_ptr()))
+        with torch.cuda.stream(self._stream()):
+            for i in range(0, len(x), self._PIECE):
+                part = x[i:i + self._PIECE]
+                n = len(part)
+                xd = torch.from_numpy(part).to(dev)
+                yd = torch.empty(n, dtype=torch.float32, device=dev)
+                N.check(lib.emt6_mlp_predict_rows(self._h, xd.data_ptr(), n, N.ptr(mean),
+                                                  N.ptr(std), yd.data_ptr()))
                 torch.from_numpy(out[i:i + n]).copy_(yd)
         # the copies have waited: no values of a launch that gave up
-        N.check(N.lib().emt6_mlp_status(self._h))
+        N.check(lib.emt6_mlp_status(self._h))
         return out
 
     def predict_std(self, x_std) -> np.ndarray:
