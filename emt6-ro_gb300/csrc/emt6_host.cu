@@ -282,6 +282,10 @@ struct DevBuf {
 // side by side a batch with both kinds of regions gains from far fewer steps on
 // (100 discs of radius 16, which outgrow the narrow tier, 300 steps: 3.6 vs 5.9 ms).
 constexpr uint32_t kSplitSteps = 24;
+// The same for batches of four simulations per SM where the tiers hold fewer at once,
+// so single steps: 20 records of 608 discs of radius 24 on 54 x 60, one step each, 4.1
+// vs 4.6 ms, of radius 8 1.5 vs 1.8; of radius 14, two steps each, 2.6 vs 2.4.
+constexpr uint32_t kSplitStepsMore = 2;
 
 struct emt6_batch {
   std::mutex mu;
@@ -303,6 +307,7 @@ struct emt6_batch {
   bool use_graph = false;
   bool occ_known = false;
   bool resident = false, lone = false;
+  uint32_t brief_below = 0;  // steps of a launch below which the tiers are not split
   int route = 0;  // emt6_test_batch_route
   int sms = 0, per_sm[emt6::kTiers] = {1, 1};
   cudaGraphExec_t graph_exec = nullptr;
@@ -439,6 +444,7 @@ struct emt6_batch {
     // tier, in one launch.
     resident = n <= (int64_t)std::min(per_sm[emt6::kTierNarrow], per_sm[emt6::kTierWide]) * sms;
     lone = n <= (int64_t)emt6::max_ctas_per_sm(kp, emt6::kTierLone) * sms;
+    brief_below = resident ? kSplitSteps : n <= (int64_t)4 * sms ? kSplitStepsMore : 0;
     // Side by side, the lone tier takes a part where the wide one is slower than it
     // in turns of one simulation per SM.  Regions above 6 x 12 slots with two
     // simulations per SM, or with four where the wide tier holds three: 150 steps of
@@ -475,7 +481,7 @@ struct emt6_batch {
 
   int launch(emt6::RunArgs a, uint32_t end, int tier, cudaStream_t st, unsigned long long *count) {
     int grid = (int)std::min<int64_t>(n, 0x7fffffff);
-    if (sched == 1 && !resident) {
+    if (sched == 1 && a.order) {
       grid = (int)std::min<int64_t>(n, (int64_t)per_sm[tier] * sms);
       a.queue = 1;
       a.ticket = ticket.p + (a.tier_of ? tier : emt6::kTiers);
@@ -495,7 +501,7 @@ struct emt6_batch {
     while (t < target) {
       const uint32_t end = (uint32_t)std::min<uint64_t>(target, (uint64_t)t + chunk);
       if (has_horizon && t >= max_horizon) break;
-      const bool brief = resident && (route ? route == 2 : end - t < kSplitSteps);
+      const bool brief = route ? route == 2 : end - t < brief_below;
       const int part = lone_part && (seen[emt6::kRegionLargest] || seen[lone_part]) ? lone_part : 0;
       if (lone || (brief && !part)) {
         a.order = nullptr;
@@ -506,7 +512,7 @@ struct emt6_batch {
         // simulations expected to fit it: one after the other would leave most
         // SMs idle at the end of each.  What outgrows the narrow tier meanwhile
         // is finished by the last launch.
-        if (resident) {
+        if (resident || brief) {
           a.order = nullptr;
           EMT6_CUDA(emt6::launch_tiers(a, tier.p, part, !brief, stream));
           *count += 1;

@@ -218,3 +218,30 @@ def test_a_tumour_that_shrank_is_expected_on_the_narrow_tier(params):
     assert tiers() == [0, 0]
     b.reset()
     assert tiers() == [1, 0]
+
+
+@pytest.mark.parametrize("dims,radii,n,schedule,launches", [
+    ((54, 60), (6, 12, 18, 22), 500, 1, 1),   # wide alone, though not all resident
+    ((54, 60), (6, 24, 27, 40), 500, 3, 3),   # large regions beside it
+    ((51, 51), (6, 12, 18, 22), 608, 1, 1),
+    ((54, 60), (6, 12, 18, 22), 700, 1, 6)])
+def test_runs_of_single_steps(dims, radii, n, schedule, launches, oracle):
+    """Recordings of every step: launches per run and the oracle's lattices."""
+    from emt6ro import workloads as wl
+    from emt6ro.batch import Batch
+    params = wl.default_parameters()
+    params.native.lattice_height, params.native.lattice_width = dims
+    tumors = [wl.disc_tumor(params, r, seed=60 + r) for r in radii]
+    st, k, steps = np.arange(n) % 4, 8, 36
+    b = Batch(params, tumors, [[(0, 0.5)]], st, np.zeros(n, np.int32), seed=14)
+    b.set_schedule(schedule, 0)
+    before = b.launches()
+    for _ in range(steps):
+        b.run(1)
+    assert b.launches() - before == launches * steps
+    ob = oracle.Batch(oracle.params_copy(params.native), k, 14)
+    for j in range(k):
+        ob.set(j, tumors[st[j]].sites, b.doses[0], resolution=300, length=144_000)
+    ob.run(steps, nthreads=8)
+    for j in range(k):
+        assert b.state(j).sites.tobytes() == ob.get(j).tobytes(), j
