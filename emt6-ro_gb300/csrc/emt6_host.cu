@@ -286,6 +286,11 @@ constexpr uint32_t kSplitSteps = 24;
 // so single steps: 20 records of 608 discs of radius 24 on 54 x 60, one step each, 4.1
 // vs 4.6 ms, of radius 8 1.5 vs 1.8; of radius 14, two steps each, 2.6 vs 2.4.
 constexpr uint32_t kSplitStepsMore = 2;
+// Below this the wide tier alone is joined by the lone one, which loads and stores its
+// states in turns (prepare_launch), for regions of the largest tile only: 20 records of
+// 260 discs of radius 22 to 24, one step each, 2.1 vs 2.4 ms with it, five steps 5.2
+// and 5.3, 20 steps 15.8 vs 14.3.
+constexpr uint32_t kLoneSteps = 4;
 
 struct emt6_batch {
   std::mutex mu;
@@ -330,7 +335,7 @@ struct emt6_batch {
   // pinned memory; what it holds by the time of a run only chooses the launches.
   int lone_part = 0;
   volatile uint8_t *seen = nullptr, *seen_dev = nullptr;
-  uint8_t tpl_seen[emt6::kRegionClasses] = {0, 0, 0};  // of the tumours
+  uint8_t tpl_seen[emt6::kRegionClasses] = {0};  // of the tumours
   DevBuf<uint32_t> step, horizon, counts, err, ticket, order_hist;
   DevBuf<int64_t> order;  // per chunk: simulations by region, largest first
   DevBuf<unsigned long long> diffused;
@@ -446,20 +451,22 @@ struct emt6_batch {
     lone = n <= (int64_t)emt6::max_ctas_per_sm(kp, emt6::kTierLone) * sms;
     brief_below = resident ? kSplitSteps : n <= (int64_t)4 * sms ? kSplitStepsMore : 0;
     // Side by side, the lone tier takes a part where the wide one is slower than it
-    // in turns of one simulation per SM.  Regions above 6 x 12 slots with two
-    // simulations per SM, or with four where the wide tier holds three: 150 steps of
-    // 304 discs of radius 24 4.5 vs 5.5 ms, of radius 26 5.5 vs 6.5, 608 of radius 24
-    // on 54 x 60 9.0 vs 11.4 (with three or four on an SM at once the wide tier is
-    // the faster one: 420 of radius 24 6.5 vs 6.7).  Regions of the largest tile,
-    // which the wide tier spills, in any number: 608 of radius 27 on 54 x 60 11.2 vs
-    // 18.0 ms, 3,000 55.4 vs 68.9.
+    // in turns of one simulation per SM.  Regions from 72 slots on with two simulations
+    // per SM (150 steps of 304 discs of radius 23 5.3 vs 5.6 ms, of radius 24 4.5 vs
+    // 5.5, of radius 26 5.5 vs 6.5; in short runs those above 6 x 12 slots, as 10 steps
+    // of radius 23 are 0.41 vs 0.39), and above 6 x 12 slots with four where the wide
+    // tier holds three: 608 of radius 24 on 54 x 60 9.0 vs 11.4 (with three or four on
+    // an SM at once the wide tier is the faster one: 420 of radius 24 6.5 vs 6.7).
+    // Regions of the largest tile, which the wide tier spills, in any number: 608 of
+    // radius 27 on 54 x 60 11.2 vs 18.0 ms, 3,000 55.4 vs 68.9.
     const int64_t load = (n + sms - 1) / sms;
-    lone_part = load <= 2 || (load == 4 && per_sm[emt6::kTierWide] == 3) ? emt6::kRegionLarge
+    lone_part = load <= 2 ? emt6::kRegionMedium
+                : load == 4 && per_sm[emt6::kTierWide] == 3 ? emt6::kRegionLarge
                 : W > emt6::kLargestWidth ? emt6::kRegionLargest : 0;
     if (route) {
       lone = route == 1;
       resident = route < 4;
-      lone_part = route == 5 ? emt6::kRegionLarge : 0;
+      lone_part = route == 5 ? emt6::kRegionMedium : 0;
     }
     if (lone) lone_part = 0;
     if (lone_part && !seen) {
@@ -477,6 +484,15 @@ struct emt6_batch {
     if (!lone && !fork) EMT6_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     occ_known = true;
     return EMT6_OK;
+  }
+
+  // the class of regions from which on a split launch uses the lone tier, 0: it does not
+  int lone_from(uint32_t steps, bool brief) const {
+    const int least = !brief ? 0 : steps < kLoneSteps ? emt6::kRegionLargest : emt6::kRegionLarge;
+    const int from = std::max(lone_part, least);
+    for (int k = from; lone_part && k < emt6::kRegionClasses; ++k)
+      if (seen[k]) return from;
+    return 0;
   }
 
   int launch(emt6::RunArgs a, uint32_t end, int tier, cudaStream_t st, unsigned long long *count) {
@@ -502,7 +518,7 @@ struct emt6_batch {
       const uint32_t end = (uint32_t)std::min<uint64_t>(target, (uint64_t)t + chunk);
       if (has_horizon && t >= max_horizon) break;
       const bool brief = route ? route == 2 : end - t < brief_below;
-      const int part = lone_part && (seen[emt6::kRegionLargest] || seen[lone_part]) ? lone_part : 0;
+      const int part = lone_from(end - t, brief);
       if (lone || (brief && !part)) {
         a.order = nullptr;
         const int rc = launch(a, end, lone ? emt6::kTierLone : emt6::kTierWide, stream, count);
@@ -514,7 +530,7 @@ struct emt6_batch {
         // is finished by the last launch.
         if (resident || brief) {
           a.order = nullptr;
-          EMT6_CUDA(emt6::launch_tiers(a, tier.p, part, !brief, stream));
+          EMT6_CUDA(emt6::launch_tiers(a, tier.p, part, !brief, sms, stream));
           *count += 1;
         } else {
           EMT6_CUDA(emt6::launch_order(a, end, order_hist.p, order.p, tier.p, part, stream));
@@ -1172,7 +1188,7 @@ int emt6_test_batch_tiers(emt6_batch *b, uint8_t *out) {
   if (!b || !out) return fail(EMT6_ERR_INVALID, "null argument");
   std::lock_guard<std::mutex> lk(b->mu);
   DeviceGuard g(b->device);
-  EMT6_CUDA(emt6::launch_tiers(b->run_args(), b->tier.p, 0, true, b->stream));
+  EMT6_CUDA(emt6::launch_tiers(b->run_args(), b->tier.p, 0, true, 0, b->stream));
   EMT6_CUDA(cudaMemcpyAsync(out, b->tier.p, (size_t)b->n, cudaMemcpyDeviceToHost, b->stream));
   EMT6_CUDA(cudaStreamSynchronize(b->stream));
   return EMT6_OK;

@@ -458,21 +458,20 @@ __device__ __forceinline__ void diffuse_by_parts(float *fld, int plane, const ui
     diffuse_parts<14>(f, colmask, slots, part, 1 + field, r0, c0, h, w, p.W, ext, ca, cb, cd, p.nfree);
 }
 
-// The class (kRegion*) of a region: what tile_mapping's tiles hold of it.  "Large"
-// starts where the lone tier is faster for short runs, too (10 steps of 304 discs of
-// distance 23, which 6 x 12 slots hold: 0.42 ms there, 0.39 on the wide tier; of
-// distance 24 0.38 and 0.41).
+// The class (kRegion*) of a region: what tile_mapping's tiles hold of it.
 __host__ __device__ inline int class_of(int h, int w, int d, int H, int W) {
-  constexpr TileShape below = tile_shape(kPartTiles), largest = tile_shape(kNumTiles - 2);
-  static_assert(!below.RE && !below.CE && largest.RE && !largest.CE && 4 * largest.R >= 56 &&
-                    8 * largest.C - 1 == kLargestWidth,
+  constexpr TileShape small = tile_shape(kPartTiles - 1), medium = tile_shape(kPartTiles),
+                      largest = tile_shape(kNumTiles - 2);
+  static_assert(small.RE && !small.CE && !medium.RE && !medium.CE && largest.RE && !largest.CE &&
+                    4 * largest.R >= 56 && 8 * largest.C - 1 == kLargestWidth,
                 "what the tiles hold");
   const bool block = h == 2 * d + 1 && w == h;
   const bool next = block && h + 2 <= H - 2 && w + 2 <= W - 2;  // a block one site larger, too
   const int nr = block ? 2 * d : h + 2, nc = block ? 2 * d : w + 2;
   const int grown = next ? w + 1 : (w + 2 < W - 2 ? w + 2 : W - 2) + 2;
   if (h > 0 && (nc > kLargestWidth || grown > kLargestWidth)) return kRegionLargest;
-  return nr > 4 * below.R - 1 || nc > 8 * below.C - 1 ? kRegionLarge : kRegionSmall;
+  if (nr > 4 * medium.R - 1 || nc > 8 * medium.C - 1) return kRegionLarge;
+  return nr > 4 * small.R || nc > 8 * small.C - 1 ? kRegionMedium : kRegionSmall;
 }
 
 int region_class(const int32_t roi[5], int H, int W) { return class_of(roi[2], roi[3], roi[4], H, W); }
@@ -1230,14 +1229,13 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(uint32_t *hist) {
 // tiles' limit is given to the wide tier, which runs it nearly as fast: it may
 // grow in the next steps, and what is left for the last launch runs alone.  Regions
 // from class `lone` on (unless 0) go to the lone tier.
-__device__ __forceinline__ uint8_t expected_tier(const RunArgs &a, int64_t sim, int lone,
-                                                  bool narrow) {
+__device__ __forceinline__ uint8_t expected_tier(const RunArgs &a, int64_t sim, int lone) {
   const int *roi = a.roi + sim * 8;
   const int h = roi[2], w = roi[3], d = roi[4];
   const int n = (a.step[sim] == 0 ? roi[5] : a.meta[sim].x) + 64;
   const bool small = (h == 2 * d + 1 && w == h) ? d <= 15 : h + 2 <= 30 && w + 2 <= 30;
   if (lone && class_of(h, w, d, a.p.H, a.p.W) >= lone) return kTierLone;
-  if (narrow && small && n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierNarrow).entries)
+  if (small && n < smem_layout(a.p.H, a.p.W, a.p.lcap, kTierNarrow).entries)
     return kTierNarrow;
   return kTierWide;
 }
@@ -1247,13 +1245,31 @@ __global__ void order_scatter_kernel(const RunArgs a, uint32_t t_end, uint32_t *
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.nsims;
        i += (int64_t)gridDim.x * blockDim.x) {
     out[atomicAdd(&hist[order_key(a, i, t_end)], 1u)] = i;
-    if (tier) tier[i] = expected_tier(a, i, lone, true);
+    if (tier) tier[i] = expected_tier(a, i, lone);
   }
 }
 
-__global__ void tier_kernel(const RunArgs a, uint8_t *tier, int lone, bool narrow) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < a.nsims) tier[i] = expected_tier(a, i, lone, narrow);
+// Tiers of a batch that is resident at once, by one block.  The lone tier takes whole
+// SMs, and the wide one would crowd on what is left of them; where its simulations
+// would be more than two to an SM there (`sms` SMs, 0: no such rule), they go to the
+// lone tier, too (260 discs of radius 22 to 24, 300 steps: 9.0 ms, 10.3 on the wide tier
+// alone; crowded they took 12.1).
+constexpr int kTierThreads = 1024;
+__global__ void __launch_bounds__(kTierThreads) tier_kernel(const RunArgs a, uint8_t *tier, int lone,
+                                                            bool narrow, int sms) {
+  __shared__ int count[kTiers];
+  if (threadIdx.x < kTiers) count[threadIdx.x] = 0;
+  __syncthreads();
+  if (lone && sms)
+    for (int64_t i = threadIdx.x; i < a.nsims; i += kTierThreads)
+      atomicAdd(&count[expected_tier(a, i, lone)], 1);
+  __syncthreads();
+  const bool crowded = count[kTierWide] > 2 * max(sms - count[kTierLone], 0);
+  for (int64_t i = threadIdx.x; i < a.nsims; i += kTierThreads) {
+    uint8_t t = expected_tier(a, i, lone);
+    if (t == kTierWide && crowded) t = kTierLone;
+    tier[i] = t == kTierNarrow && !narrow ? (uint8_t)kTierWide : t;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1478,9 +1494,9 @@ cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64
   return cudaGetLastError();
 }
 
-cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, int lone, bool narrow,
+cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, int lone, bool narrow, int sms,
                          cudaStream_t stream) {
-  tier_kernel<<<(unsigned)((a.nsims + 127) / 128), 128, 0, stream>>>(a, tier, lone, narrow);
+  tier_kernel<<<1, kTierThreads, 0, stream>>>(a, tier, lone, narrow, sms);
   return cudaGetLastError();
 }
 

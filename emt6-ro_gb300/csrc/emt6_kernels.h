@@ -59,10 +59,11 @@ struct ResetArgs {
 // (regions too wide or lists too long for the shared memory that lets 5 CTAs
 // share an SM); it holds any.
 enum { kTierNarrow = 0, kTierWide = 1, kTierLone = 2, kTiers = 3 };
-// Classes of regions, by the wide tier's tile: up to 6 x 12 slots per lane, above,
-// and those that only the largest tile holds (or will, one site larger).  A launch of
-// several tiers side by side may give the lone one the regions from a class on.
-enum { kRegionSmall = 0, kRegionLarge = 1, kRegionLargest = 2, kRegionClasses = 3 };
+// Classes of regions, by the wide tier's tile: below 6 x 12 slots per lane, those,
+// above, and those that only the largest tile holds (or will, one site larger).  A
+// launch of several tiers side by side may give the lone one the regions from a class
+// on.
+enum { kRegionSmall = 0, kRegionMedium = 1, kRegionLarge = 2, kRegionLargest = 3, kRegionClasses = 4 };
 constexpr int kLargestWidth = 55;  // wider whole regions need the largest tile
 int region_class(const int32_t roi[5], int H, int W);
 size_t run_kernel_smem(int H, int W, int lcap, int tier);
@@ -77,8 +78,10 @@ cudaError_t launch_reset(const ResetArgs &a, cudaStream_t stream);
 constexpr uint32_t kOrderKeys = 4096;
 cudaError_t launch_order(const RunArgs &a, uint32_t t_end, uint32_t *hist, int64_t *out,
                          uint8_t *tier, int lone, cudaStream_t stream);
-// the tiers alone, for a batch that needs no order, without the narrow one if asked
-cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, int lone, bool narrow, cudaStream_t stream);
+// the tiers alone, for a batch that needs no order, without the narrow one if asked,
+// and (sms not 0) with the wide one's on the lone one if they would crowd beside it
+cudaError_t launch_tiers(const RunArgs &a, uint8_t *tier, int lone, bool narrow, int sms,
+                         cudaStream_t stream);
 cudaError_t instr_read(unsigned long long counts[4], double *sum_dp, unsigned long long *hist);
 cudaError_t instr_reset();
 cudaError_t fp32_peak(int device, double *tflops);

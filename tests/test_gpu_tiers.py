@@ -159,6 +159,7 @@ def test_cells_on_a_vacant_far_border_count_for_the_region(n, params, oracle):
 
 @pytest.mark.parametrize("dims,radii,n,schedule,launches", [
     ((51, 51), (5, 24, 26, 36), 200, 0, (5, 3)),   # two simulations per SM
+    ((51, 51), (20, 22, 23, 24), 260, 2, (5, 3)),  # too many others for the SMs left
     ((51, 51), (5, 12, 17, 20), 200, 2, (4, 1)),   # no large region
     ((51, 51), (5, 24, 26, 36), 400, 0, (4, 1)),   # more per SM
     ((51, 51), (5, 24, 26, 36), 700, 1, (6, 6)),
@@ -222,7 +223,8 @@ def test_a_tumour_that_shrank_is_expected_on_the_narrow_tier(params):
 
 @pytest.mark.parametrize("dims,radii,n,schedule,launches", [
     ((54, 60), (6, 12, 18, 22), 500, 1, 1),   # wide alone, though not all resident
-    ((54, 60), (6, 24, 27, 40), 500, 3, 3),   # large regions beside it
+    ((54, 60), (6, 24, 27, 40), 500, 3, 3),   # the largest tile beside it
+    ((51, 51), (6, 24, 26, 36), 200, 0, 1),   # large, but too few steps
     ((51, 51), (6, 12, 18, 22), 608, 1, 1),
     ((54, 60), (6, 12, 18, 22), 700, 1, 6)])
 def test_runs_of_single_steps(dims, radii, n, schedule, launches, oracle):
